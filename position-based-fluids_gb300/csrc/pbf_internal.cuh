@@ -326,11 +326,11 @@ struct DeviceState {
   uint32_t *offsets = nullptr;         // ncells + 1
   uint4 *runs = nullptr;               // offset_runs_capacity(ncells) queued runs
   uint32_t *runs_count = nullptr;
-  uint4 *nbr = nullptr;                // neighbour lists, 4 slots or 8 staged indices per word (paper)
-  uint32_t *nbr_cnt = nullptr;         // neighbour counts (paper)
+  uint4 *nbr = nullptr;                // neighbour lists, 4 slots or 8 staged indices per word
+  uint32_t *nbr_cnt = nullptr;         // neighbour counts
   uint32_t *nbr_max = nullptr;         // largest neighbour count of the step (paper)
   uint32_t *sort_scratch = nullptr;
-  uint32_t *cell_scratch = nullptr;    // counting sort by cell (paper)
+  uint32_t *cell_scratch = nullptr;    // counting sort by cell
   uint32_t *err = nullptr;             // device error flag word
   SceneDesc *scenes = nullptr;         // device scene table
   float4 *io_pos = nullptr, *io_vel = nullptr; // input-order staging
@@ -438,25 +438,42 @@ cudaError_t gather_scalar_to_input_order(const float *src, const uint32_t *ID,
 cudaError_t iota_u32(uint32_t *dst, uint32_t n, cudaStream_t st);
 
 // --------------------------------------------------- ref-compat launches --
+// Neighbour lists in the reference's visiting order.  maxn = 0: there was no
+// room for lists (nbr4 and cnt unused), every pass walks the cells.
+struct RefLists {
+  const uint4 *nbr4;
+  const uint32_t *cnt;
+  uint32_t n, maxn;
+};
+// The sort of a step runs over the particles in descending input index
+// (element t is particle n - 1 - t) and numbers the cells with z fastest: see
+// pbf_refcompat.cu.  Prediction, and the digit histograms of the radix sort
+// or the counts of the counting sort.
 cudaError_t rc_predict_hash(float4 *X, float4 *V, float4 *P, uint32_t n,
                             const RefConsts &k, const SceneDesc *scenes,
                             uint32_t *keys, const SortPlan &plan,
                             uint32_t *sort_scratch, cudaStream_t st);
-// PS[m] = P[perm[m]]: the predicted positions by sorted slot.
+cudaError_t rc_predict_count(float4 *X, float4 *V, float4 *P, uint32_t n, const RefConsts &k,
+                             const SceneDesc *scenes, uint32_t *keys, const CellSortPlan &plan,
+                             uint32_t *cell_scratch, cudaStream_t st);
+// PS[m] = P of the particle in slot m: the predicted positions by slot.
 cudaError_t rc_gather(const float4 *P, const uint32_t *perm, uint32_t n, float4 *PS,
                       cudaStream_t st);
+// Neighbour lists of the positions PS.
+cudaError_t rc_build(const float4 *PS, const uint32_t *offsets, uint32_t n, const RefConsts &k,
+                     uint32_t maxn, uint4 *nbr, uint32_t *nbr_cnt, cudaStream_t st);
 // The passes read neighbours by sorted slot (PS, SS, VS) and write their own
 // slot's values there; the last delta-p pass also writes P and V by input
 // index for the commit.
-cudaError_t rc_lambda(float4 *PS, float *SS, const uint32_t *offsets, uint32_t n,
-                      const RefConsts &k, cudaStream_t st);
-cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const uint32_t *perm,
-                     const uint32_t *offsets, const float4 *X, float4 *V, float4 *P,
-                     float4 *VS, uint32_t n, const RefConsts &k, const SceneDesc *scenes,
-                     bool last, cudaStream_t st);
-cudaError_t rc_xsph(const float4 *PS, const float4 *VS, float4 *DV, const uint32_t *perm,
-                    const uint32_t *offsets, uint32_t n, const RefConsts &k,
-                    cudaStream_t st);
+cudaError_t rc_lambda(float4 *PS, float *SS, const RefLists &lists, const uint32_t *offsets,
+                      uint32_t n, const RefConsts &k, cudaStream_t st);
+cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const RefLists &lists,
+                     const uint32_t *perm, const uint32_t *offsets, const float4 *X, float4 *V,
+                     float4 *P, float4 *VS, uint32_t n, const RefConsts &k,
+                     const SceneDesc *scenes, bool last, cudaStream_t st);
+cudaError_t rc_xsph(const float4 *PS, const float4 *VS, float4 *DV, const RefLists &lists,
+                    const uint32_t *perm, const uint32_t *offsets, uint32_t n,
+                    const RefConsts &k, cudaStream_t st);
 cudaError_t rc_commit(float4 *X, float4 *V, const float4 *P, const float4 *DV,
                       uint32_t n, cudaStream_t st);
 

@@ -8,16 +8,28 @@
 //   apply_vorticity_and_viscosity.cl:12-104, update_positions.cl:9-12.
 //
 // State stays in input order (X, V, P = predicted with .w = density).  The
-// neighbour structure is the stable sort of (cell, index) plus CSR offsets;
-// each gather kernel visits the 27 cells around the particle's *current*
-// cell in the reference's loop order (x outer, z inner) and each cell's
-// particles in descending index -- the order a sequential launch of
-// update_cells.cl leaves in the reference's linked lists.  With that order
-// the results equal the reference's kernels bit for bit.  During the step
-// the passes keep P, V and lambda by sorted slot as well (PS, VS, SS), so a
-// cell's particles are read from consecutive slots -- the same values in
-// the same order as through the permutation.
-#include "pbf_device.cuh"
+// reference visits the 27 cells around the particle's *current* cell with x
+// outermost and z innermost, and each cell's particles in descending index --
+// the order a sequential launch of update_cells.cl leaves in its linked
+// lists.  The neighbour structure is laid out in exactly that order: cells
+// are numbered with z fastest (rc_cell) and the particles are sorted in
+// descending input index (sort element t is particle n - 1 - t), so the three
+// cells of one (x, y) row are one contiguous run of sorted slots that is
+// visited front to back.  Results then equal the reference's kernels bit for
+// bit.  During the step the passes keep P, V and lambda by sorted slot as
+// well (PS, VS, SS).
+//
+// The lambda and delta-p passes of one solver iteration evaluate the same
+// pairs: lambda moves nothing.  So each iteration's pairs are found once
+// (k_rc_build: the candidates of the nine rows tested into masks, members
+// stored in visiting order as neighbour lists) and both passes walk the list;
+// the XSPH pass has a list of its own, built at the final positions.  With
+// every pass scanning the 27 cells itself, a warp ran the pair arithmetic
+// (square roots and divisions) for nearly every one of ~216 candidates with
+// 15 of 32 lanes active: 572, 537 and 443 us per lambda, delta-p and XSPH
+// pass at 1,048,576 particles.  A particle with more members than the list
+// holds walks the cells in every pass instead.
+#include "pbf_lists.cuh"
 
 namespace pbf {
 
@@ -25,41 +37,101 @@ namespace {
 
 constexpr int kThreads = 128;
 
-// Calls f(m, load(m)) for the sorted slot m != q of every particle of the 27
-// cells around the current cell of position p, in the reference's order.
-// A cell's slots are loaded kGroup at a time (indices clamped into the cell),
-// so the group's loads are in flight together; f still sees them one by one
-// in descending slot order.
-template <int kGroup = 4, typename Load, typename F>
-__device__ __forceinline__ void ref_neighbours(uint32_t q, float4 p,
-                                               const RefConsts &k,
-                                               const uint32_t *__restrict__ off,
-                                               Load &&load, F &&f) {
-  int cc[3];
-  cc[0] = (int)((p.x - k.min[0]) / k.clen[0]);
-  cc[1] = (int)((p.y - k.min[1]) / k.clen[1]);
-  cc[2] = (int)((p.z - k.min[2]) / k.clen[2]);
-  const int nx = (int)k.ncell[0], ny = (int)k.ncell[1];
-  for (int dx = -1; dx <= 1; ++dx)
-    for (int dy = -1; dy <= 1; ++dy)
-      for (int dz = -1; dz <= 1; ++dz) {
-        const int n0 = cc[0] + dx, n1 = cc[1] + dy, n2 = cc[2] + dz;
-        if (n0 < 0 || (float)n0 >= k.ncell[0] || n1 < 0 ||
-            (float)n1 >= k.ncell[1] || n2 < 0 || (float)n2 >= k.ncell[2])
-          continue;
-        const uint32_t ci = (uint32_t)n0 + (uint32_t)nx * ((uint32_t)n1 + (uint32_t)ny * (uint32_t)n2);
-        const uint32_t a = __ldg(&off[ci]);
-        for (uint32_t top = __ldg(&off[ci + 1]); top > a; top = top - a > kGroup ? top - kGroup : a) {
-          decltype(load(0u)) d[kGroup];
-#pragma unroll
-          for (int e = 0; e < kGroup; ++e) d[e] = load(top - a > (uint32_t)e ? top - 1u - e : a);
-#pragma unroll
-          for (int e = 0; e < kGroup; ++e) {
-            const uint32_t m = top - 1u - e;
-            if (top - a > (uint32_t)e && m != q) f(m, d[e]);
-          }
-        }
-      }
+// Calls row(a, b) for the slot range [a, b) of each row of up to three cells
+// around the current cell of position p, in visiting order.  Cells outside
+// the grid hold nothing (the current cell itself may be outside).
+template <typename Row>
+__device__ __forceinline__ void ref_rows(float4 p, const RefConsts &k,
+                                         const uint32_t *__restrict__ off, Row &&row) {
+  const int nx = (int)k.ncell[0], ny = (int)k.ncell[1], nz = (int)k.ncell[2];
+  // two cells outside is as far as any: keeps the sums below in range
+  const int c0 = min(max((int)((p.x - k.min[0]) / k.clen[0]), -2), nx + 1);
+  const int c1 = min(max((int)((p.y - k.min[1]) / k.clen[1]), -2), ny + 1);
+  const int c2 = min(max((int)((p.z - k.min[2]) / k.clen[2]), -2), nz + 1);
+  const int z0 = max(c2 - 1, 0), z1 = min(c2 + 1, nz - 1);
+  if (z0 > z1) return;
+  for (int x = max(c0 - 1, 0); x <= min(c0 + 1, nx - 1); ++x)
+    for (int y = max(c1 - 1, 0); y <= min(c1 + 1, ny - 1); ++y) {
+      const uint32_t first = (uint32_t)nz * ((uint32_t)y + (uint32_t)ny * (uint32_t)x);
+      row(__ldg(&off[first + z0]), __ldg(&off[first + z1 + 1]));
+    }
+}
+
+// The reference's pair test on its r^2 (rounded operation by operator).
+__device__ __forceinline__ bool ref_pair(const float4 &pi, const float4 &pj, float h2) {
+  const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
+  const float r2 = rx * rx + ry * ry + rz * rz;
+  return r2 > 0.0f && r2 < h2;
+}
+
+// Calls f(load(m)) for the members of slot q in visiting order (and for q
+// itself as padding, which the pair test drops): from the list, or over all
+// candidates of the cells when the list does not hold the set.
+template <typename Load, typename F>
+__device__ __forceinline__ void ref_members(uint32_t q, float4 p, const RefConsts &k,
+                                            const RefLists &l, const uint32_t *__restrict__ off,
+                                            Load &&load, F &&f) {
+  const uint32_t cnt = l.maxn ? load_own(&l.cnt[q]) : 0u;
+  if (l.maxn && cnt <= l.maxn) {
+    for_each_listed<4>(l.nbr4, l.n, q, cnt, load, f);
+  } else {
+    ref_rows(p, k, off, [&](uint32_t a, uint32_t b) {
+      for (uint32_t m = a; m < b; ++m) f(load(m));
+    });
+  }
+}
+
+// Cell of a position with z fastest, as the passes' neighbour structure
+// numbers the cells (scene_cell is the reference's numbering, x fastest).
+__device__ __forceinline__ uint32_t rc_cell(float x, float y, float z, const SceneDesc &s) {
+  const int cx = axis_cell(x, s.gmin[0], s.clen[0], s.ncell[0]);
+  const int cy = axis_cell(y, s.gmin[1], s.clen[1], s.ncell[1]);
+  const int cz = axis_cell(z, s.gmin[2], s.clen[2], s.ncell[2]);
+  return (uint32_t)cz +
+         (uint32_t)s.ncell[2] * ((uint32_t)cy + (uint32_t)s.ncell[1] * (uint32_t)cx);
+}
+
+// Input index of sorted slot q (perm is a permutation of [0, n) unless the
+// sort reported an error).
+__device__ __forceinline__ uint32_t rc_input(const uint32_t *__restrict__ perm, uint32_t q,
+                                             uint32_t n) {
+  return n - 1u - min(perm[q], n - 1u);
+}
+
+// Prediction of sort element t (particle n - 1 - t) and its cell.
+__device__ __forceinline__ uint32_t rc_predict(uint32_t t, uint32_t n, const float4 *X, float4 *V,
+                                               float4 *P, const RefConsts &k,
+                                               const SceneDesc &scene) {
+  const uint32_t i = n - 1u - t;
+  const float4 x = X[i];
+  float4 v = V[i];
+  v.x = v.x + k.dt * 0.0f;
+  v.y = v.y + k.dt * -9.81f;
+  v.z = v.z + k.dt * 0.0f;
+  V[i] = v;
+  float4 p = P[i];
+  p.x = x.x + k.dt * v.x;
+  p.y = x.y + k.dt * v.y;
+  p.z = x.z + k.dt * v.z;
+  P[i] = p;
+  return rc_cell(p.x, p.y, p.z, scene);
+}
+
+// Prediction and cell of every particle, counted for the counting sort
+// (grid-stride, whole warps iterate together).
+__global__ void __launch_bounds__(256)
+    k_rc_predict_count(const float4 *__restrict__ X, float4 *__restrict__ V,
+                       float4 *__restrict__ P, uint32_t n, RefConsts k,
+                       const SceneDesc *__restrict__ scenes, uint32_t *__restrict__ keys,
+                       uint32_t *__restrict__ counts, uint32_t *__restrict__ pos) {
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
+    const uint32_t t = base + threadIdx.x;
+    const bool valid = t < n;
+    uint32_t key = 0;
+    if (valid) keys[t] = key = rc_predict(t, n, X, V, P, k, scenes[0]);
+    count_cell_key(key, valid, t, counts, pos);
+  }
 }
 
 __global__ void __launch_bounds__(256)
@@ -72,25 +144,14 @@ __global__ void __launch_bounds__(256)
   const uint32_t hist_words = passes << digit_bits;
   for (uint32_t t = threadIdx.x; t < hist_words; t += blockDim.x) s_hist[t] = 0;
   __syncthreads();
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < n;
-  uint32_t key = 0;
-  if (valid) {
-    const float4 x = X[i];
-    float4 v = V[i];
-    v.x = v.x + k.dt * 0.0f;
-    v.y = v.y + k.dt * -9.81f;
-    v.z = v.z + k.dt * 0.0f;
-    V[i] = v;
-    float4 p = P[i];
-    p.x = x.x + k.dt * v.x;
-    p.y = x.y + k.dt * v.y;
-    p.z = x.z + k.dt * v.z;
-    P[i] = p;
-    key = scene_cell(p.x, p.y, p.z, scenes[0]);
-    keys[i] = key;
+  const uint32_t stride = gridDim.x * blockDim.x;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
+    const uint32_t t = base + threadIdx.x;
+    const bool valid = t < n;
+    uint32_t key = 0;
+    if (valid) keys[t] = key = rc_predict(t, n, X, V, P, k, scenes[0]);
+    warp_digit_histogram(key, valid, passes, digit_bits, s_hist);
   }
-  warp_digit_histogram(key, valid, passes, digit_bits, s_hist);
   __syncthreads();
   for (uint32_t t = threadIdx.x; t < hist_words; t += blockDim.x)
     if (s_hist[t]) atomicAdd(&hist[t], s_hist[t]);
@@ -101,18 +162,43 @@ __global__ void __launch_bounds__(256)
                 float4 *__restrict__ PS) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
-  // perm is a permutation of [0, n) unless the sort reported an error.
-  PS[q] = P[min(perm[q], n - 1u)];
+  PS[q] = P[rc_input(perm, q, n)];
+}
+
+// Neighbour lists of the current positions in visiting order; the rest of
+// the last word holds the particle's own slot.  A set that outgrows the list
+// ends the scan: its passes walk the cells.
+__global__ void __launch_bounds__(kThreads)
+    k_rc_build(const float4 *__restrict__ PS, const uint32_t *__restrict__ off, uint32_t n,
+               RefConsts k, uint32_t maxn, uint4 *__restrict__ nbr4,
+               uint32_t *__restrict__ nbr_cnt) {
+  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  const float4 pi = PS[q];
+  uint32_t *__restrict__ out = reinterpret_cast<uint32_t *>(nbr4) + 4ull * q;
+  const size_t stride = 4ull * n;  // words from one list group to the next
+  uint32_t cnt = 0;
+  ref_rows(pi, k, off, [&](uint32_t a, uint32_t b) {
+    if (cnt > maxn) return;
+    scan_row_masked(
+        PS, a, b, [&](const float4 &pj) { return ref_pair(pi, pj, k.h2); },
+        [&](uint32_t m) {
+          if (cnt < maxn) out[(size_t)(cnt >> 2) * stride + (cnt & 3u)] = m;
+          ++cnt;
+        });
+  });
+  pad_list(out, stride, cnt, maxn, q);
+  nbr_cnt[q] = cnt;
 }
 
 __global__ void __launch_bounds__(kThreads)
-    k_rc_lambda(float4 *__restrict__ PS, float *__restrict__ SS,
+    k_rc_lambda(float4 *__restrict__ PS, float *__restrict__ SS, RefLists lists,
                 const uint32_t *__restrict__ off, uint32_t n, RefConsts k) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const float4 pi = PS[q];
   float dens = 0.0f, gsum = 0.0f, gvx = 0.0f, gvy = 0.0f, gvz = 0.0f;
-  ref_neighbours(q, pi, k, off, [&](uint32_t m) { return PS[m]; }, [&](uint32_t, float4 pj) {
+  ref_members(q, pi, k, lists, off, [&](uint32_t m) { return PS[m]; }, [&](float4 pj) {
     const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
     const float r2 = rx * rx + ry * ry + rz * rz;
     if (r2 > 0.0f && r2 < k.h2) {
@@ -137,7 +223,7 @@ __global__ void __launch_bounds__(kThreads)
 
 __global__ void __launch_bounds__(kThreads)
     k_rc_delta(const float4 *__restrict__ PS, float4 *__restrict__ PS2,
-               const float *__restrict__ SS, const uint32_t *__restrict__ perm,
+               const float *__restrict__ SS, RefLists lists, const uint32_t *__restrict__ perm,
                const uint32_t *__restrict__ off, const float4 *__restrict__ X,
                float4 *__restrict__ V, float4 *__restrict__ P, float4 *__restrict__ VS,
                uint32_t n, RefConsts k, const SceneDesc *__restrict__ scenes, int last) {
@@ -150,9 +236,9 @@ __global__ void __launch_bounds__(kThreads)
     float4 p;
     float s;
   };
-  ref_neighbours(
-      q, pi, k, off, [&](uint32_t m) { return PSl{__ldg(&PS[m]), __ldg(&SS[m])}; },
-      [&](uint32_t, const PSl &d) {
+  ref_members(
+      q, pi, k, lists, off, [&](uint32_t m) { return PSl{__ldg(&PS[m]), __ldg(&SS[m])}; },
+      [&](const PSl &d) {
     const float4 pj = d.p;
     const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
     const float r2 = rx * rx + ry * ry + rz * rz;
@@ -182,7 +268,7 @@ __global__ void __launch_bounds__(kThreads)
   const float4 np = make_float4(pi.x + dx, pi.y + dy, pi.z + dz, pi.w);
   PS2[q] = np;
   if (last) {
-    const uint32_t i = min(perm[q], n - 1u);
+    const uint32_t i = rc_input(perm, q, n);
     P[i] = np;
     // updateVelocities
     const float4 x = X[i];
@@ -197,18 +283,22 @@ __global__ void __launch_bounds__(kThreads)
 
 __global__ void __launch_bounds__(kThreads)
     k_rc_xsph(const float4 *__restrict__ PS, const float4 *__restrict__ VS,
-              float4 *__restrict__ DV, const uint32_t *__restrict__ perm,
+              float4 *__restrict__ DV, RefLists lists, const uint32_t *__restrict__ perm,
               const uint32_t *__restrict__ off, uint32_t n, RefConsts k) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const float4 pi = PS[q];
   const float4 vi = VS[q];
   float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-  ref_neighbours(q, pi, k, off, [&](uint32_t m) { return __ldg(&PS[m]); }, [&](uint32_t m, float4 pj) {
+  struct PV {
+    float4 p, v;
+  };
+  ref_members(q, pi, k, lists, off, [&](uint32_t m) { return PV{__ldg(&PS[m]), __ldg(&VS[m])}; },
+              [&](const PV &d) {
+    const float4 pj = d.p, vj = d.v;
     const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
     const float r2 = rx * rx + ry * ry + rz * rz;
     if (r2 > 0.0f && r2 < k.h2) {
-      const float4 vj = __ldg(&VS[m]);
       const float vx = vj.x - vi.x, vy = vj.y - vi.y, vz = vj.z - vi.z;
       const float poly = k.poly6 * (k.h2 - r2) * (k.h2 - r2) * (k.h2 - r2);
       const float inv = 1.0f / pj.w;
@@ -217,7 +307,7 @@ __global__ void __launch_bounds__(kThreads)
       sz += inv * vz * poly;
     }
   });
-  DV[min(perm[q], n - 1u)] = make_float4(0.01f * sx, 0.01f * sy, 0.01f * sz, 0.0f);
+  DV[rc_input(perm, q, n)] = make_float4(0.01f * sx, 0.01f * sy, 0.01f * sz, 0.0f);
 }
 
 __global__ void __launch_bounds__(256)
@@ -246,9 +336,23 @@ cudaError_t rc_predict_hash(float4 *X, float4 *V, float4 *P, uint32_t n,
                             const RefConsts &k, const SceneDesc *scenes,
                             uint32_t *keys, const SortPlan &plan,
                             uint32_t *sort_scratch, cudaStream_t st) {
-  k_rc_predict_hash<<<blocks_for(n, 256), 256, 0, st>>>(
+  k_rc_predict_hash<<<min(blocks_for(n, 256), kStrideCtas), 256, 0, st>>>(
       X, V, P, n, k, scenes, keys, plan.passes, plan.digit_bits,
       sort_scratch + plan.off_hist);
+  return cudaGetLastError();
+}
+
+cudaError_t rc_predict_count(float4 *X, float4 *V, float4 *P, uint32_t n, const RefConsts &k,
+                             const SceneDesc *scenes, uint32_t *keys, const CellSortPlan &plan,
+                             uint32_t *cell_scratch, cudaStream_t st) {
+  k_rc_predict_count<<<min(blocks_for(n, 256), kStrideCtas), 256, 0, st>>>(
+      X, V, P, n, k, scenes, keys, cell_scratch + plan.off_counts, cell_scratch + plan.off_pos);
+  return cudaGetLastError();
+}
+
+cudaError_t rc_build(const float4 *PS, const uint32_t *offsets, uint32_t n, const RefConsts &k,
+                     uint32_t maxn, uint4 *nbr, uint32_t *nbr_cnt, cudaStream_t st) {
+  k_rc_build<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, offsets, n, k, maxn, nbr, nbr_cnt);
   return cudaGetLastError();
 }
 
@@ -258,25 +362,26 @@ cudaError_t rc_gather(const float4 *P, const uint32_t *perm, uint32_t n, float4 
   return cudaGetLastError();
 }
 
-cudaError_t rc_lambda(float4 *PS, float *SS, const uint32_t *offsets, uint32_t n,
-                      const RefConsts &k, cudaStream_t st) {
-  k_rc_lambda<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, SS, offsets, n, k);
+cudaError_t rc_lambda(float4 *PS, float *SS, const RefLists &lists, const uint32_t *offsets,
+                      uint32_t n, const RefConsts &k, cudaStream_t st) {
+  k_rc_lambda<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, SS, lists, offsets, n, k);
   return cudaGetLastError();
 }
 
-cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const uint32_t *perm,
+cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const RefLists &lists,
+                     const uint32_t *perm,
                      const uint32_t *offsets, const float4 *X, float4 *V, float4 *P,
                      float4 *VS, uint32_t n, const RefConsts &k, const SceneDesc *scenes,
                      bool last, cudaStream_t st) {
   k_rc_delta<<<blocks_for(n, kThreads), kThreads, 0, st>>>(
-      PS, PS2, SS, perm, offsets, X, V, P, VS, n, k, scenes, last ? 1 : 0);
+      PS, PS2, SS, lists, perm, offsets, X, V, P, VS, n, k, scenes, last ? 1 : 0);
   return cudaGetLastError();
 }
 
-cudaError_t rc_xsph(const float4 *PS, const float4 *VS, float4 *DV, const uint32_t *perm,
-                    const uint32_t *offsets, uint32_t n, const RefConsts &k,
+cudaError_t rc_xsph(const float4 *PS, const float4 *VS, float4 *DV, const RefLists &lists,
+                    const uint32_t *perm, const uint32_t *offsets, uint32_t n, const RefConsts &k,
                     cudaStream_t st) {
-  k_rc_xsph<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, VS, DV, perm, offsets, n, k);
+  k_rc_xsph<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, VS, DV, lists, perm, offsets, n, k);
   return cudaGetLastError();
 }
 

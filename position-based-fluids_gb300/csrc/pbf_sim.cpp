@@ -42,7 +42,11 @@ struct pbf_sim {
   RefConsts rc{};
   SceneDesc scene{};
   SortPlan plan;
-  CellSortPlan cplan;  // paper mode's counting sort
+  CellSortPlan cplan;  // counting sort by cell
+  // ref-compat: counting sort (radix on grids of mostly empty cells) and the
+  // neighbour lists' capacity (0: no lists, every pass walks the cells)
+  bool rc_count_sort = false;
+  uint32_t rc_maxn = 0;
   uint32_t ncells = 0;
   std::vector<void *> allocations;
   size_t device_bytes = 0;
@@ -212,8 +216,6 @@ int launch_step(pbf_sim *s) {
     PBF_TRY_STATUS(mark(s, 0, "sort_onesweep", 1 + passes, &ev));
     PBF_TRY(step_offsets(s));
     PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
-  } else {
-    PBF_TRY(sort_clear(s->plan, d.sort_scratch, st));
   }
   if (s->paper) {
     PBF_TRY(paper_reorder(d.perm, d.X, d.V, d.ID, n, s->pc, d.X2, d.V2, d.ID2,
@@ -264,28 +266,47 @@ int launch_step(pbf_sim *s) {
       PBF_TRY(join_count_copy(s));
     }
   } else {
-    PBF_TRY(rc_predict_hash(d.X, d.V, d.P, n, s->rc, d.scenes, d.keys, s->plan,
-                            d.sort_scratch, st));
-    PBF_TRY_STATUS(mark(s, 0, "rc_predict_hash", 1, &ev));
-    PBF_TRY(sort_scan(s->plan, d.sort_scratch, st));
-    PBF_TRY(sort_passes(s->plan, d.keys, nullptr, d.skeys, d.perm,
-                        d.sort_scratch, d.err, st));
-    PBF_TRY_STATUS(mark(s, 0, "sort_onesweep", 1 + passes, &ev));
-    PBF_TRY(step_offsets(s));
-    PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
+    if (s->rc_count_sort) {
+      PBF_TRY(cell_sort_clear(s->cplan, d.cell_scratch, false, st));
+      PBF_TRY(rc_predict_count(d.X, d.V, d.P, n, s->rc, d.scenes, d.keys, s->cplan,
+                               d.cell_scratch, st));
+      PBF_TRY_STATUS(mark(s, 0, "rc_predict_hash", 1, &ev));
+      PBF_TRY(cell_sort_finish(s->cplan, d.keys, d.cell_scratch, d.offsets, d.skeys, d.perm,
+                               d.err, st));
+      PBF_TRY_STATUS(mark(s, 0, "cell_sort", cell_sort_launches(), &ev));
+    } else {
+      PBF_TRY(sort_clear(s->plan, d.sort_scratch, st));
+      PBF_TRY(rc_predict_hash(d.X, d.V, d.P, n, s->rc, d.scenes, d.keys, s->plan,
+                              d.sort_scratch, st));
+      PBF_TRY_STATUS(mark(s, 0, "rc_predict_hash", 1, &ev));
+      PBF_TRY(sort_scan(s->plan, d.sort_scratch, st));
+      PBF_TRY(sort_passes(s->plan, d.keys, nullptr, d.skeys, d.perm, d.sort_scratch, d.err, st));
+      PBF_TRY_STATUS(mark(s, 0, "sort_onesweep", 1 + passes, &ev));
+      PBF_TRY(step_offsets(s));
+      PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
+    }
     PBF_TRY(rc_gather(d.P, d.perm, n, d.PS, st));
     PBF_TRY_STATUS(mark(s, 0, "rc_gather", 1, &ev));
+    const RefLists lists{d.nbr, d.nbr_cnt, n, s->rc_maxn};
     float4 *cur = d.PS, *alt = d.PS2;
     const uint32_t iters = s->prm.solver_iterations;
     for (uint32_t it = 0; it < iters; ++it) {
-      PBF_TRY(rc_lambda(cur, d.SS, d.offsets, n, s->rc, st));
+      if (s->rc_maxn) {
+        PBF_TRY(rc_build(cur, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt, st));
+        PBF_TRY_STATUS(mark(s, 1, "rc_build", 1, &ev));
+      }
+      PBF_TRY(rc_lambda(cur, d.SS, lists, d.offsets, n, s->rc, st));
       PBF_TRY_STATUS(mark(s, 1, "rc_lambda", 1, &ev));
-      PBF_TRY(rc_delta(cur, alt, d.SS, d.perm, d.offsets, d.X, d.V, d.P, d.VS, n, s->rc,
+      PBF_TRY(rc_delta(cur, alt, d.SS, lists, d.perm, d.offsets, d.X, d.V, d.P, d.VS, n, s->rc,
                        d.scenes, it + 1 == iters, st));
       PBF_TRY_STATUS(mark(s, 2, "rc_delta", 1, &ev));
       std::swap(cur, alt);
     }
-    PBF_TRY(rc_xsph(cur, d.VS, d.DV, d.perm, d.offsets, n, s->rc, st));
+    if (s->rc_maxn) {
+      PBF_TRY(rc_build(cur, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt, st));
+      PBF_TRY_STATUS(mark(s, 3, "rc_build", 1, &ev));
+    }
+    PBF_TRY(rc_xsph(cur, d.VS, d.DV, lists, d.perm, d.offsets, n, s->rc, st));
     PBF_TRY_STATUS(mark(s, 3, "rc_xsph", 1, &ev));
     PBF_TRY(rc_commit(d.X, d.V, d.P, d.DV, n, st));
     PBF_TRY_STATUS(mark(s, 3, "rc_commit", 1, &ev));
@@ -341,8 +362,8 @@ int build_graph(pbf_sim *s) {
 // One step with its stage boundaries, captured and launched as a graph.
 int launch_timed_step(pbf_sim *s) {
   // the boundary events exist before the capture (one per mark of a step:
-  // at most 8 outside the solver loop, 2 per iteration)
-  const size_t marks = 16 + 2 * (size_t)s->prm.solver_iterations;
+  // at most 9 outside the solver loop, 3 per iteration)
+  const size_t marks = 16 + 3 * (size_t)s->prm.solver_iterations;
   while (s->events.size() < marks) {
     cudaEvent_t e;
     PBF_TRY(cudaEventCreate(&e));
@@ -391,7 +412,59 @@ int collect_times(pbf_sim *s) {
   return PBF_OK;
 }
 
+// Neighbour lists of the reference-equation passes: max_neighbours entries
+// per particle (8 to 128), halved until they take at most half of the free
+// memory; a scene so large that not even 8 entries fit runs without lists.
+int alloc_ref_lists(pbf_sim *s) {
+  size_t free_bytes = 0, total = 0;
+  PBF_TRY(cudaMemGetInfo(&free_bytes, &total));
+  uint32_t maxn = std::min(128u, std::max(8u, s->prm.max_neighbours / 8u * 8u));
+  s->rc_maxn = 0;
+  for (; maxn >= 8u; maxn = maxn / 16u * 8u) {
+    const size_t count = (size_t)paper_list_words(maxn) * s->n;
+    if (count * sizeof(uint4) > free_bytes / 2) continue;
+    if (dalloc(s, &s->d.nbr, count) == PBF_OK) {
+      s->rc_maxn = maxn;
+      return PBF_OK;
+    }
+    cudaGetLastError();  // try fewer entries
+  }
+  return PBF_OK;
+}
+
 bool ready(const pbf_sim *s) { return s && s->inited; }
+
+// pbf_get_cells in REF_COMPAT mode, in the reference's numbering (x fastest,
+// ties by input index): the step's own structure numbers the cells with z
+// fastest and runs over descending input index, so the views are counted out
+// here from each particle's cell.
+int ref_cells(pbf_sim *s, uint32_t *hash, uint32_t *perm, int32_t *ranges) {
+  const size_t n = s->n;
+  std::vector<uint32_t> key(n);
+  PBF_TRY(cudaMemcpyAsync(key.data(), s->d.keys, n * 4, cudaMemcpyDeviceToHost, s->stream));
+  PBF_TRY(cudaStreamSynchronize(s->stream));
+  std::reverse(key.begin(), key.end());
+  const uint32_t nx = (uint32_t)s->scene.ncell[0], ny = (uint32_t)s->scene.ncell[1],
+                 nz = (uint32_t)s->scene.ncell[2];
+  for (uint32_t &k : key) {
+    const uint32_t z = k % nz, y = k / nz % ny, x = k / nz / ny;
+    k = x + nx * (y + ny * z);
+  }
+  if (hash) std::memcpy(hash, key.data(), n * 4);
+  if (!perm && !ranges) return PBF_OK;
+  std::vector<uint32_t> start((size_t)s->ncells + 1, 0u);
+  for (const uint32_t k : key) ++start[(size_t)k + 1];
+  for (size_t c = 0; c < s->ncells; ++c) start[c + 1] += start[c];
+  if (ranges)
+    for (size_t c = 0; c < s->ncells; ++c) {
+      const bool any = start[c] < start[c + 1];
+      ranges[2 * c] = any ? (int32_t)start[c] : -1;
+      ranges[2 * c + 1] = any ? (int32_t)start[c + 1] - 1 : -1;
+    }
+  if (perm)
+    for (size_t i = 0; i < n; ++i) perm[start[key[i]]++] = (uint32_t)i;
+  return PBF_OK;
+}
 
 // Largest list capacity (pbf_params.max_neighbours range).
 constexpr uint32_t kMaxListCapacity = 1024;
@@ -478,6 +551,9 @@ int pbf_init(pbf_sim *s) {
   A(&d.perm, n);
   A(&d.offsets, (size_t)s->ncells + 1);
   s->offset_runs = (uint64_t)s->ncells * 2u >= (uint64_t)n;
+  // The counting sort's passes over the cells outweigh the radix sort's over
+  // the keys once most cells are empty.
+  s->rc_count_sort = !s->paper && (uint64_t)s->ncells <= 4u * (uint64_t)n + (1u << 16);
   if (s->offset_runs) {
     A(&d.runs, offset_runs_capacity(s->ncells));
     A(&d.runs_count, 1);
@@ -511,6 +587,9 @@ int pbf_init(pbf_sim *s) {
     A(&d.VS, n);
     A(&d.DV, n);
     A(&d.SS, n);
+    A(&d.nbr_cnt, n);
+    if (s->rc_count_sort) A(&d.cell_scratch, s->cplan.words);
+    if (rc == PBF_OK) rc = alloc_ref_lists(s);
   }
   if (rc == PBF_OK && s->paper) {
     cudaError_t te = tile_init();
@@ -535,7 +614,8 @@ int pbf_init(pbf_sim *s) {
     vel[i] = make_float4(p.v[0], p.v[1], p.v[2], p.m);
   }
   PBF_TRY(cudaMemsetAsync(d.err, 0, sizeof(uint32_t), s->stream));
-  if (s->paper) PBF_TRY(cell_sort_clear(s->cplan, d.cell_scratch, true, s->stream));
+  if (s->paper || s->rc_count_sort)
+    PBF_TRY(cell_sort_clear(s->cplan, d.cell_scratch, true, s->stream));
   PBF_TRY(cudaMemsetAsync(d.P, 0, n * sizeof(float4), s->stream));
   PBF_TRY(cudaMemsetAsync(d.offsets, 0, ((size_t)s->ncells + 1) * sizeof(uint32_t),
                           s->stream));
@@ -719,14 +799,14 @@ int pbf_set_graph(pbf_sim *s, int enable) {
 int pbf_launches_per_step(const pbf_sim *s, uint32_t *launches) {
   if (!s || !launches) return PBF_ERR_INVALID;
   const uint32_t it = s->prm.solver_iterations;
-  const uint32_t sort = s->paper && !s->d.tune.radix_sort
+  const uint32_t sort = (s->paper ? !s->d.tune.radix_sort : s->rc_count_sort)
                             ? cell_sort_launches()
                             : 1u /*scan*/ + s->plan.passes + (s->offset_runs ? 2u : 1u) /*offsets*/;
   if (s->paper)
     *launches = 1u /*predict+hash*/ + sort + 1u /*reorder*/ + paper_first_launches(s->d) +
                 2u * it - 1u + 2u;
   else
-    *launches = 1u + sort + 1u /*gather*/ + 2u * it + 2u;
+    *launches = 1u + sort + 1u /*gather*/ + 2u * it + 2u + (s->rc_maxn ? it + 1u : 0u);
   return PBF_OK;
 }
 
@@ -824,12 +904,10 @@ int pbf_get_cells(pbf_sim *s, uint32_t *hash, uint32_t *perm, int32_t *ranges) {
   if (!ready(s)) return PBF_ERR_STATE;
   if (!s->stepped) return PBF_ERR_STATE;
   const size_t n = s->n;
-  std::vector<uint32_t> skeys(n), p(n), id(n);
+  if (!s->paper) return ref_cells(s, hash, perm, ranges);
+  std::vector<uint32_t> skeys(n), p(n);
   PBF_TRY(cudaMemcpyAsync(skeys.data(), s->d.skeys, n * 4, cudaMemcpyDeviceToHost, s->stream));
-  PBF_TRY(cudaMemcpyAsync(p.data(), s->paper ? s->d.ID : s->d.perm, n * 4,
-                          cudaMemcpyDeviceToHost, s->stream));
-  if (!s->paper && hash)
-    PBF_TRY(cudaMemcpyAsync(hash, s->d.keys, n * 4, cudaMemcpyDeviceToHost, s->stream));
+  PBF_TRY(cudaMemcpyAsync(p.data(), s->d.ID, n * 4, cudaMemcpyDeviceToHost, s->stream));
   if (ranges) {
     if (!s->d_ranges) PBF_TRY_STATUS(dalloc(s, &s->d_ranges, 2 * (size_t)s->ncells));
     PBF_TRY(find_cells(s->d.offsets, s->ncells, s->d_ranges, s->stream));
@@ -837,7 +915,7 @@ int pbf_get_cells(pbf_sim *s, uint32_t *hash, uint32_t *perm, int32_t *ranges) {
                             cudaMemcpyDeviceToHost, s->stream));
   }
   PBF_TRY(cudaStreamSynchronize(s->stream));
-  if (s->paper && hash)
+  if (hash)
     for (size_t q = 0; q < n; ++q) hash[p[q]] = skeys[q];
   if (perm) std::memcpy(perm, p.data(), n * 4);
   return PBF_OK;
