@@ -154,7 +154,7 @@ int launch_batch_step(pbf_batch *b) {
     PBF_TRY(sort_passes(b->plan, d.keys, nullptr, d.skeys, d.perm, d.sort_scratch, d.err, st));
     PBF_TRY(cell_offsets_runs(d.skeys, n, b->cells_total, d.offsets, d.runs, d.runs_count, st));
   }
-  PBF_TRY(paper_reorder(d.perm, d.X, d.V, d.ID, n, pc, d.X2, d.V2, d.ID2, d.P, d.D, st));
+  PBF_TRY(paper_reorder(d.perm, d.X, d.V, d.ID, n, pc, d.X2, d.V2, d.ID2, d.P, d.D, d.W, st));
   const uint32_t iters = b->solver.solver_iterations;
   if (d.tune.staged) {
     PBF_TRY(tile_plan(d, pc, d.sid, (uint32_t)b->scenes.size(), st));
@@ -272,7 +272,7 @@ int pbf_batch_create(const pbf_params *solver, uint32_t max_scenes, uint32_t max
     if (rc == PBF_OK) rc = balloc(b.get(), p, count);
   };
   A(&d.X, M); A(&d.V, M); A(&d.X2, M); A(&d.V2, M); A(&d.P, M); A(&d.Q, M);
-  A(&d.D, M); A(&d.U, M); A(&d.W, M); A(&d.S, M);
+  A(&d.D, M); A(&d.U, M); A(&d.W, std::max(M, kMinPlaneSlots)); A(&d.S, M);
   A(&d.ID, M); A(&d.ID2, M); A(&d.keys, M); A(&d.skeys, M); A(&d.perm, M);
   A(&d.nbr_cnt, M); A(&d.R, M); A(&d.sid, M);
   A(&d.nbr, (size_t)paper_list_words(b->pc.maxn) * M);

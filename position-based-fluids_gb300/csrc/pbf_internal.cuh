@@ -400,10 +400,18 @@ cudaError_t paper_predict_count(const float4 *X, const float4 *V, uint32_t n,
                                 const uint16_t *sid, uint32_t *keys,
                                 const CellSortPlan &plan, uint32_t *cell_scratch,
                                 cudaStream_t st);
+// The list builds read the step-start positions as three planes of
+// plane_floats(n) values (whole 16-byte words).  They live in an array of n
+// float4 that the step only writes later (the vorticity in paper mode, the
+// XSPH velocity change in ref-compat mode), of at least kMinPlaneSlots slots
+// so that the padding of small scenes fits.
+PBF_HOST_DEVICE inline uint32_t plane_floats(uint32_t n) { return (n + 3u) & ~3u; }
+constexpr size_t kMinPlaneSlots = 16;
 cudaError_t paper_reorder(const uint32_t *perm, const float4 *X,
                           const float4 *V, const uint32_t *ID, uint32_t n,
                           const PaperConsts &c, float4 *X2, float4 *V2,
-                          uint32_t *ID2, float4 *P, float4 *D, cudaStream_t st);
+                          uint32_t *ID2, float4 *P, float4 *D, float4 *planes,
+                          cudaStream_t st);
 // Neighbour lists of the step (from the predicted positions P).
 cudaError_t paper_nbr_build(const DeviceState &d, const PaperConsts &c,
                             const uint16_t *sid, cudaStream_t st);
@@ -457,11 +465,13 @@ cudaError_t rc_predict_count(float4 *X, float4 *V, float4 *P, uint32_t n, const 
                              const SceneDesc *scenes, uint32_t *keys, const CellSortPlan &plan,
                              uint32_t *cell_scratch, cudaStream_t st);
 // PS[m] = P of the particle in slot m: the predicted positions by slot.
+// The build reads the positions as planes (plane_floats above).
 cudaError_t rc_gather(const float4 *P, const uint32_t *perm, uint32_t n, float4 *PS,
-                      cudaStream_t st);
+                      float4 *planes, cudaStream_t st);
 // Neighbour lists of the positions PS.
-cudaError_t rc_build(const float4 *PS, const uint32_t *offsets, uint32_t n, const RefConsts &k,
-                     uint32_t maxn, uint4 *nbr, uint32_t *nbr_cnt, cudaStream_t st);
+cudaError_t rc_build(const float4 *PS, const float4 *planes, const uint32_t *offsets, uint32_t n,
+                     const RefConsts &k, uint32_t maxn, uint4 *nbr, uint32_t *nbr_cnt,
+                     cudaStream_t st);
 // The passes read neighbours by sorted slot (PS, SS, VS) and write their own
 // slot's values there; the last delta-p pass also writes P and V by input
 // index for the commit.
@@ -469,8 +479,8 @@ cudaError_t rc_lambda(float4 *PS, float *SS, const RefLists &lists, const uint32
                       uint32_t n, const RefConsts &k, cudaStream_t st);
 cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const RefLists &lists,
                      const uint32_t *perm, const uint32_t *offsets, const float4 *X, float4 *V,
-                     float4 *P, float4 *VS, uint32_t n, const RefConsts &k,
-                     const SceneDesc *scenes, bool last, cudaStream_t st);
+                     float4 *P, float4 *VS, float4 *planes, uint32_t n,
+                     const RefConsts &k, const SceneDesc *scenes, bool last, cudaStream_t st);
 cudaError_t rc_xsph(const float4 *PS, const float4 *VS, float4 *DV, const RefLists &lists,
                     const uint32_t *perm, const uint32_t *offsets, uint32_t n,
                     const RefConsts &k, cudaStream_t st);

@@ -123,7 +123,8 @@ __global__ void __launch_bounds__(256)
               const float4 *__restrict__ V, const uint32_t *__restrict__ ID,
               uint32_t n, PaperConsts c, float4 *__restrict__ X2,
               float4 *__restrict__ V2, uint32_t *__restrict__ ID2,
-              float4 *__restrict__ P, float4 *__restrict__ D) {
+              float4 *__restrict__ P, float4 *__restrict__ D, float *__restrict__ planes,
+              uint32_t plane) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   // perm is a permutation of [0, n) unless the sort reported an error.
@@ -137,73 +138,82 @@ __global__ void __launch_bounds__(256)
   ID2[k] = ID[src];
   P[k] = make_float4(p.x, p.y, p.z, 0.0f);
   D[k] = make_float4(d.x, d.y, d.z, 0.0f);
+  planes[k] = p.x;
+  planes[plane + k] = p.y;
+  planes[2 * (size_t)plane + k] = p.z;
 }
 
 // Neighbour-list build from the predicted positions P (which equal the
-// step-start positions the fallback recomputes).  Each member's slot is
-// stored straight into its list word; the rest of the last word holds the
-// particle's own slot.  kMasked: the candidates of each row are tested into
-// a membership mask first and the members stored from it afterwards
-// (scan_members_masked); the same lists either way.
+// step-start positions the fallback recomputes).  kMasked: the members come
+// from row masks over the position planes and reach the list in whole words;
+// otherwise each member's slot is stored as it is found.  The same lists
+// either way; the rest of the last word holds the particle's own slot.
 template <int kBlock, bool kMasked>
 __global__ void __launch_bounds__(kBlock)
-    k_nbr_build(const float4 *__restrict__ P, NbrCtx nc, PaperConsts c,
+    k_nbr_build(const float4 *__restrict__ P, Planes planes, NbrCtx nc, PaperConsts c,
                 uint4 *__restrict__ nbr4, uint32_t *__restrict__ nbr_cnt) {
   const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
   if (k >= c.n) return;
   const float4 pk = P[k];
-  uint32_t *__restrict__ out = reinterpret_cast<uint32_t *>(nbr4) + 4ull * k;
-  const size_t stride = 4ull * c.n;  // words from one list group to the next
   uint32_t cnt = 0;
-  const auto store = [&](uint32_t j) {
-    if (cnt < c.maxn) out[(size_t)(cnt >> 2) * stride + (cnt & 3u)] = j;
-    ++cnt;
-  };
   const SceneDesc &sc = scene_of(nc.scenes, nc.sid, k);
-  if constexpr (kMasked)
-    scan_members_masked(pk, nc.skeys[k], sc, nc.off, P, c, store);
-  else
-    scan_members(pk, nc.skeys[k], sc, nc.off, P, c, [&](uint32_t j, const Sep &) { store(j); });
-  pad_list(out, stride, cnt, c.maxn, k);
+  if constexpr (kMasked) {
+    cnt = scan_members_planes(
+        pk, k, nc.skeys[k], sc, nc.off, planes, c,
+        [&](uint32_t w, const uint4 &j) {
+          if (4u * w < c.maxn) nbr4[(size_t)w * c.n + k] = j;
+        });
+  } else {
+    uint32_t *__restrict__ out = reinterpret_cast<uint32_t *>(nbr4) + 4ull * k;
+    const size_t stride = 4ull * c.n;  // words from one list group to the next
+    scan_members(pk, nc.skeys[k], sc, nc.off, P, c, [&](uint32_t j, const Sep &) {
+      if (cnt < c.maxn) out[(size_t)(cnt >> 2) * stride + (cnt & 3u)] = j;
+      ++cnt;
+    });
+    pad_list(out, stride, cnt, c.maxn, k);
+  }
   nbr_cnt[k] = cnt;
   record_count(nc.cnt_max, cnt);
 }
 
 // k_nbr_build fused with the first lambda pass: the same lists, and lambda
 // summed over the members in the order the lists store them -- the bits
-// k_lambda computes from the lists.  (In one kernel a warp executes the
-// lambda arithmetic whenever any of its lanes has a member, so which form is
-// faster depends on the scene; the tuner picks.)  kMasked: the members come
-// from row masks (scan_members_masked) and each member's separation is
-// evaluated again from its position, the same operations on the same values.
+// k_lambda computes from the lists.  kMasked sums each list word as it is
+// handed on, four members' positions in flight, as k_lambda does (the scan
+// and the sums then both run with most lanes of a warp busy); otherwise a
+// warp executes the lambda arithmetic whenever any of its lanes has a member.
+// Which of this and the split passes is faster depends on the scene; the
+// tuner picks.
 template <int kBlock, bool kMasked>
 __global__ void __launch_bounds__(kBlock)
-    k_nbr_lambda(const float4 *__restrict__ P, NbrCtx nc, PaperConsts c,
+    k_nbr_lambda(const float4 *__restrict__ P, Planes planes, NbrCtx nc, PaperConsts c,
                  uint4 *__restrict__ nbr4, uint32_t *__restrict__ nbr_cnt,
                  float4 *__restrict__ Q, float *__restrict__ R) {
   const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
   if (k >= c.n) return;
   const float4 pk = P[k];
-  uint32_t *__restrict__ out = reinterpret_cast<uint32_t *>(nbr4) + 4ull * k;
-  const size_t stride = 4ull * c.n;  // words from one list group to the next
   uint32_t cnt = 0;
   LambdaAcc acc{c.w_self, 0.f, 0.f, 0.f, 0.f};
-  const auto store = [&](uint32_t j) {
-    if (cnt < c.maxn) out[(size_t)(cnt >> 2) * stride + (cnt & 3u)] = j;
-    ++cnt;
-  };
   const SceneDesc &sc = scene_of(nc.scenes, nc.sid, k);
-  if constexpr (kMasked)
-    scan_members_masked(pk, nc.skeys[k], sc, nc.off, P, c, [&](uint32_t j) {
-      store(j);
-      acc.add(separation(pk, __ldg(&P[j])), c);
-    });
-  else
+  if constexpr (kMasked) {
+    cnt = scan_members_planes(
+        pk, k, nc.skeys[k], sc, nc.off, planes, c,
+        [&](uint32_t w, const uint4 &j) {
+          if (4u * w < c.maxn) nbr4[(size_t)w * c.n + k] = j;
+          const float4 d[4] = {__ldg(&P[j.x]), __ldg(&P[j.y]), __ldg(&P[j.z]), __ldg(&P[j.w])};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) lambda_pair(acc, pk, d[e], c);
+        });
+  } else {
+    uint32_t *__restrict__ out = reinterpret_cast<uint32_t *>(nbr4) + 4ull * k;
+    const size_t stride = 4ull * c.n;  // words from one list group to the next
     scan_members(pk, nc.skeys[k], sc, nc.off, P, c, [&](uint32_t j, const Sep &r) {
-      store(j);
+      if (cnt < c.maxn) out[(size_t)(cnt >> 2) * stride + (cnt & 3u)] = j;
+      ++cnt;
       acc.add(r, c);
     });
-  pad_list(out, stride, cnt, c.maxn, k);
+    pad_list(out, stride, cnt, c.maxn, k);
+  }
   nbr_cnt[k] = cnt;
   record_count(nc.cnt_max, cnt);
   Q[k] = make_float4(pk.x, pk.y, pk.z, acc.lambda(c));
@@ -335,6 +345,11 @@ inline uint32_t blocks_for(uint64_t n, uint32_t t) {
   return (uint32_t)((n + t - 1) / t);
 }
 
+Planes make_planes(const float4 *planes, uint32_t n) {
+  const size_t words = plane_floats(n) / 4u;
+  return Planes{planes, planes + words, planes + 2 * words};
+}
+
 NbrCtx make_ctx(const DeviceState &d, const PaperConsts &c, const uint16_t *sid) {
   NbrCtx nc;
   nc.nbr4 = d.nbr;
@@ -381,9 +396,11 @@ cudaError_t paper_predict_count(const float4 *X, const float4 *V, uint32_t n,
 cudaError_t paper_reorder(const uint32_t *perm, const float4 *X,
                           const float4 *V, const uint32_t *ID, uint32_t n,
                           const PaperConsts &c, float4 *X2, float4 *V2,
-                          uint32_t *ID2, float4 *P, float4 *D,
+                          uint32_t *ID2, float4 *P, float4 *D, float4 *planes,
                           cudaStream_t st) {
-  k_reorder<<<blocks_for(n, 256), 256, 0, st>>>(perm, X, V, ID, n, c, X2, V2, ID2, P, D);
+  k_reorder<<<blocks_for(n, 256), 256, 0, st>>>(perm, X, V, ID, n, c, X2, V2, ID2, P, D,
+                                                reinterpret_cast<float *>(planes),
+                                                plane_floats(n));
   return cudaGetLastError();
 }
 
@@ -422,14 +439,14 @@ cudaError_t paper_reorder(const uint32_t *perm, const float4 *X,
 
 cudaError_t paper_nbr_build(const DeviceState &d, const PaperConsts &c,
                             const uint16_t *sid, cudaStream_t st) {
-  PBF_BUILD_LAUNCH(k_nbr_build, kKindNbr, d.P, make_ctx(d, c, sid), c, d.nbr, d.nbr_cnt);
+  PBF_BUILD_LAUNCH(k_nbr_build, kKindNbr, d.P, make_planes(d.W, c.n), make_ctx(d, c, sid), c, d.nbr, d.nbr_cnt);
   return cudaGetLastError();
 }
 
 cudaError_t paper_nbr_lambda(const DeviceState &d, const PaperConsts &c,
                              const uint16_t *sid, cudaStream_t st) {
-  PBF_BUILD_LAUNCH(k_nbr_lambda, kKindNbrLambda, d.P, make_ctx(d, c, sid), c, d.nbr, d.nbr_cnt,
-                   d.Q, d.R);
+  PBF_BUILD_LAUNCH(k_nbr_lambda, kKindNbrLambda, d.P, make_planes(d.W, c.n), make_ctx(d, c, sid),
+                   c, d.nbr, d.nbr_cnt, d.Q, d.R);
   return cudaGetLastError();
 }
 

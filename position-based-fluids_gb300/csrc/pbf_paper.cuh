@@ -64,8 +64,9 @@ __device__ __forceinline__ float3 start_position(const NbrCtx &c, uint32_t j) {
 // Particles j != k closer than h form a pair.  Distances below
 // sqrt(FLT_MIN) ~ 1.1e-19 count as coincident (like r = 0, whose direction
 // is undefined), so r^2 is a normal number wherever a kernel is evaluated.
+constexpr float kMinPair2 = 1.17549435e-38f;
 __device__ __forceinline__ bool is_pair(float r2, float h2) {
-  return r2 >= 1.17549435e-38f && r2 < h2;
+  return r2 >= kMinPair2 && r2 < h2;
 }
 
 // All arithmetic on pair and particle values below is written with
@@ -257,21 +258,19 @@ __device__ __forceinline__ void scan_members(const float4 &pk, uint32_t key, con
   }
 }
 
-// scan_members with the member work taken out of the candidate loop: each
-// row is tested 32 candidates at a time into a membership mask (bit e for
-// candidate c0 + e), then member(j) runs for the mask's set bits in
-// ascending order -- the same members in the same order as scan_members.
-// Lanes of a warp test candidates of different cells, so in scan_members
-// the member branch runs for nearly every candidate (some lane of the warp
-// has a member); here the candidate loop is the load, the distance and one
-// bit in every lane, and the member work runs as many times per chunk as
-// the warp's largest member count in it.
-template <typename F>
-__device__ __forceinline__ void scan_members_masked(const float4 &pk, uint32_t key,
-                                                    const SceneDesc &s,
-                                                    const uint32_t *__restrict__ off,
-                                                    const float4 *__restrict__ P,
-                                                    const PaperConsts &c, F &&member) {
+// The same members in the same order, found as masks: each row is tested up
+// to 32 candidates at a time from the position planes, and the masks' members
+// reach word(w, slots) in whole list words.  Returns the number of members.  Only the row of k's own cell can
+// hold k itself or a coincident particle, so only there r^2 is tested against
+// zero as well.  The candidate loop is 23 instructions per four candidates
+// (12 of them packed), where one candidate at a time with its member work
+// inside took about 18 each.
+template <typename Word>
+__device__ __forceinline__ uint32_t scan_members_planes(const float4 &pk, uint32_t k, uint32_t key,
+                                                        const SceneDesc &s,
+                                                        const uint32_t *__restrict__ off,
+                                                        const Planes &planes,
+                                                        const PaperConsts &c, Word &&word) {
   const int nx = s.ncell[0], ny = s.ncell[1], nz = s.ncell[2];
   const uint32_t local = key - s.cell_base;
   const int cx = (int)(local % (uint32_t)nx);
@@ -280,6 +279,10 @@ __device__ __forceinline__ void scan_members_masked(const float4 &pk, uint32_t k
   const int cz = (int)(t / (uint32_t)ny);
   const int x0 = cx > 0 ? cx - 1 : 0;
   const int x1 = cx + 1 < nx ? cx + 1 : nx - 1;
+  const float2 px = make_float2(-pk.x, -pk.x), py = make_float2(-pk.y, -pk.y),
+               pz = make_float2(-pk.z, -pk.z);
+  MaskQueue<kMaskQueue> list;
+  uint32_t cnt = 0;
   for (int dz = -1; dz <= 1; ++dz) {
     const int z = cz + dz;
     if (z < 0 || z >= nz) continue;
@@ -289,10 +292,18 @@ __device__ __forceinline__ void scan_members_masked(const float4 &pk, uint32_t k
       const uint32_t row = s.cell_base + (uint32_t)nx * ((uint32_t)y + (uint32_t)ny * (uint32_t)z);
       const uint32_t a = __ldg(&off[row + x0]);
       const uint32_t b = __ldg(&off[row + x1 + 1]);
-      scan_row_masked(
-          P, a, b, [&](const float4 &d) { return is_pair(separation(pk, d).r2, c.h2); }, member);
+      const bool own = (dz | dy) == 0;
+      for (uint32_t c0 = a & ~3u; c0 < b; c0 += 32u) {
+        const uint32_t m =
+            own ? row_mask<PaperDistance, true>(planes, c0, a, b, px, py, pz, kMinPair2, c.h2)
+                : row_mask<PaperDistance, false>(planes, c0, a, b, px, py, pz, 0.f, c.h2);
+        cnt += (uint32_t)__popc(m);
+        list.add(m, c0, word);
+      }
     }
   }
+  list.finish(k, word);
+  return cnt;
 }
 
 // ------------------------------------------------------------ pair terms --

@@ -27,7 +27,8 @@
 // every pass scanning the 27 cells itself, a warp ran the pair arithmetic
 // (square roots and divisions) for nearly every one of ~216 candidates with
 // 15 of 32 lanes active: 572, 537 and 443 us per lambda, delta-p and XSPH
-// pass at 1,048,576 particles.  A particle with more members than the list
+// pass at 1,048,576 particles, against 157 us per build and 117, 110 and 119 us
+// per pass over the lists.  A particle with more members than the list
 // holds walks the cells in every pass instead.
 #include "pbf_lists.cuh"
 
@@ -57,12 +58,8 @@ __device__ __forceinline__ void ref_rows(float4 p, const RefConsts &k,
     }
 }
 
-// The reference's pair test on its r^2 (rounded operation by operator).
-__device__ __forceinline__ bool ref_pair(const float4 &pi, const float4 &pj, float h2) {
-  const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
-  const float r2 = rx * rx + ry * ry + rz * rz;
-  return r2 > 0.0f && r2 < h2;
-}
+// r^2 > 0 as a lower bound: the smallest positive binary32 number.
+constexpr float kDenormMin = 1.40129846e-45f;
 
 // Calls f(load(m)) for the members of slot q in visiting order (and for q
 // itself as padding, which the pair test drops): from the list, or over all
@@ -89,6 +86,13 @@ __device__ __forceinline__ uint32_t rc_cell(float x, float y, float z, const Sce
   const int cz = axis_cell(z, s.gmin[2], s.clen[2], s.ncell[2]);
   return (uint32_t)cz +
          (uint32_t)s.ncell[2] * ((uint32_t)cy + (uint32_t)s.ncell[1] * (uint32_t)cx);
+}
+
+__device__ __forceinline__ void store_planes(float *__restrict__ planes, uint32_t plane,
+                                             uint32_t q, const float4 &p) {
+  planes[q] = p.x;
+  planes[plane + q] = p.y;
+  planes[2 * (size_t)plane + q] = p.z;
 }
 
 // Input index of sorted slot q (perm is a permutation of [0, n) unless the
@@ -159,35 +163,41 @@ __global__ void __launch_bounds__(256)
 
 __global__ void __launch_bounds__(256)
     k_rc_gather(const float4 *__restrict__ P, const uint32_t *__restrict__ perm, uint32_t n,
-                float4 *__restrict__ PS) {
+                float4 *__restrict__ PS, float *__restrict__ planes, uint32_t plane) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
-  PS[q] = P[rc_input(perm, q, n)];
+  const float4 p = P[rc_input(perm, q, n)];
+  PS[q] = p;
+  store_planes(planes, plane, q, p);
 }
 
-// Neighbour lists of the current positions in visiting order; the rest of
-// the last word holds the particle's own slot.  A set that outgrows the list
-// ends the scan: its passes walk the cells.
+// Neighbour lists of the current positions in visiting order, from row masks
+// over the position planes; the rest of the last word holds the particle's
+// own slot.  A set that outgrows the list ends the scan: its passes walk the
+// cells.  (The particle itself and coincident ones can sit in any row here:
+// the cells are the step start's, the rows follow the current position.)
 __global__ void __launch_bounds__(kThreads)
-    k_rc_build(const float4 *__restrict__ PS, const uint32_t *__restrict__ off, uint32_t n,
-               RefConsts k, uint32_t maxn, uint4 *__restrict__ nbr4,
+    k_rc_build(const float4 *__restrict__ PS, Planes planes, const uint32_t *__restrict__ off,
+               uint32_t n, RefConsts k, uint32_t maxn, uint4 *__restrict__ nbr4,
                uint32_t *__restrict__ nbr_cnt) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const float4 pi = PS[q];
-  uint32_t *__restrict__ out = reinterpret_cast<uint32_t *>(nbr4) + 4ull * q;
-  const size_t stride = 4ull * n;  // words from one list group to the next
+  const float2 px = make_float2(-pi.x, -pi.x), py = make_float2(-pi.y, -pi.y),
+               pz = make_float2(-pi.z, -pi.z);
+  MaskQueue<kMaskQueue> list;
+  const auto word = [&](uint32_t w, const uint4 &j) {
+    if (4u * w < maxn) nbr4[(size_t)w * n + q] = j;
+  };
   uint32_t cnt = 0;
   ref_rows(pi, k, off, [&](uint32_t a, uint32_t b) {
-    if (cnt > maxn) return;
-    scan_row_masked(
-        PS, a, b, [&](const float4 &pj) { return ref_pair(pi, pj, k.h2); },
-        [&](uint32_t m) {
-          if (cnt < maxn) out[(size_t)(cnt >> 2) * stride + (cnt & 3u)] = m;
-          ++cnt;
-        });
+    for (uint32_t c0 = a & ~3u; c0 < b && cnt <= maxn; c0 += 32u) {
+      const uint32_t m = row_mask<RefDistance, true>(planes, c0, a, b, px, py, pz, kDenormMin, k.h2);
+      cnt += (uint32_t)__popc(m);
+      list.add(m, c0, word);
+    }
   });
-  pad_list(out, stride, cnt, maxn, q);
+  list.finish(q, word);
   nbr_cnt[q] = cnt;
 }
 
@@ -226,7 +236,8 @@ __global__ void __launch_bounds__(kThreads)
                const float *__restrict__ SS, RefLists lists, const uint32_t *__restrict__ perm,
                const uint32_t *__restrict__ off, const float4 *__restrict__ X,
                float4 *__restrict__ V, float4 *__restrict__ P, float4 *__restrict__ VS,
-               uint32_t n, RefConsts k, const SceneDesc *__restrict__ scenes, int last) {
+               float *__restrict__ planes, uint32_t plane, uint32_t n, RefConsts k,
+               const SceneDesc *__restrict__ scenes, int last) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const float4 pi = PS[q];
@@ -267,6 +278,7 @@ __global__ void __launch_bounds__(kThreads)
   const float dx = fx - pi.x, dy = fy - pi.y, dz = fz - pi.z;
   const float4 np = make_float4(pi.x + dx, pi.y + dy, pi.z + dz, pi.w);
   PS2[q] = np;
+  store_planes(planes, plane, q, np);
   if (last) {
     const uint32_t i = rc_input(perm, q, n);
     P[i] = np;
@@ -350,15 +362,21 @@ cudaError_t rc_predict_count(float4 *X, float4 *V, float4 *P, uint32_t n, const 
   return cudaGetLastError();
 }
 
-cudaError_t rc_build(const float4 *PS, const uint32_t *offsets, uint32_t n, const RefConsts &k,
-                     uint32_t maxn, uint4 *nbr, uint32_t *nbr_cnt, cudaStream_t st) {
-  k_rc_build<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, offsets, n, k, maxn, nbr, nbr_cnt);
+cudaError_t rc_build(const float4 *PS, const float4 *planes, const uint32_t *offsets, uint32_t n,
+                     const RefConsts &k, uint32_t maxn, uint4 *nbr, uint32_t *nbr_cnt,
+                     cudaStream_t st) {
+  const size_t words = plane_floats(n) / 4u;
+  const Planes p{planes, planes + words, planes + 2 * words};
+  k_rc_build<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, p, offsets, n, k, maxn, nbr,
+                                                           nbr_cnt);
   return cudaGetLastError();
 }
 
 cudaError_t rc_gather(const float4 *P, const uint32_t *perm, uint32_t n, float4 *PS,
-                      cudaStream_t st) {
-  k_rc_gather<<<blocks_for(n, 256), 256, 0, st>>>(P, perm, n, PS);
+                      float4 *planes, cudaStream_t st) {
+  k_rc_gather<<<blocks_for(n, 256), 256, 0, st>>>(P, perm, n, PS,
+                                                  reinterpret_cast<float *>(planes),
+                                                  plane_floats(n));
   return cudaGetLastError();
 }
 
@@ -371,10 +389,11 @@ cudaError_t rc_lambda(float4 *PS, float *SS, const RefLists &lists, const uint32
 cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const RefLists &lists,
                      const uint32_t *perm,
                      const uint32_t *offsets, const float4 *X, float4 *V, float4 *P,
-                     float4 *VS, uint32_t n, const RefConsts &k, const SceneDesc *scenes,
-                     bool last, cudaStream_t st) {
+                     float4 *VS, float4 *planes, uint32_t n, const RefConsts &k,
+                     const SceneDesc *scenes, bool last, cudaStream_t st) {
   k_rc_delta<<<blocks_for(n, kThreads), kThreads, 0, st>>>(
-      PS, PS2, SS, lists, perm, offsets, X, V, P, VS, n, k, scenes, last ? 1 : 0);
+      PS, PS2, SS, lists, perm, offsets, X, V, P, VS, reinterpret_cast<float *>(planes),
+      plane_floats(n), n, k, scenes, last ? 1 : 0);
   return cudaGetLastError();
 }
 

@@ -219,7 +219,7 @@ int launch_step(pbf_sim *s) {
   }
   if (s->paper) {
     PBF_TRY(paper_reorder(d.perm, d.X, d.V, d.ID, n, s->pc, d.X2, d.V2, d.ID2,
-                          d.P, d.D, st));
+                          d.P, d.D, d.W, st));
     PBF_TRY_STATUS(mark(s, 0, "reorder", 1, &ev));
     const uint32_t iters = s->prm.solver_iterations;
     if (d.tune.staged) {
@@ -285,25 +285,25 @@ int launch_step(pbf_sim *s) {
       PBF_TRY(step_offsets(s));
       PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
     }
-    PBF_TRY(rc_gather(d.P, d.perm, n, d.PS, st));
+    PBF_TRY(rc_gather(d.P, d.perm, n, d.PS, d.DV, st));
     PBF_TRY_STATUS(mark(s, 0, "rc_gather", 1, &ev));
     const RefLists lists{d.nbr, d.nbr_cnt, n, s->rc_maxn};
     float4 *cur = d.PS, *alt = d.PS2;
     const uint32_t iters = s->prm.solver_iterations;
     for (uint32_t it = 0; it < iters; ++it) {
       if (s->rc_maxn) {
-        PBF_TRY(rc_build(cur, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt, st));
+        PBF_TRY(rc_build(cur, d.DV, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt, st));
         PBF_TRY_STATUS(mark(s, 1, "rc_build", 1, &ev));
       }
       PBF_TRY(rc_lambda(cur, d.SS, lists, d.offsets, n, s->rc, st));
       PBF_TRY_STATUS(mark(s, 1, "rc_lambda", 1, &ev));
-      PBF_TRY(rc_delta(cur, alt, d.SS, lists, d.perm, d.offsets, d.X, d.V, d.P, d.VS, n, s->rc,
-                       d.scenes, it + 1 == iters, st));
+      PBF_TRY(rc_delta(cur, alt, d.SS, lists, d.perm, d.offsets, d.X, d.V, d.P, d.VS, d.DV, n,
+                       s->rc, d.scenes, it + 1 == iters, st));
       PBF_TRY_STATUS(mark(s, 2, "rc_delta", 1, &ev));
       std::swap(cur, alt);
     }
     if (s->rc_maxn) {
-      PBF_TRY(rc_build(cur, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt, st));
+      PBF_TRY(rc_build(cur, d.DV, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt, st));
       PBF_TRY_STATUS(mark(s, 3, "rc_build", 1, &ev));
     }
     PBF_TRY(rc_xsph(cur, d.VS, d.DV, lists, d.perm, d.offsets, n, s->rc, st));
@@ -571,7 +571,7 @@ int pbf_init(pbf_sim *s) {
     A(&d.Q, n);
     A(&d.D, n);
     A(&d.U, n);
-    A(&d.W, n);
+    A(&d.W, std::max(n, kMinPlaneSlots));
     A(&d.S, n);
     A(&d.R, n);
     A(&d.nbr_cnt, n);
@@ -585,7 +585,7 @@ int pbf_init(pbf_sim *s) {
     A(&d.PS, n);
     A(&d.PS2, n);
     A(&d.VS, n);
-    A(&d.DV, n);
+    A(&d.DV, std::max(n, kMinPlaneSlots));
     A(&d.SS, n);
     A(&d.nbr_cnt, n);
     if (s->rc_count_sort) A(&d.cell_scratch, s->cplan.words);
