@@ -141,11 +141,9 @@ int launch_batch_step(pbf_batch *b) {
   const uint32_t n = b->n_total;
   const PaperConsts &pc = b->pc;
   if (!d.tune.radix_sort) {
-    PBF_TRY(cell_sort_clear(b->cplan, d.cell_scratch, false, st));
     PBF_TRY(paper_predict_count(d.X, d.V, n, pc, d.scenes, d.sid, d.keys, b->cplan,
                                 d.cell_scratch, st));
-    PBF_TRY(cell_sort_finish(b->cplan, d.keys, d.cell_scratch, d.offsets, d.skeys, d.perm, d.err,
-                             st));
+    PBF_TRY(cell_sort_place(b->cplan, d.keys, d.cell_scratch, d.offsets, d.skeys, d.perm, d.err, st));
   } else {
     PBF_TRY(sort_clear(b->plan, d.sort_scratch, st));
     PBF_TRY(paper_predict_hash(d.X, d.V, n, pc, d.scenes, d.sid, d.keys, b->plan,
@@ -154,7 +152,8 @@ int launch_batch_step(pbf_batch *b) {
     PBF_TRY(sort_passes(b->plan, d.keys, nullptr, d.skeys, d.perm, d.sort_scratch, d.err, st));
     PBF_TRY(cell_offsets_runs(d.skeys, n, b->cells_total, d.offsets, d.runs, d.runs_count, st));
   }
-  PBF_TRY(paper_reorder(d.perm, d.X, d.V, d.ID, n, pc, d.X2, d.V2, d.ID2, d.P, d.D, d.W, st));
+  const StepClear clear = step_clear(b->cplan, d.cell_scratch, nullptr);
+  PBF_TRY(paper_reorder(d, n, pc, d.tune.radix_sort ? nullptr : &clear, st));
   const uint32_t iters = b->solver.solver_iterations;
   if (d.tune.staged) {
     PBF_TRY(tile_plan(d, pc, d.sid, (uint32_t)b->scenes.size(), st));
@@ -482,7 +481,7 @@ int pbf_batch_launches_per_step(const pbf_batch *b, uint32_t *launches) {
                                        bits_for(std::max<uint32_t>(b->cells_total, 1)));
   // predict + hash, the sort (counting: 4 launches; radix: scan, digit
   // passes, two for the offsets), reorder, the solver, the velocity passes
-  const uint32_t sort = b->d.tune.radix_sort ? 1u + plan.passes + 2u : cell_sort_launches();
+  const uint32_t sort = b->d.tune.radix_sort ? 1u + plan.passes + 2u : kCellPlaceLaunches;
   *launches = 1u + sort + 1u + paper_first_launches(b->d) +
               2u * b->solver.solver_iterations - 1u + 2u;
   return PBF_OK;

@@ -183,8 +183,12 @@ uint32_t sort_pass_launches(const SortPlan &plan);
 // (leaving the counts zero for the next step), scatters the particles and
 // puts each cell back in index order, so skeys / perm are the stable sort's.
 // Layout of its scratch (32-bit words):
+// The step's own order of the particles in a cell is left to the kernel that
+// gathers the state (ordered_slot) for cells of up to this many.
+constexpr uint32_t kRankCell = 64;
 struct CellSortPlan {
   uint32_t n = 0, ncells = 0, tiles = 0;
+  uint32_t scan_chunks = 0;  // chunks of 2048 counts per scan tile (1 or 4)
   uint32_t small_cap = 0, med_cap = 0, big_cap = 0, huge_cap = 0;
   uint32_t bm_words = 0;   // words of a bitmap over the n particle indices
   uint32_t bm_stride = 0;  // words from one CTA's bitmap to the next
@@ -213,7 +217,24 @@ cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, bool co
 cudaError_t cell_sort_finish(const CellSortPlan &plan, const uint32_t *keys, uint32_t *scratch,
                              uint32_t *offsets, uint32_t *skeys, uint32_t *perm, uint32_t *err,
                              cudaStream_t stream);
-uint32_t cell_sort_launches();
+// The same for a step, whose gather of the state orders the cells of up to
+// kRankCell particles (ordered_slot): perm holds those in the order their
+// counts were taken.  The control words must be zero (cell_sort_clear once;
+// the gather leaves them so).
+cudaError_t cell_sort_place(const CellSortPlan &plan, const uint32_t *keys, uint32_t *scratch,
+                            uint32_t *offsets, uint32_t *skeys, uint32_t *perm, uint32_t *err,
+                            cudaStream_t stream);
+constexpr uint32_t kCellPlaceLaunches = 3;
+// The words a step's gather zeroes for the next step (ctl, words) and for the
+// rest of this one (one word, may be null).
+struct StepClear {
+  uint32_t *ctl;
+  uint32_t words;
+  uint32_t *also;
+};
+inline StepClear step_clear(const CellSortPlan &plan, uint32_t *scratch, uint32_t *also) {
+  return StepClear{scratch + plan.off_ctl, (uint32_t)plan.ctl_words, also};
+}
 // The predict kernel's counting from a key array; a key outside
 // [0, plan.ncells) is left out and sets kDevErrKey in *err.
 cudaError_t cell_sort_count(const CellSortPlan &plan, const uint32_t *keys, uint32_t *scratch,
@@ -311,7 +332,7 @@ struct DeviceState {
   uint32_t *ID = nullptr;              // input index of each slot (paper)
   // step scratch
   float4 *X2 = nullptr, *V2 = nullptr; // reordered state (paper)
-  uint32_t *ID2 = nullptr;
+  uint32_t *ID2 = nullptr;             // input index of each slot during the step
   float4 *P = nullptr, *Q = nullptr;   // predicted positions (+lambda)
   float4 *D = nullptr;                 // displacement since step start (paper)
   float4 *U = nullptr;                 // velocity and 1/rho (paper)
@@ -407,11 +428,11 @@ cudaError_t paper_predict_count(const float4 *X, const float4 *V, uint32_t n,
 // so that the padding of small scenes fits.
 PBF_HOST_DEVICE inline uint32_t plane_floats(uint32_t n) { return (n + 3u) & ~3u; }
 constexpr size_t kMinPlaneSlots = 16;
-cudaError_t paper_reorder(const uint32_t *perm, const float4 *X,
-                          const float4 *V, const uint32_t *ID, uint32_t n,
-                          const PaperConsts &c, float4 *X2, float4 *V2,
-                          uint32_t *ID2, float4 *P, float4 *D, float4 *planes,
-                          cudaStream_t st);
+// The state into slot order.  `clear`: the sort left the small cells
+// unordered (cell_sort_place), and these words are to be zeroed; null after
+// the radix sort.
+cudaError_t paper_reorder(const DeviceState &d, uint32_t n, const PaperConsts &c,
+                          const StepClear *clear, cudaStream_t st);
 // Neighbour lists of the step (from the predicted positions P).
 cudaError_t paper_nbr_build(const DeviceState &d, const PaperConsts &c,
                             const uint16_t *sid, cudaStream_t st);
@@ -464,10 +485,9 @@ cudaError_t rc_predict_hash(float4 *X, float4 *V, float4 *P, uint32_t n,
 cudaError_t rc_predict_count(float4 *X, float4 *V, float4 *P, uint32_t n, const RefConsts &k,
                              const SceneDesc *scenes, uint32_t *keys, const CellSortPlan &plan,
                              uint32_t *cell_scratch, cudaStream_t st);
-// PS[m] = P of the particle in slot m: the predicted positions by slot.
-// The build reads the positions as planes (plane_floats above).
-cudaError_t rc_gather(const float4 *P, const uint32_t *perm, uint32_t n, float4 *PS,
-                      float4 *planes, cudaStream_t st);
+// P by slot (PS, and the planes the build reads) and the input index of each
+// slot (ID2); `clear` as in paper_reorder.
+cudaError_t rc_gather(const DeviceState &d, uint32_t n, const StepClear *clear, cudaStream_t st);
 // Neighbour lists of the positions PS.
 cudaError_t rc_build(const float4 *PS, const float4 *planes, const uint32_t *offsets, uint32_t n,
                      const RefConsts &k, uint32_t maxn, uint4 *nbr, uint32_t *nbr_cnt,
@@ -478,11 +498,11 @@ cudaError_t rc_build(const float4 *PS, const float4 *planes, const uint32_t *off
 cudaError_t rc_lambda(float4 *PS, float *SS, const RefLists &lists, const uint32_t *offsets,
                       uint32_t n, const RefConsts &k, cudaStream_t st);
 cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const RefLists &lists,
-                     const uint32_t *perm, const uint32_t *offsets, const float4 *X, float4 *V,
+                     const uint32_t *input, const uint32_t *offsets, const float4 *X, float4 *V,
                      float4 *P, float4 *VS, float4 *planes, uint32_t n,
                      const RefConsts &k, const SceneDesc *scenes, bool last, cudaStream_t st);
 cudaError_t rc_xsph(const float4 *PS, const float4 *VS, float4 *DV, const RefLists &lists,
-                    const uint32_t *perm, const uint32_t *offsets, uint32_t n,
+                    const uint32_t *input, const uint32_t *offsets, uint32_t n,
                     const RefConsts &k, cudaStream_t st);
 cudaError_t rc_commit(float4 *X, float4 *V, const float4 *P, const float4 *DV,
                       uint32_t n, cudaStream_t st);

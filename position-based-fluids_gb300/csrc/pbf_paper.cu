@@ -118,24 +118,37 @@ __global__ void __launch_bounds__(256)
     if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
+// The state in slot order: slot k of `perm` (kRanked: cells of up to kRankCell
+// particles still unordered, each particle finding its slot in its cell --
+// about eight indices its cell-mates read as well, where a pass over the
+// cells that put them in order took 5 us at 1M particles and a launch).
+// kRanked also leaves the sort's control words and the step's largest
+// neighbour count zero.
+template <bool kRanked>
 __global__ void __launch_bounds__(256)
-    k_reorder(const uint32_t *__restrict__ perm, const float4 *__restrict__ X,
-              const float4 *__restrict__ V, const uint32_t *__restrict__ ID,
-              uint32_t n, PaperConsts c, float4 *__restrict__ X2,
-              float4 *__restrict__ V2, uint32_t *__restrict__ ID2,
-              float4 *__restrict__ P, float4 *__restrict__ D, float *__restrict__ planes,
-              uint32_t plane) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
+    k_reorder(const uint32_t *__restrict__ perm, const uint32_t *__restrict__ skeys,
+              const uint32_t *__restrict__ off, StepClear clear, const float4 *__restrict__ X,
+              const float4 *__restrict__ V, const uint32_t *__restrict__ ID, uint32_t n,
+              PaperConsts c, float4 *__restrict__ X2, float4 *__restrict__ V2,
+              uint32_t *__restrict__ ID2, float4 *__restrict__ P, float4 *__restrict__ D,
+              float *__restrict__ planes, uint32_t plane) {
+  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (kRanked) {
+    for (uint32_t i = q; i < clear.words; i += gridDim.x * blockDim.x) clear.ctl[i] = 0u;
+    if (q == 0 && clear.also) *clear.also = 0u;
+  }
+  if (q >= n) return;
   // perm is a permutation of [0, n) unless the sort reported an error.
-  const uint32_t src = min(perm[k], n - 1);
+  const uint32_t src = min(perm[q], n - 1);
   const float4 x = X[src];
   const float4 v1 = gravity_velocity(V[src], c.dt, c.gy);
+  const uint32_t id = ID[src];
+  const uint32_t k = kRanked ? ordered_slot(perm, off, skeys[q], q, src, n) : q;
   const float3 d = displacement(v1, c.dt);
   const float3 p = add3(x, d);
   X2[k] = x;
   V2[k] = v1;
-  ID2[k] = ID[src];
+  ID2[k] = id;
   P[k] = make_float4(p.x, p.y, p.z, 0.0f);
   D[k] = make_float4(d.x, d.y, d.z, 0.0f);
   planes[k] = p.x;
@@ -393,14 +406,12 @@ cudaError_t paper_predict_count(const float4 *X, const float4 *V, uint32_t n,
   return cudaGetLastError();
 }
 
-cudaError_t paper_reorder(const uint32_t *perm, const float4 *X,
-                          const float4 *V, const uint32_t *ID, uint32_t n,
-                          const PaperConsts &c, float4 *X2, float4 *V2,
-                          uint32_t *ID2, float4 *P, float4 *D, float4 *planes,
-                          cudaStream_t st) {
-  k_reorder<<<blocks_for(n, 256), 256, 0, st>>>(perm, X, V, ID, n, c, X2, V2, ID2, P, D,
-                                                reinterpret_cast<float *>(planes),
-                                                plane_floats(n));
+cudaError_t paper_reorder(const DeviceState &d, uint32_t n, const PaperConsts &c,
+                          const StepClear *clear, cudaStream_t st) {
+  const auto kernel = clear ? k_reorder<true> : k_reorder<false>;
+  kernel<<<blocks_for(n, 256), 256, 0, st>>>(
+      d.perm, d.skeys, d.offsets, clear ? *clear : StepClear{}, d.X, d.V, d.ID, n, c, d.X2, d.V2,
+      d.ID2, d.P, d.D, reinterpret_cast<float *>(d.W), plane_floats(n));
   return cudaGetLastError();
 }
 

@@ -95,13 +95,6 @@ __device__ __forceinline__ void store_planes(float *__restrict__ planes, uint32_
   planes[2 * (size_t)plane + q] = p.z;
 }
 
-// Input index of sorted slot q (perm is a permutation of [0, n) unless the
-// sort reported an error).
-__device__ __forceinline__ uint32_t rc_input(const uint32_t *__restrict__ perm, uint32_t q,
-                                             uint32_t n) {
-  return n - 1u - min(perm[q], n - 1u);
-}
-
 // Prediction of sort element t (particle n - 1 - t) and its cell.
 __device__ __forceinline__ uint32_t rc_predict(uint32_t t, uint32_t n, const float4 *X, float4 *V,
                                                float4 *P, const RefConsts &k,
@@ -161,13 +154,26 @@ __global__ void __launch_bounds__(256)
     if (s_hist[t]) atomicAdd(&hist[t], s_hist[t]);
 }
 
+// Predicted positions by slot (PS, planes) and each slot's input index.
+// kRanked: as k_reorder (pbf_paper.cu), the cells of up to kRankCell particles
+// are put in order here, and the sort's control words left zero.
+template <bool kRanked>
 __global__ void __launch_bounds__(256)
-    k_rc_gather(const float4 *__restrict__ P, const uint32_t *__restrict__ perm, uint32_t n,
-                float4 *__restrict__ PS, float *__restrict__ planes, uint32_t plane) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const float4 p = P[rc_input(perm, q, n)];
+    k_rc_gather(const float4 *__restrict__ P, const uint32_t *__restrict__ perm,
+                const uint32_t *__restrict__ skeys, const uint32_t *__restrict__ off,
+                StepClear clear, uint32_t n, float4 *__restrict__ PS, uint32_t *__restrict__ input,
+                float *__restrict__ planes, uint32_t plane) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (kRanked)
+    for (uint32_t i = t; i < clear.words; i += gridDim.x * blockDim.x) clear.ctl[i] = 0u;
+  if (t >= n) return;
+  // perm is a permutation of [0, n) unless the sort reported an error.
+  const uint32_t element = min(perm[t], n - 1u);
+  const uint32_t q = kRanked ? ordered_slot(perm, off, skeys[t], t, element, n) : t;
+  const uint32_t i = n - 1u - element;
+  const float4 p = P[i];
   PS[q] = p;
+  input[q] = i;
   store_planes(planes, plane, q, p);
 }
 
@@ -233,7 +239,7 @@ __global__ void __launch_bounds__(kThreads)
 
 __global__ void __launch_bounds__(kThreads)
     k_rc_delta(const float4 *__restrict__ PS, float4 *__restrict__ PS2,
-               const float *__restrict__ SS, RefLists lists, const uint32_t *__restrict__ perm,
+               const float *__restrict__ SS, RefLists lists, const uint32_t *__restrict__ input,
                const uint32_t *__restrict__ off, const float4 *__restrict__ X,
                float4 *__restrict__ V, float4 *__restrict__ P, float4 *__restrict__ VS,
                float *__restrict__ planes, uint32_t plane, uint32_t n, RefConsts k,
@@ -280,7 +286,7 @@ __global__ void __launch_bounds__(kThreads)
   PS2[q] = np;
   store_planes(planes, plane, q, np);
   if (last) {
-    const uint32_t i = rc_input(perm, q, n);
+    const uint32_t i = input[q];
     P[i] = np;
     // updateVelocities
     const float4 x = X[i];
@@ -295,7 +301,7 @@ __global__ void __launch_bounds__(kThreads)
 
 __global__ void __launch_bounds__(kThreads)
     k_rc_xsph(const float4 *__restrict__ PS, const float4 *__restrict__ VS,
-              float4 *__restrict__ DV, RefLists lists, const uint32_t *__restrict__ perm,
+              float4 *__restrict__ DV, RefLists lists, const uint32_t *__restrict__ input,
               const uint32_t *__restrict__ off, uint32_t n, RefConsts k) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
@@ -319,7 +325,7 @@ __global__ void __launch_bounds__(kThreads)
       sz += inv * vz * poly;
     }
   });
-  DV[rc_input(perm, q, n)] = make_float4(0.01f * sx, 0.01f * sy, 0.01f * sz, 0.0f);
+  DV[input[q]] = make_float4(0.01f * sx, 0.01f * sy, 0.01f * sz, 0.0f);
 }
 
 __global__ void __launch_bounds__(256)
@@ -372,11 +378,11 @@ cudaError_t rc_build(const float4 *PS, const float4 *planes, const uint32_t *off
   return cudaGetLastError();
 }
 
-cudaError_t rc_gather(const float4 *P, const uint32_t *perm, uint32_t n, float4 *PS,
-                      float4 *planes, cudaStream_t st) {
-  k_rc_gather<<<blocks_for(n, 256), 256, 0, st>>>(P, perm, n, PS,
-                                                  reinterpret_cast<float *>(planes),
-                                                  plane_floats(n));
+cudaError_t rc_gather(const DeviceState &d, uint32_t n, const StepClear *clear, cudaStream_t st) {
+  const auto kernel = clear ? k_rc_gather<true> : k_rc_gather<false>;
+  kernel<<<blocks_for(n, 256), 256, 0, st>>>(d.P, d.perm, d.skeys, d.offsets,
+                                             clear ? *clear : StepClear{}, n, d.PS, d.ID2,
+                                             reinterpret_cast<float *>(d.DV), plane_floats(n));
   return cudaGetLastError();
 }
 
@@ -387,20 +393,19 @@ cudaError_t rc_lambda(float4 *PS, float *SS, const RefLists &lists, const uint32
 }
 
 cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const RefLists &lists,
-                     const uint32_t *perm,
-                     const uint32_t *offsets, const float4 *X, float4 *V, float4 *P,
-                     float4 *VS, float4 *planes, uint32_t n, const RefConsts &k,
+                     const uint32_t *input, const uint32_t *offsets, const float4 *X, float4 *V,
+                     float4 *P, float4 *VS, float4 *planes, uint32_t n, const RefConsts &k,
                      const SceneDesc *scenes, bool last, cudaStream_t st) {
   k_rc_delta<<<blocks_for(n, kThreads), kThreads, 0, st>>>(
-      PS, PS2, SS, lists, perm, offsets, X, V, P, VS, reinterpret_cast<float *>(planes),
+      PS, PS2, SS, lists, input, offsets, X, V, P, VS, reinterpret_cast<float *>(planes),
       plane_floats(n), n, k, scenes, last ? 1 : 0);
   return cudaGetLastError();
 }
 
 cudaError_t rc_xsph(const float4 *PS, const float4 *VS, float4 *DV, const RefLists &lists,
-                    const uint32_t *perm, const uint32_t *offsets, uint32_t n, const RefConsts &k,
+                    const uint32_t *input, const uint32_t *offsets, uint32_t n, const RefConsts &k,
                     cudaStream_t st) {
-  k_rc_xsph<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, VS, DV, lists, perm, offsets, n, k);
+  k_rc_xsph<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, VS, DV, lists, input, offsets, n, k);
   return cudaGetLastError();
 }
 

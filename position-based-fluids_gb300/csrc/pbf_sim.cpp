@@ -196,14 +196,11 @@ int launch_step(pbf_sim *s) {
   if (s->paper && !d.tune.radix_sort) {
     // counting sort by cell: the counts, the offsets, the scatter and the
     // order within each cell
-    PBF_TRY(cell_sort_clear(s->cplan, d.cell_scratch, false, st));
-    PBF_TRY(cudaMemsetAsync(d.nbr_max, 0, sizeof(uint32_t), st));
     PBF_TRY(paper_predict_count(d.X, d.V, n, s->pc, d.scenes, nullptr, d.keys, s->cplan,
                                 d.cell_scratch, st));
     PBF_TRY_STATUS(mark(s, 0, "predict_hash", 1, &ev));
-    PBF_TRY(cell_sort_finish(s->cplan, d.keys, d.cell_scratch, d.offsets, d.skeys, d.perm, d.err,
-                             st));
-    PBF_TRY_STATUS(mark(s, 0, "cell_sort", cell_sort_launches(), &ev));
+    PBF_TRY(cell_sort_place(s->cplan, d.keys, d.cell_scratch, d.offsets, d.skeys, d.perm, d.err, st));
+    PBF_TRY_STATUS(mark(s, 0, "cell_sort", kCellPlaceLaunches, &ev));
   } else if (s->paper) {
     PBF_TRY(sort_clear(s->plan, d.sort_scratch, st));
     PBF_TRY(cudaMemsetAsync(d.nbr_max, 0, sizeof(uint32_t), st));
@@ -218,8 +215,8 @@ int launch_step(pbf_sim *s) {
     PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
   }
   if (s->paper) {
-    PBF_TRY(paper_reorder(d.perm, d.X, d.V, d.ID, n, s->pc, d.X2, d.V2, d.ID2,
-                          d.P, d.D, d.W, st));
+    const StepClear clear = step_clear(s->cplan, d.cell_scratch, d.nbr_max);
+    PBF_TRY(paper_reorder(d, n, s->pc, d.tune.radix_sort ? nullptr : &clear, st));
     PBF_TRY_STATUS(mark(s, 0, "reorder", 1, &ev));
     const uint32_t iters = s->prm.solver_iterations;
     if (d.tune.staged) {
@@ -267,13 +264,11 @@ int launch_step(pbf_sim *s) {
     }
   } else {
     if (s->rc_count_sort) {
-      PBF_TRY(cell_sort_clear(s->cplan, d.cell_scratch, false, st));
       PBF_TRY(rc_predict_count(d.X, d.V, d.P, n, s->rc, d.scenes, d.keys, s->cplan,
                                d.cell_scratch, st));
       PBF_TRY_STATUS(mark(s, 0, "rc_predict_hash", 1, &ev));
-      PBF_TRY(cell_sort_finish(s->cplan, d.keys, d.cell_scratch, d.offsets, d.skeys, d.perm,
-                               d.err, st));
-      PBF_TRY_STATUS(mark(s, 0, "cell_sort", cell_sort_launches(), &ev));
+      PBF_TRY(cell_sort_place(s->cplan, d.keys, d.cell_scratch, d.offsets, d.skeys, d.perm, d.err, st));
+      PBF_TRY_STATUS(mark(s, 0, "cell_sort", kCellPlaceLaunches, &ev));
     } else {
       PBF_TRY(sort_clear(s->plan, d.sort_scratch, st));
       PBF_TRY(rc_predict_hash(d.X, d.V, d.P, n, s->rc, d.scenes, d.keys, s->plan,
@@ -285,7 +280,8 @@ int launch_step(pbf_sim *s) {
       PBF_TRY(step_offsets(s));
       PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
     }
-    PBF_TRY(rc_gather(d.P, d.perm, n, d.PS, d.DV, st));
+    const StepClear clear = step_clear(s->cplan, d.cell_scratch, nullptr);
+    PBF_TRY(rc_gather(d, n, s->rc_count_sort ? &clear : nullptr, st));
     PBF_TRY_STATUS(mark(s, 0, "rc_gather", 1, &ev));
     const RefLists lists{d.nbr, d.nbr_cnt, n, s->rc_maxn};
     float4 *cur = d.PS, *alt = d.PS2;
@@ -297,7 +293,7 @@ int launch_step(pbf_sim *s) {
       }
       PBF_TRY(rc_lambda(cur, d.SS, lists, d.offsets, n, s->rc, st));
       PBF_TRY_STATUS(mark(s, 1, "rc_lambda", 1, &ev));
-      PBF_TRY(rc_delta(cur, alt, d.SS, lists, d.perm, d.offsets, d.X, d.V, d.P, d.VS, d.DV, n,
+      PBF_TRY(rc_delta(cur, alt, d.SS, lists, d.ID2, d.offsets, d.X, d.V, d.P, d.VS, d.DV, n,
                        s->rc, d.scenes, it + 1 == iters, st));
       PBF_TRY_STATUS(mark(s, 2, "rc_delta", 1, &ev));
       std::swap(cur, alt);
@@ -306,7 +302,7 @@ int launch_step(pbf_sim *s) {
       PBF_TRY(rc_build(cur, d.DV, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt, st));
       PBF_TRY_STATUS(mark(s, 3, "rc_build", 1, &ev));
     }
-    PBF_TRY(rc_xsph(cur, d.VS, d.DV, lists, d.perm, d.offsets, n, s->rc, st));
+    PBF_TRY(rc_xsph(cur, d.VS, d.DV, lists, d.ID2, d.offsets, n, s->rc, st));
     PBF_TRY_STATUS(mark(s, 3, "rc_xsph", 1, &ev));
     PBF_TRY(rc_commit(d.X, d.V, d.P, d.DV, n, st));
     PBF_TRY_STATUS(mark(s, 3, "rc_commit", 1, &ev));
@@ -587,6 +583,7 @@ int pbf_init(pbf_sim *s) {
     A(&d.VS, n);
     A(&d.DV, std::max(n, kMinPlaneSlots));
     A(&d.SS, n);
+    A(&d.ID2, n);
     A(&d.nbr_cnt, n);
     if (s->rc_count_sort) A(&d.cell_scratch, s->cplan.words);
     if (rc == PBF_OK) rc = alloc_ref_lists(s);
@@ -800,7 +797,7 @@ int pbf_launches_per_step(const pbf_sim *s, uint32_t *launches) {
   if (!s || !launches) return PBF_ERR_INVALID;
   const uint32_t it = s->prm.solver_iterations;
   const uint32_t sort = (s->paper ? !s->d.tune.radix_sort : s->rc_count_sort)
-                            ? cell_sort_launches()
+                            ? kCellPlaceLaunches
                             : 1u /*scan*/ + s->plan.passes + (s->offset_runs ? 2u : 1u) /*offsets*/;
   if (s->paper)
     *launches = 1u /*predict+hash*/ + sort + 1u /*reorder*/ + paper_first_launches(s->d) +

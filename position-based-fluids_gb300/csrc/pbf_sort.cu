@@ -414,8 +414,10 @@ inline uint32_t blocks_for(uint64_t n, uint32_t t) {
 // ones through a per-CTA bitmap of the particle indices.
 constexpr uint32_t kScanItems = 8;                            // counts per thread and chunk
 constexpr uint32_t kScanChunk = kSortThreads * kScanItems;   // 2048
-constexpr uint32_t kScanChunks = 4;
-constexpr uint32_t kScanTile = kScanChunk * kScanChunks;     // counts per scan tile
+constexpr uint32_t kScanChunks = 4;    // chunks per scan tile, where there are many
+// Grids of few cells take one chunk per tile: the scan is then one chunk and
+// the look-back over at most these tiles (they fit the control words).
+constexpr uint32_t kFewTiles = 56;
 constexpr uint32_t kSmallCell = 16;
 constexpr uint32_t kWarpCell = 64;  // cells of 17..64 particles: one warp each
 // control words: [0] scan tiles started, [1] big cells, [2] huge cells,
@@ -463,11 +465,16 @@ __device__ __forceinline__ uint32_t warp_lookback(uint32_t *lookback, uint32_t t
 }
 
 // off[c] = particles in cells below c, for c in [0, ncells]; counts[c] -> 0.
-// Tiles of kScanTile counts (kScanChunks chunks of 2048, each thread holding
-// 8 consecutive counts of every chunk) are numbered in the order CTAs start.
+// Tiles of kScanChunks chunks of 2048 counts (each thread holding 8
+// consecutive counts of every chunk) are numbered in the order CTAs start.
+// kList: cells of more than kRankCell particles are listed for k_cell_fix_big.
+template <uint32_t kScanChunks, bool kList>
 __global__ void __launch_bounds__(kSortThreads)
     k_count_scan(uint32_t *__restrict__ counts, uint32_t ncells, uint32_t total,
-                 uint32_t *__restrict__ off, uint32_t *ctl, uint32_t *err) {
+                 uint32_t *__restrict__ off, uint32_t *ctl, uint32_t *err,
+                 uint32_t *__restrict__ big, uint32_t big_cap, uint32_t *__restrict__ huge,
+                 uint32_t huge_cap) {
+  constexpr uint32_t kScanTile = kScanChunk * kScanChunks;
   __shared__ uint32_t s_tile, s_excl;
   __shared__ uint32_t s_chunk[kScanChunks];
   __shared__ uint32_t s_warp[kSortWarps];
@@ -500,7 +507,18 @@ __global__ void __launch_bounds__(kSortThreads)
       }
     }
 #pragma unroll
-    for (uint32_t j = 0; j < kScanItems; ++j) sum += v[q][j];
+    for (uint32_t j = 0; j < kScanItems; ++j) {
+      sum += v[q][j];
+      if (kList && v[q][j] > kRankCell) {
+        if (v[q][j] <= kBigCell) {
+          const uint32_t at = atomicAdd(&ctl[1], 1u);
+          if (at < big_cap) big[at] = base + j;
+        } else {
+          const uint32_t at = atomicAdd(&ctl[2], 1u);
+          if (at < huge_cap) huge[at] = base + j;
+        }
+      }
+    }
     texcl[q] = block_exclusive_scan(sum, s_warp);
     if (tid == kSortThreads - 1) s_chunk[q] = texcl[q] + sum;
     __syncthreads();
@@ -899,11 +917,19 @@ cudaError_t cell_hash(const float4 *pred, uint32_t n, const SceneDesc &scene,
   return cudaGetLastError();
 }
 
+static void set_scan_tiles(CellSortPlan &p) {
+  static_assert(kCtlHeader + kFewTiles <= 64, "the control words are padded to 64");
+  const uint32_t few = (uint32_t)(((uint64_t)p.ncells + kScanChunk - 1) / kScanChunk);
+  p.scan_chunks = few <= kFewTiles ? 1u : kScanChunks;
+  p.tiles = (few + p.scan_chunks - 1) / p.scan_chunks;
+  p.ctl_words = kCtlHeader + (size_t)p.tiles;
+}
+
 CellSortPlan make_cell_sort_plan(uint32_t n, uint32_t ncells) {
   CellSortPlan p;
   p.n = n;
   p.ncells = ncells;
-  p.tiles = (uint32_t)(((uint64_t)ncells + kScanTile - 1) / kScanTile);
+  set_scan_tiles(p);
   p.small_cap = (uint32_t)std::min<uint64_t>(ncells, (uint64_t)n / 2 + 1);
   p.med_cap = (uint32_t)std::min<uint64_t>(ncells, (uint64_t)n / (kSmallCell + 1) + 1);
   p.big_cap = (uint32_t)std::min<uint64_t>(ncells, (uint64_t)n / (kWarpCell + 1) + 1);
@@ -918,8 +944,9 @@ CellSortPlan make_cell_sort_plan(uint32_t n, uint32_t ncells) {
   w += n;
   w = (w + 63) & ~size_t(63);
   p.off_ctl = w;
-  p.ctl_words = kCtlHeader + (size_t)p.tiles;
-  w += p.ctl_words;
+  // room for tiles of either size (kFewTiles of the small ones fit 64 words)
+  w += kCtlHeader + (size_t)(((uint64_t)ncells + kScanChunk * kScanChunks - 1) /
+                             (kScanChunk * kScanChunks));
   w = (w + 63) & ~size_t(63);
   p.off_small = w;
   w += p.small_cap;
@@ -940,8 +967,7 @@ CellSortPlan resize_cell_sort_plan(const CellSortPlan &cap, uint32_t n, uint32_t
   CellSortPlan p = cap;
   p.n = std::min(n, cap.n);
   p.ncells = std::min(ncells, cap.ncells);
-  p.tiles = (uint32_t)(((uint64_t)p.ncells + kScanTile - 1) / kScanTile);
-  p.ctl_words = kCtlHeader + (size_t)p.tiles;
+  set_scan_tiles(p);
   p.bm_words = (p.n + 31u) / 32u;
   return p;
 }
@@ -956,19 +982,50 @@ cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, bool co
   return cudaMemsetAsync(scratch + plan.off_ctl, 0, plan.ctl_words * sizeof(uint32_t), stream);
 }
 
+// The offsets from the counts and every particle at its place.
+template <bool kList>
+static cudaError_t scan_and_scatter(const CellSortPlan &plan, const uint32_t *keys,
+                                    uint32_t *scratch, uint32_t *offsets, uint32_t *skeys,
+                                    uint32_t *perm, uint32_t *err, cudaStream_t stream) {
+  if (plan.ncells == 0) return cudaErrorInvalidValue;
+  const auto scan =
+      plan.scan_chunks == 1 ? k_count_scan<1, kList> : k_count_scan<kScanChunks, kList>;
+  scan<<<plan.tiles, kSortThreads, 0, stream>>>(
+      scratch + plan.off_counts, plan.ncells, plan.n, offsets, scratch + plan.off_ctl, err,
+      scratch + plan.off_big, plan.big_cap, scratch + plan.off_huge, plan.huge_cap);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess || plan.n == 0) return e;
+  k_count_scatter<<<blocks_for(plan.n, 256), 256, 0, stream>>>(
+      keys, scratch + plan.off_pos, offsets, plan.n, plan.ncells, skeys, perm);
+  return cudaGetLastError();
+}
+
+static cudaError_t fix_big(const CellSortPlan &plan, uint32_t *scratch, const uint32_t *offsets,
+                           uint32_t *perm, uint32_t ctas, cudaStream_t stream) {
+  k_cell_fix_big<<<ctas, kSortThreads, 0, stream>>>(
+      offsets, perm, scratch + plan.off_small, plan.small_cap, scratch + plan.off_med,
+      plan.med_cap, scratch + plan.off_big, plan.big_cap, scratch + plan.off_huge, plan.huge_cap,
+      scratch + plan.off_ctl, scratch + plan.off_bitmap, plan.bm_words, plan.bm_stride);
+  return cudaGetLastError();
+}
+
+cudaError_t cell_sort_place(const CellSortPlan &plan, const uint32_t *keys, uint32_t *scratch,
+                            uint32_t *offsets, uint32_t *skeys, uint32_t *perm, uint32_t *err,
+                            cudaStream_t stream) {
+  const cudaError_t e = scan_and_scatter<true>(plan, keys, scratch, offsets, skeys, perm, err,
+                                               stream);
+  if (e != cudaSuccess || plan.n == 0) return e;
+  // at most n / (kRankCell + 1) cells are listed
+  const uint32_t ctas = min(kStrideCtas / 4u, max(kHugeCtas, plan.n / (kRankCell + 1u) + 1u));
+  return fix_big(plan, scratch, offsets, perm, ctas, stream);
+}
+
 cudaError_t cell_sort_finish(const CellSortPlan &plan, const uint32_t *keys, uint32_t *scratch,
                              uint32_t *offsets, uint32_t *skeys, uint32_t *perm, uint32_t *err,
                              cudaStream_t stream) {
   uint32_t *ctl = scratch + plan.off_ctl;
-  if (plan.ncells == 0) return cudaErrorInvalidValue;
-  k_count_scan<<<plan.tiles, kSortThreads, 0, stream>>>(scratch + plan.off_counts, plan.ncells,
-                                                         plan.n, offsets, ctl, err);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = scan_and_scatter<false>(plan, keys, scratch, offsets, skeys, perm, err, stream);
   if (e != cudaSuccess || plan.n == 0) return e;
-  k_count_scatter<<<blocks_for(plan.n, 256), 256, 0, stream>>>(
-      keys, scratch + plan.off_pos, offsets, plan.n, plan.ncells, skeys, perm);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
   // dense grids sort their small cells in the pass over the cells, sparse
   // ones list them (measured: 1M particles in 64^3 cells, 14.6M in 14.6M)
   if ((uint64_t)plan.ncells * 2u <= plan.n)
@@ -983,14 +1040,8 @@ cudaError_t cell_sort_finish(const CellSortPlan &plan, const uint32_t *keys, uin
         scratch + plan.off_huge, plan.huge_cap, ctl);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_cell_fix_big<<<kStrideCtas / 4u, kSortThreads, 0, stream>>>(
-      offsets, perm, scratch + plan.off_small, plan.small_cap, scratch + plan.off_med,
-      plan.med_cap, scratch + plan.off_big, plan.big_cap, scratch + plan.off_huge, plan.huge_cap,
-      ctl, scratch + plan.off_bitmap, plan.bm_words, plan.bm_stride);
-  return cudaGetLastError();
+  return fix_big(plan, scratch, offsets, perm, kStrideCtas / 4u, stream);
 }
-
-uint32_t cell_sort_launches() { return 4u; }
 
 cudaError_t cell_sort_count(const CellSortPlan &plan, const uint32_t *keys, uint32_t *scratch,
                             uint32_t *err, cudaStream_t stream) {
