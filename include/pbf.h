@@ -235,7 +235,10 @@ int pbf_launches_per_step(const pbf_sim *sim, uint32_t *launches);
  * default); both give the stable permutation.  masked_build = 1 (the
  * default) has the list build (0 and 1) test each row of candidates into a
  * membership mask and store the members from the mask afterwards; 0 stores
- * each member as it is found.  No choice changes a result bit.  trial_ms is the tuner's best time per launch of each pass (0 when
+ * each member as it is found.  With every field at its default, scenes of up
+ * to 16,384 particles run their gather passes with eight threads per
+ * particle instead; any other setting is taken as given.  No choice changes
+ * a result bit.  trial_ms is the tuner's best time per launch of each pass (0 when
  * untuned). */
 typedef struct pbf_tuning {
   uint32_t threads[6];

@@ -273,6 +273,10 @@ struct GatherTuning {
   // stores the members from it afterwards (same lists; 3% faster build, 6%
   // faster fused build on the 1M-particle dam break)
   uint8_t masked_build = 1;
+  // 1: scenes of few particles take eight threads per particle (pbf_group.cu)
+  // instead of these shapes.  Not part of pbf_tuning: a caller that sets any
+  // shape but the defaults gets that shape.
+  uint8_t grouped = 1;
 };
 constexpr int kBlockCodes = 3;  // 64, 128, 256
 constexpr int kBatchCodes = 2;  // 4, 8
@@ -452,6 +456,27 @@ cudaError_t paper_vorticity(const DeviceState &d, const PaperConsts &c,
                             const uint16_t *sid, cudaStream_t st);
 cudaError_t paper_xsph_commit(const DeviceState &d, const PaperConsts &c,
                               const uint16_t *sid, cudaStream_t st);
+// The same passes with eight threads per particle (pbf_group.cu); paper_*
+// takes them where use_groups says so.  Measured per step, eight threads
+// against one: 1,000 particles 43 against 74 us, 4,096 49 / 86, 8,000 57 / 89,
+// 17,576 79 / 90, 32,768 119 / 97 -- from about 25,000 particles on the GPU is
+// busy and the eight threads' extra instructions (132 against 46 per particle
+// in delta-p) show.  The line lies below that, where several scenes stepped at
+// once gain as well.
+constexpr uint32_t kGroupParticles = 16384;
+inline bool use_groups(const DeviceState &d, const PaperConsts &c) {
+  return d.tune.grouped && c.n <= kGroupParticles;
+}
+cudaError_t group_nbr_lambda(const DeviceState &d, const PaperConsts &c, const uint16_t *sid,
+                             cudaStream_t st);
+cudaError_t group_lambda(const DeviceState &d, const PaperConsts &c, const uint16_t *sid,
+                         cudaStream_t st);
+cudaError_t group_delta(const DeviceState &d, const PaperConsts &c, const uint16_t *sid,
+                        bool last, cudaStream_t st);
+cudaError_t group_vorticity(const DeviceState &d, const PaperConsts &c, const uint16_t *sid,
+                            cudaStream_t st);
+cudaError_t group_xsph_commit(const DeviceState &d, const PaperConsts &c, const uint16_t *sid,
+                              cudaStream_t st);
 // state <-> input order
 cudaError_t gather_to_input_order(const float4 *X, const float4 *V,
                                   const uint32_t *ID, uint32_t n,

@@ -118,6 +118,25 @@ struct RefDistance {  // (x x + y y) + z z, rounded operator by operator
   }
 };
 
+// Bits 31 - e, e < 4: candidate e of the words has low <= r^2 < h2.
+template <typename Distance, bool kLow = true>
+__device__ __forceinline__ uint32_t four_mask(const float4 &x, const float4 &y, const float4 &z,
+                                              float2 nx, float2 ny, float2 nz, float low,
+                                              float h2) {
+  const float2 r01 = Distance::r2(__fadd2_rn(make_float2(x.x, x.y), nx),
+                                  __fadd2_rn(make_float2(y.x, y.y), ny),
+                                  __fadd2_rn(make_float2(z.x, z.y), nz));
+  const float2 r23 = Distance::r2(__fadd2_rn(make_float2(x.z, x.w), nx),
+                                  __fadd2_rn(make_float2(y.z, y.w), ny),
+                                  __fadd2_rn(make_float2(z.z, z.w), nz));
+  const float r[4] = {r01.x, r01.y, r23.x, r23.y};
+  uint32_t m = 0;
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if ((!kLow || r[e] >= low) && r[e] < h2) m |= 0x80000000u >> e;
+  return m;
+}
+
 // Bit 31 - e of the result: candidate c0 + e of [a, b) has low <= r^2 < h2
 // (kLow) or r^2 < h2.  c0 is a multiple of 4, less than b, and a - c0 < 32.
 template <typename Distance, bool kLow>
@@ -130,16 +149,7 @@ __device__ __forceinline__ uint32_t row_mask(const Planes &p, uint32_t c0, uint3
   for (uint32_t g = 0; g < 8; ++g) {
     if (c0 + 4u * g >= b) break;
     const float4 x = __ldg(p.x + w0 + g), y = __ldg(p.y + w0 + g), z = __ldg(p.z + w0 + g);
-    const float2 r01 = Distance::r2(__fadd2_rn(make_float2(x.x, x.y), nx),
-                                    __fadd2_rn(make_float2(y.x, y.y), ny),
-                                    __fadd2_rn(make_float2(z.x, z.y), nz));
-    const float2 r23 = Distance::r2(__fadd2_rn(make_float2(x.z, x.w), nx),
-                                    __fadd2_rn(make_float2(y.z, y.w), ny),
-                                    __fadd2_rn(make_float2(z.z, z.w), nz));
-    const float r[4] = {r01.x, r01.y, r23.x, r23.y};
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if ((!kLow || r[e] >= low) && r[e] < h2) m |= 0x80000000u >> (4 * g + e);
+    m |= four_mask<Distance, kLow>(x, y, z, nx, ny, nz, low, h2) >> (4 * g);
   }
   if (a > c0) m &= ~0u >> (a - c0);
   if (b - c0 < 32u) m &= ~(~0u >> (b - c0));

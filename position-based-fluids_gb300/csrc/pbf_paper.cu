@@ -299,8 +299,8 @@ __global__ void __launch_bounds__(kBlock)
   visit_neighbours<kBatch>(
       nc, k, [&](uint32_t j) { return __ldg(&PW[j]); },
       [&](const float4 &pj) { acc.pair(pk, pj, c); });
-  xsph_commit(k, pk, load_own(&U[k]), load_own(&Wv[k]), load_own(&XS[k]), load_own(&SS[k]), acc,
-              nc, c, ID2, X, V, ID);
+  xsph_store(k, pk, load_own(&U[k]), load_own(&Wv[k]), load_own(&XS[k]), load_own(&SS[k]), acc,
+             c, load_own(&nc.V2[k]).w, load_own(&ID2[k]), X, V, ID);
 }
 
 __global__ void k_gather_out(const float4 *__restrict__ X,
@@ -356,30 +356,6 @@ __global__ void k_scene_ids(const SceneDesc *__restrict__ scenes, uint32_t nscen
 
 inline uint32_t blocks_for(uint64_t n, uint32_t t) {
   return (uint32_t)((n + t - 1) / t);
-}
-
-Planes make_planes(const float4 *planes, uint32_t n) {
-  const size_t words = plane_floats(n) / 4u;
-  return Planes{planes, planes + words, planes + 2 * words};
-}
-
-NbrCtx make_ctx(const DeviceState &d, const PaperConsts &c, const uint16_t *sid) {
-  NbrCtx nc;
-  nc.nbr4 = d.nbr;
-  nc.cnt = d.nbr_cnt;
-  nc.skeys = d.skeys;
-  nc.off = d.offsets;
-  nc.X2 = d.X2;
-  nc.V2 = d.V2;
-  nc.scenes = d.scenes;
-  nc.sid = sid;
-  nc.err = d.err;
-  nc.cnt_max = d.nbr_max;
-  nc.n = c.n;
-  nc.maxn = c.maxn;
-  nc.dt = c.dt;
-  nc.h2 = c.h2;
-  return nc;
 }
 
 }  // namespace
@@ -456,6 +432,7 @@ cudaError_t paper_nbr_build(const DeviceState &d, const PaperConsts &c,
 
 cudaError_t paper_nbr_lambda(const DeviceState &d, const PaperConsts &c,
                              const uint16_t *sid, cudaStream_t st) {
+  if (use_groups(d, c)) return group_nbr_lambda(d, c, sid, st);
   PBF_BUILD_LAUNCH(k_nbr_lambda, kKindNbrLambda, d.P, make_planes(d.W, c.n), make_ctx(d, c, sid),
                    c, d.nbr, d.nbr_cnt, d.Q, d.R);
   return cudaGetLastError();
@@ -463,12 +440,14 @@ cudaError_t paper_nbr_lambda(const DeviceState &d, const PaperConsts &c,
 
 cudaError_t paper_lambda(const DeviceState &d, const PaperConsts &c,
                          const uint16_t *sid, cudaStream_t st) {
+  if (use_groups(d, c)) return group_lambda(d, c, sid, st);
   PBF_GATHER_LAUNCH(k_lambda, kKindLambda, d.P, make_ctx(d, c, sid), c, d.Q, d.R);
   return cudaGetLastError();
 }
 
 cudaError_t paper_delta(const DeviceState &d, const PaperConsts &c,
                         const uint16_t *sid, bool last, cudaStream_t st) {
+  if (use_groups(d, c)) return group_delta(d, c, sid, last, st);
   PBF_GATHER_LAUNCH(k_delta, kKindDelta, d.Q, make_ctx(d, c, sid), c, d.D, d.P, d.R, d.U,
                     last ? 1 : 0);
   return cudaGetLastError();
@@ -476,6 +455,7 @@ cudaError_t paper_delta(const DeviceState &d, const PaperConsts &c,
 
 cudaError_t paper_vorticity(const DeviceState &d, const PaperConsts &c,
                             const uint16_t *sid, cudaStream_t st) {
+  if (use_groups(d, c)) return group_vorticity(d, c, sid, st);
   PBF_GATHER_LAUNCH(k_vorticity, kKindVorticity, d.P, d.U, make_ctx(d, c, sid), c, d.W, d.D, d.Q,
                     d.S);
   return cudaGetLastError();
@@ -483,6 +463,7 @@ cudaError_t paper_vorticity(const DeviceState &d, const PaperConsts &c,
 
 cudaError_t paper_xsph_commit(const DeviceState &d, const PaperConsts &c,
                               const uint16_t *sid, cudaStream_t st) {
+  if (use_groups(d, c)) return group_xsph_commit(d, c, sid, st);
   PBF_GATHER_LAUNCH(k_xsph_commit, kKindXsph, d.D, d.U, d.W, d.Q, d.S, make_ctx(d, c, sid), c, d.ID2,
                     d.X, d.V, d.ID);
   return cudaGetLastError();

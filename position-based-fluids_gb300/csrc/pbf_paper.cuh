@@ -321,14 +321,17 @@ __device__ __forceinline__ void lambda_commit(uint32_t k, const float4 &pk, cons
 }
 
 // Delta-p pass: sum of (lambda_k + lambda_j + s_corr) grad W over the pairs.
+template <bool kTwelve>
+__device__ __forceinline__ float delta_weight(float lk, float lj, float r2, const PaperConsts &c) {
+  return __fmul_rn(__fadd_rn(__fadd_rn(lk, lj), scorr_term<kTwelve>(r2, c)), spiky_factor(r2, c));
+}
 struct DeltaAcc {
   float sx, sy, sz;
   template <bool kTwelve>
   __device__ __forceinline__ void pair(const float4 &qk, const float4 &qj, const PaperConsts &c) {
     const Sep r = separation(qk, qj);
     if (is_pair(r.r2, c.h2)) {
-      const float wgt = __fmul_rn(__fadd_rn(__fadd_rn(qk.w, qj.w), scorr_term<kTwelve>(r.r2, c)),
-                                  spiky_factor(r.r2, c));
+      const float wgt = delta_weight<kTwelve>(qk.w, qj.w, r.r2, c);
       sx = __fmaf_rn(wgt, r.x, sx);
       sy = __fmaf_rn(wgt, r.y, sy);
       sz = __fmaf_rn(wgt, r.z, sz);
@@ -338,12 +341,14 @@ struct DeltaAcc {
 // delta-p, collision response (clamp to the admissible box with the moving
 // x-min wall), Jacobi update of d and p; the last iteration also writes the
 // velocity d/dt and 1/rho for the velocity passes.
-__device__ __forceinline__ void delta_commit(uint32_t k, const DeltaAcc &a, const NbrCtx &nc,
-                                             const PaperConsts &c, float4 *__restrict__ D,
-                                             float4 *__restrict__ P, const float *__restrict__ R,
-                                             float4 *__restrict__ U, int last) {
-  const float4 x = load_own(&nc.X2[k]);
-  const float4 d0 = load_own(&D[k]);
+// (x, d0, rho: the particle's step-start position, displacement and density;
+// rho is only used by the last iteration.)
+template <typename Rho>
+__device__ __forceinline__ void delta_store(uint32_t k, const DeltaAcc &a, const float4 &x,
+                                            const float4 &d0, Rho &&rho, const NbrCtx &nc,
+                                            const PaperConsts &c, float4 *__restrict__ D,
+                                            float4 *__restrict__ P, float4 *__restrict__ U,
+                                            int last) {
   float3 d = make_float3(__fmaf_rn(a.sx, c.inv_rho0, d0.x), __fmaf_rn(a.sy, c.inv_rho0, d0.y),
                          __fmaf_rn(a.sz, c.inv_rho0, d0.z));
   float3 p = add3(x, d);
@@ -359,7 +364,15 @@ __device__ __forceinline__ void delta_commit(uint32_t k, const DeltaAcc &a, cons
   P[k] = make_float4(p.x, p.y, p.z, 0.0f);
   if (last)
     U[k] = make_float4(__fdiv_rn(d.x, c.dt), __fdiv_rn(d.y, c.dt), __fdiv_rn(d.z, c.dt),
-                       __fdiv_rn(1.0f, load_own(&R[k])));
+                       __fdiv_rn(1.0f, rho()));
+}
+__device__ __forceinline__ void delta_commit(uint32_t k, const DeltaAcc &a, const NbrCtx &nc,
+                                             const PaperConsts &c, float4 *__restrict__ D,
+                                             float4 *__restrict__ P, const float *__restrict__ R,
+                                             float4 *__restrict__ U, int last) {
+  const float4 x = load_own(&nc.X2[k]);
+  const float4 d0 = load_own(&D[k]);
+  delta_store(k, a, x, d0, [&] { return load_own(&R[k]); }, nc, c, D, P, U, last);
 }
 
 // A neighbour's (position, velocity) as the velocity passes read it.
@@ -381,27 +394,41 @@ __device__ __forceinline__ float cross_component(float a1, float b2, float a2, f
 // vector eta_k = sum (1/rho_j)(|omega_j| - |omega_k|) grad W is
 // sum (|omega_j|/rho_j) grad W - |omega_k| S_k, so that pass gathers one
 // float4 per neighbour instead of two.
+struct VortTerms {  // one pair's terms: w and s add theirs, X adds wp * u
+  float wx, wy, wz, gx, gy, gz, wp, ux, uy, uz;
+};
+__device__ __forceinline__ VortTerms vort_terms(const Sep &r, const float4 &uk, const float4 &uj,
+                                                const PaperConsts &c) {
+  VortTerms t;
+  const float f = __fmul_rn(spiky_factor(r.r2, c), uj.w);
+  t.gx = __fmul_rn(f, r.x);
+  t.gy = __fmul_rn(f, r.y);
+  t.gz = __fmul_rn(f, r.z);
+  t.ux = __fsub_rn(uj.x, uk.x);
+  t.uy = __fsub_rn(uj.y, uk.y);
+  t.uz = __fsub_rn(uj.z, uk.z);
+  t.wx = cross_component(t.gy, t.uz, t.gz, t.uy);
+  t.wy = cross_component(t.gz, t.ux, t.gx, t.uz);
+  t.wz = cross_component(t.gx, t.uy, t.gy, t.ux);
+  t.wp = __fmul_rn(poly6_value(r.r2, c), uj.w);
+  return t;
+}
 struct VortAcc {
   float wx, wy, wz, sx, sy, sz, xx, xy, xz;
   __device__ __forceinline__ void pair(const float4 &pk, const float4 &uk, const PU &d,
                                        const PaperConsts &c) {
     const Sep r = separation(pk, d.p);
     if (is_pair(r.r2, c.h2)) {
-      const float4 uj = d.u;
-      const float f = __fmul_rn(spiky_factor(r.r2, c), uj.w);
-      const float gx = __fmul_rn(f, r.x), gy = __fmul_rn(f, r.y), gz = __fmul_rn(f, r.z);
-      const float ux = __fsub_rn(uj.x, uk.x), uy = __fsub_rn(uj.y, uk.y),
-                  uz = __fsub_rn(uj.z, uk.z);
-      wx = __fadd_rn(wx, cross_component(gy, uz, gz, uy));
-      wy = __fadd_rn(wy, cross_component(gz, ux, gx, uz));
-      wz = __fadd_rn(wz, cross_component(gx, uy, gy, ux));
-      sx = __fadd_rn(sx, gx);
-      sy = __fadd_rn(sy, gy);
-      sz = __fadd_rn(sz, gz);
-      const float wp = __fmul_rn(poly6_value(r.r2, c), uj.w);
-      xx = __fmaf_rn(wp, ux, xx);
-      xy = __fmaf_rn(wp, uy, xy);
-      xz = __fmaf_rn(wp, uz, xz);
+      const VortTerms t = vort_terms(r, uk, d.u, c);
+      wx = __fadd_rn(wx, t.wx);
+      wy = __fadd_rn(wy, t.wy);
+      wz = __fadd_rn(wz, t.wz);
+      sx = __fadd_rn(sx, t.gx);
+      sy = __fadd_rn(sy, t.gy);
+      sz = __fadd_rn(sz, t.gz);
+      xx = __fmaf_rn(t.wp, t.ux, xx);
+      xy = __fmaf_rn(t.wp, t.uy, xy);
+      xz = __fmaf_rn(t.wp, t.uz, xz);
     }
   }
 };
@@ -438,12 +465,11 @@ struct XsphAcc {
 // eta = E - |omega_k| S_k; v = v + dt f_vorticity + c_xsph X_k with
 // f_vorticity = eps (eta/|eta|) x omega; commits x (.w = |v|), v (.w = mass)
 // and the input index of slot k.
-__device__ __forceinline__ void xsph_commit(uint32_t k, const float4 &pk, const float4 &uk,
-                                            const float4 &wk, const float4 &xs, const float4 &ss,
-                                            const XsphAcc &a, const NbrCtx &nc,
-                                            const PaperConsts &c, const uint32_t *__restrict__ ID2,
-                                            float4 *__restrict__ X, float4 *__restrict__ V,
-                                            uint32_t *__restrict__ ID) {
+__device__ __forceinline__ void xsph_store(uint32_t k, const float4 &pk, const float4 &uk,
+                                           const float4 &wk, const float4 &xs, const float4 &ss,
+                                           const XsphAcc &a, const PaperConsts &c, float mass,
+                                           uint32_t id, float4 *__restrict__ X,
+                                           float4 *__restrict__ V, uint32_t *__restrict__ ID) {
   const float ex = __fmaf_rn(-wk.w, ss.x, a.ex), ey = __fmaf_rn(-wk.w, ss.y, a.ey),
               ez = __fmaf_rn(-wk.w, ss.z, a.ez);
   const float el2 = __fmaf_rn(ez, ez, __fmaf_rn(ey, ey, __fmul_rn(ex, ex)));
@@ -461,8 +487,32 @@ __device__ __forceinline__ void xsph_commit(uint32_t k, const float4 &pk, const 
   const float vy = __fmaf_rn(c.xsph_c, xs.y, __fmaf_rn(c.dt, fy, uk.y));
   const float vz = __fmaf_rn(c.xsph_c, xs.z, __fmaf_rn(c.dt, fz, uk.z));
   X[k] = make_float4(pk.x, pk.y, pk.z, norm3(vx, vy, vz));
-  V[k] = make_float4(vx, vy, vz, load_own(&nc.V2[k]).w);
-  ID[k] = load_own(&ID2[k]);
+  V[k] = make_float4(vx, vy, vz, mass);
+  ID[k] = id;
+}
+
+// The launch arguments shared by the passes over the L1 lists.
+inline Planes make_planes(const float4 *planes, uint32_t n) {
+  const size_t words = plane_floats(n) / 4u;
+  return Planes{planes, planes + words, planes + 2 * words};
+}
+inline NbrCtx make_ctx(const DeviceState &d, const PaperConsts &c, const uint16_t *sid) {
+  NbrCtx nc;
+  nc.nbr4 = d.nbr;
+  nc.cnt = d.nbr_cnt;
+  nc.skeys = d.skeys;
+  nc.off = d.offsets;
+  nc.X2 = d.X2;
+  nc.V2 = d.V2;
+  nc.scenes = d.scenes;
+  nc.sid = sid;
+  nc.err = d.err;
+  nc.cnt_max = d.nbr_max;
+  nc.n = c.n;
+  nc.maxn = c.maxn;
+  nc.dt = c.dt;
+  nc.h2 = c.h2;
+  return nc;
 }
 
 }  // namespace

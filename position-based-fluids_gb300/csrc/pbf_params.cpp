@@ -5,6 +5,7 @@
 // compute_scaling.cl:16, XSPH c = 0.01 at apply_vorticity_and_viscosity.cl:103,
 // gravity -9.81 at predict_positions.cl:8, 4 iterations at
 // src/Simulation.cpp:503).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -279,6 +280,11 @@ int to_gather_tuning(const pbf_tuning &t, GatherTuning *out) {
     return PBF_ERR_INVALID;
   }
   g.masked_build = (uint8_t)t.masked_build;
+  const GatherTuning standard;
+  g.grouped = !g.staged && g.fuse_first == standard.fuse_first &&
+              g.masked_build == standard.masked_build &&
+              std::equal(g.block, g.block + kGatherKinds, standard.block) &&
+              std::equal(g.batch, g.batch + kGatherKinds, standard.batch);
   *out = g;
   return PBF_OK;
 }

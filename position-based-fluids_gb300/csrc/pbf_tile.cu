@@ -566,28 +566,9 @@ __global__ void __launch_bounds__(kThreads, kCtasOne)
     } else {
       visit_neighbours<4>(nc, k, [&](uint32_t j) { return __ldg(&PW[j]); }, pair);
     }
-    xsph_commit(k, pk, load_own(&U[k]), load_own(&Wv[k]), load_own(&XS[k]), load_own(&SS[k]), acc,
-                nc, c, ID2, X, V, ID);
+    xsph_store(k, pk, load_own(&U[k]), load_own(&Wv[k]), load_own(&XS[k]), load_own(&SS[k]), acc,
+               c, load_own(&nc.V2[k]).w, load_own(&ID2[k]), X, V, ID);
   });
-}
-
-NbrCtx make_ctx(const DeviceState &d, const PaperConsts &c, const uint16_t *sid) {
-  NbrCtx nc;
-  nc.nbr4 = d.nbr;
-  nc.cnt = d.nbr_cnt;
-  nc.skeys = d.skeys;
-  nc.off = d.offsets;
-  nc.X2 = d.X2;
-  nc.V2 = d.V2;
-  nc.scenes = d.scenes;
-  nc.sid = sid;
-  nc.err = d.err;
-  nc.cnt_max = d.nbr_max;
-  nc.n = c.n;
-  nc.maxn = c.maxn;
-  nc.dt = c.dt;
-  nc.h2 = c.h2;
-  return nc;
 }
 
 BlockCtx make_blocks(const DeviceState &d, uint32_t nscenes) {

@@ -16,7 +16,8 @@ namespace pbf {
 // shape from the same state, and keeps for every gather pass the shape with
 // the shortest launches.  Then it times whole steps of that choice against
 // the staged tiles (pbf_tile.cu) from the same state and keeps the staged
-// passes when their steps are more than kTuneMargin faster.  The current shapes are timed first and a pass
+// passes when their steps are more than kTuneMargin faster, and for small
+// scenes against the passes with eight threads per particle (pbf_group.cu).  The current shapes are timed first and a pass
 // moves to another shape only when that one is more than kTuneMargin
 // faster: on a near-tie the pick would follow timing noise, and the
 // defaults are the shapes measured fastest over a whole dam break, where
@@ -59,11 +60,12 @@ int paper_autotune(DeviceState &d, uint32_t n, cudaStream_t st, uint32_t trials,
       t.batch[k] = (uint8_t)batch;
     }
     t.fuse_first = (uint8_t)fuse;
+    t.grouped = 0;
     return t;
   };
   const GatherTuning before = d.tune;
   GatherTuning best = before;
-  best.staged = 0;
+  best.staged = best.grouped = 0;
   double best_ms[kGatherKinds];
   for (int k = 0; k < kGatherKinds; ++k) best_ms[k] = std::numeric_limits<double>::infinity();
   // Runs `trials` steps (one, untimed, when !timed) with shapes t from the
@@ -103,7 +105,7 @@ int paper_autotune(DeviceState &d, uint32_t n, cudaStream_t st, uint32_t trials,
       const bool timed = pass == 1;
       if (timed) {
         GatherTuning cur = before;
-        cur.staged = 0;
+        cur.staged = cur.grouped = 0;
         for (int fuse = 0; fuse < 2 && rc == PBF_OK; ++fuse) {
           cur.fuse_first = (uint8_t)fuse;
           if (!trial(cur, true, true)) break;
@@ -121,15 +123,19 @@ int paper_autotune(DeviceState &d, uint32_t n, cudaStream_t st, uint32_t trials,
       for (int k = 0; k < kGatherKinds; ++k)
         per_launch_ms[k] = best_ms[k] < std::numeric_limits<double>::infinity() ? best_ms[k] : 0.0;
     }
-    // whole steps: the L1-gather choice against the staged tiles
+    // whole steps: the L1-gather choice against the staged tiles and, where
+    // they apply, against eight threads per particle (which are what an
+    // untuned scene of that size runs, and so keep their place on a near-tie)
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (rc == PBF_OK && cuda(cudaEventCreate(&e0), "tune events") &&
         cuda(cudaEventCreate(&e1), "tune events")) {
-      GatherTuning staged = best;
-      staged.staged = 1;
-      float step_ms[2] = {0.f, 0.f};
-      for (int v = 0; v < 2 && rc == PBF_OK; ++v) {
-        const GatherTuning &t = v == 0 ? best : staged;
+      GatherTuning variants[3] = {best, best, GatherTuning()};
+      variants[1].staged = 1;
+      variants[2].radix_sort = best.radix_sort;
+      const int count = n <= kGroupParticles ? 3 : 2;
+      float step_ms[3] = {0.f, 0.f, 0.f};
+      for (int v = 0; v < count && rc == PBF_OK; ++v) {
+        const GatherTuning &t = variants[v];
         if (!trial(t, false, false)) break;  // loads the variant's kernels
         if (!copy_state(false)) break;
         d.tune = t;
@@ -140,7 +146,11 @@ int paper_autotune(DeviceState &d, uint32_t n, cudaStream_t st, uint32_t trials,
             !cuda(cudaEventElapsedTime(&step_ms[v], e0, e1), "tune timing"))
           break;
       }
-      if (rc == PBF_OK && step_ms[1] < step_ms[0] * (1.0 - kTuneMargin)) best = staged;
+      if (rc == PBF_OK) {
+        int pick = step_ms[1] < step_ms[0] * (1.0 - kTuneMargin) ? 1 : 0;
+        if (count == 3 && step_ms[pick] >= step_ms[2] * (1.0 - kTuneMargin)) pick = 2;
+        best = variants[pick];
+      }
     }
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
