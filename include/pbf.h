@@ -274,9 +274,9 @@ int pbf_neighbour_stats(pbf_sim *sim, uint32_t *max_count, uint32_t *overflow);
  * neighbour count, and when that comes within 1/8 of the capacity the lists
  * are reallocated to 1.5x the count (at most 1024) before the next step is
  * launched, unless pbf_params.grow_lists is 0.  (Batches and servers keep
- * the capacity they were created with.)  (pbf_step therefore keeps at most two steps queued: before
- * launching a step it waits for the step two back -- the first step's
- * count right after that step -- while the step before still runs.)  No
+ * the capacity they were created with.)  (pbf_step therefore keeps at most 16 steps queued: before
+ * launching a step it waits for the step 16 back -- for the first step's
+ * count right after that step -- and looks at the latest count there is.)  No
  * reference counterpart; grows may be NULL. */
 int pbf_list_capacity(const pbf_sim *sim, uint32_t *capacity, uint32_t *grows);
 /* Staged cell blocks of the last step (PAPER mode with staged = 1 in the

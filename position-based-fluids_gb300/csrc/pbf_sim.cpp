@@ -26,6 +26,14 @@ struct KernelTime {
 };
 }  // namespace
 
+// Steps a simulation keeps queued before pbf_step waits for the oldest.  Two
+// keep the GPU busy with one simulation, but hold the host back from its other
+// ones: three 1,000-particle scenes stepped in turn, eight steps a frame, took
+// 303 us a frame with two steps queued and take 163 with sixteen (32,768
+// particles, four steps: 238 and 173).  A scene that outgrows its lists
+// re-derives its sets in at most that many steps more.
+constexpr uint64_t kCountLag = 16;
+
 struct pbf_sim {
   pbf_params prm{};
   uint32_t n = 0;
@@ -73,15 +81,16 @@ struct pbf_sim {
   bool scene_dirty = false;
   // adaptive neighbour-list capacity (paper): the largest count of each
   // step lands in page-locked memory; before launching a step the host
-  // looks at the count of the step two back (the first step's right after
-  // it) and grows the lists when it came within 1/8 of the capacity
+  // looks at the count of the step kCountLag back, or of a later one that has
+  // run (the first step's right after it), and grows the lists when it came
+  // within 1/8 of the capacity
   uint32_t *nbr_max_host = nullptr;
   // the copy of that count runs on a side branch of the step (forked after
   // the list build, joined at the step's end) so the solver passes do not
   // wait for it
   cudaStream_t count_stream = nullptr;
   cudaEvent_t count_fork = nullptr, count_join = nullptr;
-  cudaEvent_t step_done[2] = {nullptr, nullptr};
+  cudaEvent_t step_done[kCountLag] = {};
   uint64_t launched = 0;  // steps launched since init or the last growth
   uint32_t list_grows = 0;
   // debug views
@@ -466,16 +475,16 @@ int ref_cells(pbf_sim *s, uint32_t *hash, uint32_t *perm, int32_t *ranges) {
 constexpr uint32_t kMaxListCapacity = 1024;
 
 // Before a paper-mode step: the largest neighbour count of a recent step
-// (the first step's right after it, later the step two back, which leaves
-// one step queued on the device while the host waits) against the list
-// capacity.  When it came within 1/8 of the capacity the lists grow to 1.5x
+// (the first step's right after it, later the step kCountLag back or the
+// latest that has run) against the list capacity.  When it came within 1/8 of the capacity the lists grow to 1.5x
 // that count (multiple of 8, at most 1024) before the step is launched, so a
 // scene whose sets outgrow the lists re-derives them from the cells in at
 // most the steps already queued.
 int adapt_lists(pbf_sim *s) {
   if (!s->paper || !s->prm.grow_lists || s->launched == 0) return PBF_OK;
-  const uint64_t wait_for = s->launched >= 2 ? s->launched - 2 : 0;
-  PBF_TRY(cudaEventSynchronize(s->step_done[wait_for & 1]));
+  const uint64_t wait_for = s->launched >= kCountLag ? s->launched - kCountLag : 0;
+  if (s->launched == 1 || s->launched >= kCountLag)
+    PBF_TRY(cudaEventSynchronize(s->step_done[wait_for % kCountLag]));
   const uint32_t mx = *reinterpret_cast<volatile uint32_t *>(s->nbr_max_host);
   const uint32_t cap = s->pc.maxn;
   if (cap >= kMaxListCapacity || mx <= cap - cap / 8) return PBF_OK;
@@ -644,7 +653,7 @@ int pbf_step(pbf_sim *s, uint32_t nsteps) {
       PBF_TRY_STATUS(launch_step(s));
     }
     if (s->paper) {
-      PBF_TRY(cudaEventRecord(s->step_done[s->launched & 1], s->stream));
+      PBF_TRY(cudaEventRecord(s->step_done[s->launched % kCountLag], s->stream));
       ++s->launched;
     }
     s->stepped = true;
