@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kGroupThreads)
             y[dy] = __ldg(planes.y + (j >> 2));
             z[dy] = __ldg(planes.z + (j >> 2));
           }
-          m = four_mask<PaperDistance>(x[dy], y[dy], z[dy], px, py, pz, low, c.h2);
+          m = four_mask<true>(x[dy], y[dy], z[dy], px, py, pz, low, c.h2);
           if (j < a[dy]) m &= ~0u >> (a[dy] - j);
           if (b[dy] - j < 4u) m &= ~(~0u >> (b[dy] - j));
           m >>= 4u * l;

@@ -427,9 +427,8 @@ cudaError_t paper_predict_count(const float4 *X, const float4 *V, uint32_t n,
                                 cudaStream_t st);
 // The list builds read the step-start positions as three planes of
 // plane_floats(n) values (whole 16-byte words).  They live in an array of n
-// float4 that the step only writes later (the vorticity in paper mode, the
-// XSPH velocity change in ref-compat mode), of at least kMinPlaneSlots slots
-// so that the padding of small scenes fits.
+// float4 that is free at that time (W in paper mode, io_pos in ref-compat mode),
+// of at least kMinPlaneSlots slots so that the padding of small scenes fits.
 PBF_HOST_DEVICE inline uint32_t plane_floats(uint32_t n) { return (n + 3u) & ~3u; }
 constexpr size_t kMinPlaneSlots = 16;
 // The state into slot order.  `clear`: the sort left the small cells
@@ -493,7 +492,7 @@ cudaError_t iota_u32(uint32_t *dst, uint32_t n, cudaStream_t st);
 
 // --------------------------------------------------- ref-compat launches --
 // Neighbour lists in the reference's visiting order.  maxn = 0: there was no
-// room for lists (nbr4 and cnt unused), every pass walks the cells.
+// room for lists (nbr4 and cnt unused), delta-p walks the cells.
 struct RefLists {
   const uint4 *nbr4;
   const uint32_t *cnt;
@@ -513,22 +512,19 @@ cudaError_t rc_predict_count(float4 *X, float4 *V, float4 *P, uint32_t n, const 
 // P by slot (PS, and the planes the build reads) and the input index of each
 // slot (ID2); `clear` as in paper_reorder.
 cudaError_t rc_gather(const DeviceState &d, uint32_t n, const StepClear *clear, cudaStream_t st);
-// Neighbour lists of the positions PS.
-cudaError_t rc_build(const float4 *PS, const float4 *planes, const uint32_t *offsets, uint32_t n,
-                     const RefConsts &k, uint32_t maxn, uint4 *nbr, uint32_t *nbr_cnt,
-                     cudaStream_t st);
-// The passes read neighbours by sorted slot (PS, SS, VS) and write their own
-// slot's values there; the last delta-p pass also writes P and V by input
-// index for the commit.
-cudaError_t rc_lambda(float4 *PS, float *SS, const RefLists &lists, const uint32_t *offsets,
-                      uint32_t n, const RefConsts &k, cudaStream_t st);
+// The passes read neighbours by sorted slot (PS, the planes, SS, VS) and write
+// their own slot's values there; lambda leaves the lists that delta-p walks,
+// and the last delta-p pass also writes P and V by input index for the commit.
+cudaError_t rc_lambda(float4 *PS, const float4 *planes, float *SS, const uint32_t *offsets,
+                      uint32_t n, const RefConsts &k, uint32_t maxn, uint4 *nbr,
+                      uint32_t *nbr_cnt, cudaStream_t st);
 cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const RefLists &lists,
                      const uint32_t *input, const uint32_t *offsets, const float4 *X, float4 *V,
                      float4 *P, float4 *VS, float4 *planes, uint32_t n,
                      const RefConsts &k, const SceneDesc *scenes, bool last, cudaStream_t st);
-cudaError_t rc_xsph(const float4 *PS, const float4 *VS, float4 *DV, const RefLists &lists,
-                    const uint32_t *input, const uint32_t *offsets, uint32_t n,
-                    const RefConsts &k, cudaStream_t st);
+cudaError_t rc_xsph(const float4 *PS, const float4 *planes, const float4 *VS, float4 *DV,
+                    const uint32_t *input, const uint32_t *offsets, uint32_t n, const RefConsts &k,
+                    cudaStream_t st);
 cudaError_t rc_commit(float4 *X, float4 *V, const float4 *P, const float4 *DV,
                       uint32_t n, cudaStream_t st);
 

@@ -102,33 +102,29 @@ __device__ __forceinline__ void for_each_listed(const uint4 *__restrict__ nbr4, 
 struct Planes {
   const float4 *x, *y, *z;
 };
+inline Planes make_planes(const float4 *planes, uint32_t n) {
+  const size_t words = plane_floats(n) / 4u;
+  return Planes{planes, planes + words, planes + 2 * words};
+}
 
-// Tests of four candidates at a time against one particle, two per packed
-// instruction (add/mul/fma.rn.f32x2: each half rounded as the scalar
-// instruction rounds it, so the squared distances are the ones the passes
-// compute; (q - p)^2 = (p - q)^2 exactly).
-struct PaperDistance {  // fma(z, z, fma(y, y, x x)), as separation()
-  __device__ __forceinline__ static float2 r2(float2 x, float2 y, float2 z) {
-    return __ffma2_rn(z, z, __ffma2_rn(y, y, __fmul2_rn(x, x)));
-  }
-};
-struct RefDistance {  // (x x + y y) + z z, rounded operator by operator
-  __device__ __forceinline__ static float2 r2(float2 x, float2 y, float2 z) {
-    return __fadd2_rn(__fadd2_rn(__fmul2_rn(x, x), __fmul2_rn(y, y)), __fmul2_rn(z, z));
-  }
-};
+// r^2 of two candidates per packed instruction (add/mul/fma.rn.f32x2: each
+// half rounded as the scalar instruction rounds it, so these are the squared
+// distances separation() gives; (q - p)^2 = (p - q)^2 exactly).
+__device__ __forceinline__ float2 packed_r2(float2 x, float2 y, float2 z) {
+  return __ffma2_rn(z, z, __ffma2_rn(y, y, __fmul2_rn(x, x)));
+}
 
 // Bits 31 - e, e < 4: candidate e of the words has low <= r^2 < h2.
-template <typename Distance, bool kLow = true>
+template <bool kLow>
 __device__ __forceinline__ uint32_t four_mask(const float4 &x, const float4 &y, const float4 &z,
                                               float2 nx, float2 ny, float2 nz, float low,
                                               float h2) {
-  const float2 r01 = Distance::r2(__fadd2_rn(make_float2(x.x, x.y), nx),
-                                  __fadd2_rn(make_float2(y.x, y.y), ny),
-                                  __fadd2_rn(make_float2(z.x, z.y), nz));
-  const float2 r23 = Distance::r2(__fadd2_rn(make_float2(x.z, x.w), nx),
-                                  __fadd2_rn(make_float2(y.z, y.w), ny),
-                                  __fadd2_rn(make_float2(z.z, z.w), nz));
+  const float2 r01 = packed_r2(__fadd2_rn(make_float2(x.x, x.y), nx),
+                               __fadd2_rn(make_float2(y.x, y.y), ny),
+                               __fadd2_rn(make_float2(z.x, z.y), nz));
+  const float2 r23 = packed_r2(__fadd2_rn(make_float2(x.z, x.w), nx),
+                               __fadd2_rn(make_float2(y.z, y.w), ny),
+                               __fadd2_rn(make_float2(z.z, z.w), nz));
   const float r[4] = {r01.x, r01.y, r23.x, r23.y};
   uint32_t m = 0;
 #pragma unroll
@@ -139,7 +135,7 @@ __device__ __forceinline__ uint32_t four_mask(const float4 &x, const float4 &y, 
 
 // Bit 31 - e of the result: candidate c0 + e of [a, b) has low <= r^2 < h2
 // (kLow) or r^2 < h2.  c0 is a multiple of 4, less than b, and a - c0 < 32.
-template <typename Distance, bool kLow>
+template <bool kLow>
 __device__ __forceinline__ uint32_t row_mask(const Planes &p, uint32_t c0, uint32_t a, uint32_t b,
                                              float2 nx, float2 ny, float2 nz, float low,
                                              float h2) {
@@ -149,7 +145,7 @@ __device__ __forceinline__ uint32_t row_mask(const Planes &p, uint32_t c0, uint3
   for (uint32_t g = 0; g < 8; ++g) {
     if (c0 + 4u * g >= b) break;
     const float4 x = __ldg(p.x + w0 + g), y = __ldg(p.y + w0 + g), z = __ldg(p.z + w0 + g);
-    m |= four_mask<Distance, kLow>(x, y, z, nx, ny, nz, low, h2) >> (4 * g);
+    m |= four_mask<kLow>(x, y, z, nx, ny, nz, low, h2) >> (4 * g);
   }
   if (a > c0) m &= ~0u >> (a - c0);
   if (b - c0 < 32u) m &= ~(~0u >> (b - c0));

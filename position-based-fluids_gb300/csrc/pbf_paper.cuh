@@ -295,8 +295,8 @@ __device__ __forceinline__ uint32_t scan_members_planes(const float4 &pk, uint32
       const bool own = (dz | dy) == 0;
       for (uint32_t c0 = a & ~3u; c0 < b; c0 += 32u) {
         const uint32_t m =
-            own ? row_mask<PaperDistance, true>(planes, c0, a, b, px, py, pz, kMinPair2, c.h2)
-                : row_mask<PaperDistance, false>(planes, c0, a, b, px, py, pz, 0.f, c.h2);
+            own ? row_mask<true>(planes, c0, a, b, px, py, pz, kMinPair2, c.h2)
+                : row_mask<false>(planes, c0, a, b, px, py, pz, 0.f, c.h2);
         cnt += (uint32_t)__popc(m);
         list.add(m, c0, word);
       }
@@ -492,10 +492,6 @@ __device__ __forceinline__ void xsph_store(uint32_t k, const float4 &pk, const f
 }
 
 // The launch arguments shared by the passes over the L1 lists.
-inline Planes make_planes(const float4 *planes, uint32_t n) {
-  const size_t words = plane_floats(n) / 4u;
-  return Planes{planes, planes + words, planes + 2 * words};
-}
 inline NbrCtx make_ctx(const DeviceState &d, const PaperConsts &c, const uint16_t *sid) {
   NbrCtx nc;
   nc.nbr4 = d.nbr;

@@ -20,16 +20,17 @@
 // well (PS, VS, SS).
 //
 // The lambda and delta-p passes of one solver iteration evaluate the same
-// pairs: lambda moves nothing.  So each iteration's pairs are found once
-// (k_rc_build: the candidates of the nine rows tested into masks, members
-// stored in visiting order as neighbour lists) and both passes walk the list;
-// the XSPH pass has a list of its own, built at the final positions.  With
-// every pass scanning the 27 cells itself, a warp ran the pair arithmetic
+// pairs: lambda moves nothing.  So the lambda pass finds its members (the
+// candidates of the nine rows tested into masks), sums their terms and leaves
+// them in visiting order as neighbour lists, and the delta-p pass walks the
+// list; the XSPH pass finds its own at the final positions.  With every pass
+// testing and evaluating candidate by candidate, a warp ran the pair arithmetic
 // (square roots and divisions) for nearly every one of ~216 candidates with
 // 15 of 32 lanes active: 572, 537 and 443 us per lambda, delta-p and XSPH
-// pass at 1,048,576 particles, against 157 us per build and 117, 110 and 119 us
-// per pass over the lists.  A particle with more members than the list
-// holds walks the cells in every pass instead.
+// pass at 1,048,576 particles, against 257, 110 and 241 us now (lambda and
+// delta-p issue instructions 73-79% of the time, over 90 per pair; XSPH's
+// gathers keep L1's data path 90% busy).  A particle with more members than
+// the list holds walks the cells in the delta-p pass instead.
 #include "pbf_lists.cuh"
 
 namespace pbf {
@@ -58,8 +59,35 @@ __device__ __forceinline__ void ref_rows(float4 p, const RefConsts &k,
     }
 }
 
-// r^2 > 0 as a lower bound: the smallest positive binary32 number.
-constexpr float kDenormMin = 1.40129846e-45f;
+// The members of slot q (position p) in visiting order, from masks over the
+// position planes, handed on four at a time as word(w, slots); the last word
+// is filled up with q itself.  Returns their number.  The masks only have to
+// hold every member: whoever takes the words applies the reference's own pair
+// test, so r^2 is evaluated with FMAs here (12 packed instructions per four
+// candidates instead of 16, and no lower bound) against an h^2 widened by more
+// than both evaluations can differ, 6 * 2^-24 relative; q itself, which every
+// scan meets, is taken out by its slot.
+template <typename Word>
+__device__ __forceinline__ uint32_t scan_ref_members(uint32_t q, const float4 &p,
+                                                     const RefConsts &k,
+                                                     const uint32_t *__restrict__ off,
+                                                     const Planes &planes, Word &&word) {
+  const float2 px = make_float2(-p.x, -p.x), py = make_float2(-p.y, -p.y),
+               pz = make_float2(-p.z, -p.z);
+  const float h2 = k.h2 * 1.000001f + 1e-44f;
+  MaskQueue<kMaskQueue> list;
+  uint32_t cnt = 0;
+  ref_rows(p, k, off, [&](uint32_t a, uint32_t b) {
+    for (uint32_t c0 = a & ~3u; c0 < b; c0 += 32u) {
+      uint32_t m = row_mask<false>(planes, c0, a, b, px, py, pz, 0.0f, h2);
+      if (q - c0 < 32u) m &= ~(0x80000000u >> (q - c0));
+      cnt += (uint32_t)__popc(m);
+      list.add(m, c0, word);
+    }
+  });
+  list.finish(q, word);
+  return cnt;
+}
 
 // Calls f(load(m)) for the members of slot q in visiting order (and for q
 // itself as padding, which the pair test drops): from the list, or over all
@@ -177,44 +205,19 @@ __global__ void __launch_bounds__(256)
   store_planes(planes, plane, q, p);
 }
 
-// Neighbour lists of the current positions in visiting order, from row masks
-// over the position planes; the rest of the last word holds the particle's
-// own slot.  A set that outgrows the list ends the scan: its passes walk the
-// cells.  (The particle itself and coincident ones can sit in any row here:
-// the cells are the step start's, the rows follow the current position.)
-__global__ void __launch_bounds__(kThreads)
-    k_rc_build(const float4 *__restrict__ PS, Planes planes, const uint32_t *__restrict__ off,
-               uint32_t n, RefConsts k, uint32_t maxn, uint4 *__restrict__ nbr4,
-               uint32_t *__restrict__ nbr_cnt) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const float4 pi = PS[q];
-  const float2 px = make_float2(-pi.x, -pi.x), py = make_float2(-pi.y, -pi.y),
-               pz = make_float2(-pi.z, -pi.z);
-  MaskQueue<kMaskQueue> list;
-  const auto word = [&](uint32_t w, const uint4 &j) {
-    if (4u * w < maxn) nbr4[(size_t)w * n + q] = j;
-  };
-  uint32_t cnt = 0;
-  ref_rows(pi, k, off, [&](uint32_t a, uint32_t b) {
-    for (uint32_t c0 = a & ~3u; c0 < b && cnt <= maxn; c0 += 32u) {
-      const uint32_t m = row_mask<RefDistance, true>(planes, c0, a, b, px, py, pz, kDenormMin, k.h2);
-      cnt += (uint32_t)__popc(m);
-      list.add(m, c0, word);
-    }
-  });
-  list.finish(q, word);
-  nbr_cnt[q] = cnt;
-}
-
-__global__ void __launch_bounds__(kThreads)
-    k_rc_lambda(float4 *__restrict__ PS, float *__restrict__ SS, RefLists lists,
-                const uint32_t *__restrict__ off, uint32_t n, RefConsts k) {
+// Lambda of every particle, and the neighbour lists for the delta-p pass of the
+// iteration: the members of slot q in visiting order, found by row masks,
+// their terms summed as each list word of four is handed on.  (48 registers:
+// 3% faster than the 56 it takes unbounded, which leave 9 CTAs an SM.)
+__global__ void __launch_bounds__(kThreads, 10)
+    k_rc_lambda(float4 *__restrict__ PS, Planes planes, float *__restrict__ SS,
+                const uint32_t *__restrict__ off, uint32_t n, RefConsts k, uint32_t maxn,
+                uint4 *__restrict__ nbr4, uint32_t *__restrict__ nbr_cnt) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const float4 pi = PS[q];
   float dens = 0.0f, gsum = 0.0f, gvx = 0.0f, gvy = 0.0f, gvz = 0.0f;
-  ref_members(q, pi, k, lists, off, [&](uint32_t m) { return PS[m]; }, [&](float4 pj) {
+  const auto pair = [&](const float4 &pj) {
     const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
     const float r2 = rx * rx + ry * ry + rz * rz;
     if (r2 > 0.0f && r2 < k.h2) {
@@ -229,7 +232,15 @@ __global__ void __launch_bounds__(kThreads)
       gvy += gy;
       gvz += gz;
     }
-  });
+  };
+  const uint32_t cnt = scan_ref_members(
+      q, pi, k, off, planes, [&](uint32_t w, const uint4 &j) {
+        if (4u * w < maxn) nbr4[(size_t)w * n + q] = j;
+        const float4 d[4] = {PS[j.x], PS[j.y], PS[j.z], PS[j.w]};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) pair(d[e]);
+      });
+  if (maxn) nbr_cnt[q] = cnt;
   gsum += sqrtf(gvx * gvx + gvy * gvy + gvz * gvz);
   // Only .w changes; concurrent readers use .xyz.
   reinterpret_cast<float *>(&PS[q])[3] = dens;
@@ -295,35 +306,37 @@ __global__ void __launch_bounds__(kThreads)
     v.y = (np.y - x.y) / k.dt;
     v.z = (np.z - x.z) / k.dt;
     V[i] = v;
-    VS[q] = v;
+    VS[q] = make_float4(v.x, v.y, v.z, 1.0f / np.w);
   }
 }
 
 __global__ void __launch_bounds__(kThreads)
-    k_rc_xsph(const float4 *__restrict__ PS, const float4 *__restrict__ VS,
-              float4 *__restrict__ DV, RefLists lists, const uint32_t *__restrict__ input,
+    k_rc_xsph(const float4 *__restrict__ PS, Planes planes, const float4 *__restrict__ VS,
+              float4 *__restrict__ DV, const uint32_t *__restrict__ input,
               const uint32_t *__restrict__ off, uint32_t n, RefConsts k) {
   const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
   const float4 pi = PS[q];
   const float4 vi = VS[q];
   float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-  struct PV {
-    float4 p, v;
-  };
-  ref_members(q, pi, k, lists, off, [&](uint32_t m) { return PV{__ldg(&PS[m]), __ldg(&VS[m])}; },
-              [&](const PV &d) {
-    const float4 pj = d.p, vj = d.v;
+  // vj.w is 1 / density
+  const auto pair = [&](const float4 &pj, const float4 &vj) {
     const float rx = pi.x - pj.x, ry = pi.y - pj.y, rz = pi.z - pj.z;
     const float r2 = rx * rx + ry * ry + rz * rz;
     if (r2 > 0.0f && r2 < k.h2) {
       const float vx = vj.x - vi.x, vy = vj.y - vi.y, vz = vj.z - vi.z;
       const float poly = k.poly6 * (k.h2 - r2) * (k.h2 - r2) * (k.h2 - r2);
-      const float inv = 1.0f / pj.w;
+      const float inv = vj.w;
       sx += inv * vx * poly;
       sy += inv * vy * poly;
       sz += inv * vz * poly;
     }
+  };
+  scan_ref_members(q, pi, k, off, planes, [&](uint32_t, const uint4 &j) {
+    const float4 p[4] = {__ldg(&PS[j.x]), __ldg(&PS[j.y]), __ldg(&PS[j.z]), __ldg(&PS[j.w])};
+    const float4 v[4] = {__ldg(&VS[j.x]), __ldg(&VS[j.y]), __ldg(&VS[j.z]), __ldg(&VS[j.w])};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) pair(p[e], v[e]);
   });
   DV[input[q]] = make_float4(0.01f * sx, 0.01f * sy, 0.01f * sz, 0.0f);
 }
@@ -368,27 +381,19 @@ cudaError_t rc_predict_count(float4 *X, float4 *V, float4 *P, uint32_t n, const 
   return cudaGetLastError();
 }
 
-cudaError_t rc_build(const float4 *PS, const float4 *planes, const uint32_t *offsets, uint32_t n,
-                     const RefConsts &k, uint32_t maxn, uint4 *nbr, uint32_t *nbr_cnt,
-                     cudaStream_t st) {
-  const size_t words = plane_floats(n) / 4u;
-  const Planes p{planes, planes + words, planes + 2 * words};
-  k_rc_build<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, p, offsets, n, k, maxn, nbr,
-                                                           nbr_cnt);
-  return cudaGetLastError();
-}
-
 cudaError_t rc_gather(const DeviceState &d, uint32_t n, const StepClear *clear, cudaStream_t st) {
   const auto kernel = clear ? k_rc_gather<true> : k_rc_gather<false>;
   kernel<<<blocks_for(n, 256), 256, 0, st>>>(d.P, d.perm, d.skeys, d.offsets,
                                              clear ? *clear : StepClear{}, n, d.PS, d.ID2,
-                                             reinterpret_cast<float *>(d.DV), plane_floats(n));
+                                             reinterpret_cast<float *>(d.io_pos), plane_floats(n));
   return cudaGetLastError();
 }
 
-cudaError_t rc_lambda(float4 *PS, float *SS, const RefLists &lists, const uint32_t *offsets,
-                      uint32_t n, const RefConsts &k, cudaStream_t st) {
-  k_rc_lambda<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, SS, lists, offsets, n, k);
+cudaError_t rc_lambda(float4 *PS, const float4 *planes, float *SS, const uint32_t *offsets,
+                      uint32_t n, const RefConsts &k, uint32_t maxn, uint4 *nbr,
+                      uint32_t *nbr_cnt, cudaStream_t st) {
+  k_rc_lambda<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, make_planes(planes, n), SS, offsets,
+                                                            n, k, maxn, nbr, nbr_cnt);
   return cudaGetLastError();
 }
 
@@ -402,10 +407,11 @@ cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const RefLi
   return cudaGetLastError();
 }
 
-cudaError_t rc_xsph(const float4 *PS, const float4 *VS, float4 *DV, const RefLists &lists,
+cudaError_t rc_xsph(const float4 *PS, const float4 *planes, const float4 *VS, float4 *DV,
                     const uint32_t *input, const uint32_t *offsets, uint32_t n, const RefConsts &k,
                     cudaStream_t st) {
-  k_rc_xsph<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, VS, DV, lists, input, offsets, n, k);
+  k_rc_xsph<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, make_planes(planes, n), VS, DV,
+                                                          input, offsets, n, k);
   return cudaGetLastError();
 }
 

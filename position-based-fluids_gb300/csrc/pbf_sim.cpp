@@ -52,7 +52,7 @@ struct pbf_sim {
   SortPlan plan;
   CellSortPlan cplan;  // counting sort by cell
   // ref-compat: counting sort (radix on grids of mostly empty cells) and the
-  // neighbour lists' capacity (0: no lists, every pass walks the cells)
+  // neighbour lists' capacity (0: no lists, delta-p walks the cells)
   bool rc_count_sort = false;
   uint32_t rc_maxn = 0;
   uint32_t ncells = 0;
@@ -296,22 +296,15 @@ int launch_step(pbf_sim *s) {
     float4 *cur = d.PS, *alt = d.PS2;
     const uint32_t iters = s->prm.solver_iterations;
     for (uint32_t it = 0; it < iters; ++it) {
-      if (s->rc_maxn) {
-        PBF_TRY(rc_build(cur, d.DV, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt, st));
-        PBF_TRY_STATUS(mark(s, 1, "rc_build", 1, &ev));
-      }
-      PBF_TRY(rc_lambda(cur, d.SS, lists, d.offsets, n, s->rc, st));
+      PBF_TRY(rc_lambda(cur, d.io_pos, d.SS, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt,
+                        st));
       PBF_TRY_STATUS(mark(s, 1, "rc_lambda", 1, &ev));
-      PBF_TRY(rc_delta(cur, alt, d.SS, lists, d.ID2, d.offsets, d.X, d.V, d.P, d.VS, d.DV, n,
-                       s->rc, d.scenes, it + 1 == iters, st));
+      PBF_TRY(rc_delta(cur, alt, d.SS, lists, d.ID2, d.offsets, d.X, d.V, d.P, d.VS, d.io_pos,
+                       n, s->rc, d.scenes, it + 1 == iters, st));
       PBF_TRY_STATUS(mark(s, 2, "rc_delta", 1, &ev));
       std::swap(cur, alt);
     }
-    if (s->rc_maxn) {
-      PBF_TRY(rc_build(cur, d.DV, d.offsets, n, s->rc, s->rc_maxn, d.nbr, d.nbr_cnt, st));
-      PBF_TRY_STATUS(mark(s, 3, "rc_build", 1, &ev));
-    }
-    PBF_TRY(rc_xsph(cur, d.VS, d.DV, lists, d.ID2, d.offsets, n, s->rc, st));
+    PBF_TRY(rc_xsph(cur, d.io_pos, d.VS, d.DV, d.ID2, d.offsets, n, s->rc, st));
     PBF_TRY_STATUS(mark(s, 3, "rc_xsph", 1, &ev));
     PBF_TRY(rc_commit(d.X, d.V, d.P, d.DV, n, st));
     PBF_TRY_STATUS(mark(s, 3, "rc_commit", 1, &ev));
@@ -367,8 +360,8 @@ int build_graph(pbf_sim *s) {
 // One step with its stage boundaries, captured and launched as a graph.
 int launch_timed_step(pbf_sim *s) {
   // the boundary events exist before the capture (one per mark of a step:
-  // at most 9 outside the solver loop, 3 per iteration)
-  const size_t marks = 16 + 3 * (size_t)s->prm.solver_iterations;
+  // at most 8 outside the solver loop, 2 per iteration)
+  const size_t marks = 16 + 2 * (size_t)s->prm.solver_iterations;
   while (s->events.size() < marks) {
     cudaEvent_t e;
     PBF_TRY(cudaEventCreate(&e));
@@ -566,7 +559,7 @@ int pbf_init(pbf_sim *s) {
   A(&d.sort_scratch, s->plan.words);
   A(&d.err, 1);
   A(&d.scenes, 1);
-  A(&d.io_pos, n);
+  A(&d.io_pos, std::max(n, kMinPlaneSlots));
   A(&d.io_vel, n);
   if (s->paper) {
     A(&d.ID, n);
@@ -590,7 +583,7 @@ int pbf_init(pbf_sim *s) {
     A(&d.PS, n);
     A(&d.PS2, n);
     A(&d.VS, n);
-    A(&d.DV, std::max(n, kMinPlaneSlots));
+    A(&d.DV, n);
     A(&d.SS, n);
     A(&d.ID2, n);
     A(&d.nbr_cnt, n);
@@ -812,7 +805,7 @@ int pbf_launches_per_step(const pbf_sim *s, uint32_t *launches) {
     *launches = 1u /*predict+hash*/ + sort + 1u /*reorder*/ + paper_first_launches(s->d) +
                 2u * it - 1u + 2u;
   else
-    *launches = 1u + sort + 1u /*gather*/ + 2u * it + 2u + (s->rc_maxn ? it + 1u : 0u);
+    *launches = 1u + sort + 1u /*gather*/ + 2u * it + 2u;
   return PBF_OK;
 }
 
