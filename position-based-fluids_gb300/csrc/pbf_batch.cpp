@@ -73,6 +73,7 @@ struct pbf_batch {
   cudaGraphExec_t graph = nullptr;
   bool graph_stale = false;
   std::vector<SceneDesc> table;
+  RenderScratch render;
 };
 
 namespace {
@@ -90,6 +91,7 @@ int balloc(pbf_batch *b, T **p, size_t count) {
 void release(pbf_batch *b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   b->graph = nullptr;
+  b->render.release();
   for (void *p : b->allocations) cudaFree(p);
   b->allocations.clear();
   if (b->stream) cudaStreamDestroy(b->stream);
@@ -551,7 +553,7 @@ int pbf_batch_render_scene(pbf_batch *b, uint32_t scene_id, const pbf_camera *ca
   box.y_max = s.desc.gmin[1] + s.desc.clen[1] * (float)s.desc.ncell[1];
   box.z_max = s.desc.gmin[2] + s.desc.clen[2] * (float)s.desc.ncell[2];
   return render_particles(b->d.X + pb, b->d.ID + pb, s.n, box, *cam, width, height, rgb,
-                          b->stream);
+                          b->render, b->stream);
 }
 
 int pbf_batch_destroy(pbf_batch *b) {

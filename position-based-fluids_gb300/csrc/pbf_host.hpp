@@ -44,10 +44,31 @@ void batch_capacity(const pbf_batch *b, uint32_t *scenes, uint32_t *particles,
 void to_pbf_tuning(const GatherTuning &g, const double trial_ms[kGatherKinds], pbf_tuning *out);
 int to_gather_tuning(const pbf_tuning &t, GatherTuning *out);
 
+// Device memory of the renderer, kept by the simulation or batch it draws
+// (11 bytes per pixel of the largest image so far and 4 per particle):
+// allocating it for every image took 160 us of a 1280 x 720 one.
+struct RenderScratch {
+  void *data = nullptr;
+  size_t bytes = 0;
+  cudaError_t reserve(size_t need) {
+    if (need <= bytes) return cudaSuccess;
+    release();
+    const cudaError_t e = cudaMalloc(&data, need);
+    if (e == cudaSuccess) bytes = need;
+    else data = nullptr;
+    return e;
+  }
+  void release() {
+    if (data) cudaFree(data);
+    data = nullptr;
+    bytes = 0;
+  }
+};
+
 // Renders n particles (X: position, .w = |v|; ID: input index of each slot,
 // or null when slot = input index) of the box of `prm` into rgb (host).
 int render_particles(const float4 *X, const uint32_t *ID, uint32_t n, const pbf_params &prm,
                      const pbf_camera &cam, uint32_t width, uint32_t height, uint8_t *rgb,
-                     cudaStream_t st);
+                     RenderScratch &scratch, cudaStream_t st);
 
 }  // namespace pbf

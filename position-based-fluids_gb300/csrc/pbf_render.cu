@@ -76,13 +76,27 @@ __global__ void k_render_clear(unsigned long long *__restrict__ zbuf, uint32_t p
   if (i < pixels) zbuf[i] = ~0ull;
 }
 
-__global__ void k_render_splat(const float4 *__restrict__ X, const uint32_t *__restrict__ ID,
-                               uint32_t n, RenderView v, unsigned long long *__restrict__ zbuf) {
-  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
+// One sprite by eight threads: a thread's column, and rows eight at a time with
+// each row's coordinate computed by one of the threads -- two divisions per
+// thread and 64 pixels, where a thread per sprite divided twice per pixel.  A
+// pixel is only written when its key beats what is there by now: in a fluid
+// most particles lie behind others, and the atomics on pixels that can no
+// longer change were the cost.  The particles are taken in an order unlike
+// their places, since an order from back to front would still write every
+// pixel every time.  152k particles at 1280 x 720, some 300 pixels each:
+// 322 -> 91 us (99 in slot order), now the reads of the keys from L2.
+constexpr uint32_t kSpriteThreads = 8;
+__global__ void __launch_bounds__(128)
+    k_render_splat(const float4 *__restrict__ X, const uint32_t *__restrict__ ID, uint32_t n,
+                   uint32_t stride, RenderView v, unsigned long long *zbuf) {
+  const uint32_t lane = threadIdx.x & (kSpriteThreads - 1u);
+  const unsigned group = 0xffu << (threadIdx.x & 31u & ~(kSpriteThreads - 1u));
+  const uint32_t i = (blockIdx.x * 128u + threadIdx.x) / kSpriteThreads;
+  if (i >= n) return;
+  const uint32_t k = (uint32_t)((uint64_t)i * stride % n);
   const float4 p = X[k];
   float x, y, z, s;
-  if (!sprite(v, p.x, p.y, p.z, x, y, z, s)) return;
+  if (!sprite(v, p.x, p.y, p.z, x, y, z, s)) return;  // the eight threads alike
   const uint32_t idx = ID ? ID[k] : k;
   const unsigned long long key = ((unsigned long long)__float_as_uint(z) << 32) | idx;
   const int W = (int)v.width, H = (int)v.height;
@@ -91,13 +105,24 @@ __global__ void k_render_splat(const float4 *__restrict__ X, const uint32_t *__r
   const int x1 = min(W - 1, (int)floorf(x + 0.5f * s - 0.5f));
   const int y0 = max(0, (int)ceilf(y - 0.5f * s - 0.5f));
   const int y1 = min(H - 1, (int)floorf(y + 0.5f * s - 0.5f));
-  for (int iy = y0; iy <= y1; ++iy)
-    for (int ix = x0; ix <= x1; ++ix) {
-      float mx, my;
-      point_coord(x, y, s, ix, iy, mx, my);
-      if (mx * mx + my * my > 1.0f) continue;
-      atomicMin(&zbuf[(size_t)iy * W + ix], key);
+  for (int ya = y0; ya <= y1; ya += (int)kSpriteThreads) {
+    float unused, my_lane;
+    point_coord(x, y, s, 0, ya + (int)lane, unused, my_lane);
+    const float my2_lane = my_lane * my_lane;
+    for (int xa = x0; xa <= x1; xa += (int)kSpriteThreads) {
+      const int ix = xa + (int)lane;
+      float mx, unused2;
+      point_coord(x, y, s, ix, 0, mx, unused2);
+      const float mx2 = mx * mx;
+      const int rows = min((int)kSpriteThreads, y1 + 1 - ya);
+      for (int r = 0; r < rows; ++r) {
+        const float my2 = __shfl_sync(group, my2_lane, r, (int)kSpriteThreads);
+        if (ix > x1 || mx2 + my2 > 1.0f) continue;
+        unsigned long long *px = &zbuf[(size_t)(ya + r) * W + ix];
+        if (key < __ldcg(px)) atomicMin(px, key);
+      }
     }
+  }
 }
 
 // Shades every pixel from its winning particle; rows are written top first.
@@ -137,6 +162,22 @@ __global__ void k_render_invert(const uint32_t *__restrict__ ID, uint32_t n,
                                 uint32_t *__restrict__ slot_of) {
   const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) slot_of[min(ID[k], n - 1u)] = k;
+}
+
+// A step through the n particles that visits each once, in an order unlike
+// their places: near 0.618 n and without a common factor.
+uint32_t sprite_stride(uint32_t n) {
+  uint32_t s = (uint32_t)(0.6180339887 * n) | 1u;
+  const auto gcd = [](uint32_t a, uint32_t b) {
+    while (b) {
+      const uint32_t t = a % b;
+      a = b;
+      b = t;
+    }
+    return a;
+  };
+  while (gcd(s, n) != 1u) ++s;
+  return s;
 }
 
 // glm-style column-major 4x4 helpers (host).
@@ -192,9 +233,12 @@ void render_view_matrix(const pbf_camera &cam, float aspect, float out[16]) {
   mat_mul(proj, view, out);
 }
 
+// More scratch than this is not kept from one image to the next.
+constexpr size_t kRenderKeep = (size_t)256 << 20;
+
 int render_particles(const float4 *X, const uint32_t *ID, uint32_t n, const pbf_params &prm,
                      const pbf_camera &cam, uint32_t width, uint32_t height, uint8_t *rgb,
-                     cudaStream_t st) {
+                     RenderScratch &scratch, cudaStream_t st) {
   if (width == 0 || height == 0 || width > 16384 || height > 16384) return PBF_ERR_INVALID;
   RenderView v;
   render_view_matrix(cam, (float)width / (float)height, v.m);
@@ -206,31 +250,28 @@ int render_particles(const float4 *X, const uint32_t *ID, uint32_t n, const pbf_
   v.half[1] = -(prm.y_max - prm.y_min) / 2.0f;
   v.half[2] = -(prm.z_max - prm.z_min) / 2.0f;
   const uint32_t pixels = width * height;
-  unsigned long long *zbuf = nullptr;
-  uint8_t *img = nullptr;
-  uint32_t *slot_of = nullptr;
   int rc = PBF_OK;
   auto cuda = [&](cudaError_t e, const char *where) {
     if (e != cudaSuccess && rc == PBF_OK) rc = cuda_status(e, where);
     return rc == PBF_OK;
   };
-  if (cuda(cudaMallocAsync(&zbuf, (size_t)pixels * 8, st), "render alloc") &&
-      cuda(cudaMallocAsync(&img, (size_t)pixels * 3, st), "render alloc") &&
-      (!ID || cuda(cudaMallocAsync(&slot_of, (size_t)n * 4, st), "render alloc"))) {
-    k_render_clear<<<(pixels + 255) / 256, 256, 0, st>>>(zbuf, pixels);
-    if (ID && n) k_render_invert<<<(n + 255) / 256, 256, 0, st>>>(ID, n, slot_of);
-    if (n) k_render_splat<<<(n + 127) / 128, 128, 0, st>>>(X, ID, n, v, zbuf);
-    k_render_shade<<<(pixels + 255) / 256, 256, 0, st>>>(X, ID, slot_of, n ? n : 1u, v, zbuf,
-                                                          img);
-    if (cuda(cudaGetLastError(), "render launch"))
-      cuda(cudaMemcpyAsync(rgb, img, (size_t)pixels * 3, cudaMemcpyDeviceToHost, st),
-           "render copy");
-    cuda(cudaStreamSynchronize(st), "render sync");
-  }
-  if (zbuf) cudaFreeAsync(zbuf, st);
-  if (img) cudaFreeAsync(img, st);
-  if (slot_of) cudaFreeAsync(slot_of, st);
-  cudaStreamSynchronize(st);
+  // depth keys, image (whole 16-byte words), slot of each input index
+  const size_t img_at = (size_t)pixels * 8, slot_at = img_at + ((size_t)pixels * 3 + 15) / 16 * 16;
+  if (!cuda(scratch.reserve(slot_at + (ID ? (size_t)n * 4 : 0)), "render alloc")) return rc;
+  unsigned char *base = static_cast<unsigned char *>(scratch.data);
+  auto *zbuf = reinterpret_cast<unsigned long long *>(base);
+  uint8_t *img = base + img_at;
+  auto *slot_of = reinterpret_cast<uint32_t *>(base + slot_at);
+  k_render_clear<<<(pixels + 255) / 256, 256, 0, st>>>(zbuf, pixels);
+  if (ID && n) k_render_invert<<<(n + 255) / 256, 256, 0, st>>>(ID, n, slot_of);
+  if (n)
+    k_render_splat<<<(uint32_t)(((uint64_t)n * kSpriteThreads + 127u) / 128u), 128, 0, st>>>(
+        X, ID, n, sprite_stride(n), v, zbuf);
+  k_render_shade<<<(pixels + 255) / 256, 256, 0, st>>>(X, ID, slot_of, n ? n : 1u, v, zbuf, img);
+  if (cuda(cudaGetLastError(), "render launch"))
+    cuda(cudaMemcpyAsync(rgb, img, (size_t)pixels * 3, cudaMemcpyDeviceToHost, st), "render copy");
+  cuda(cudaStreamSynchronize(st), "render sync");
+  if (scratch.bytes > kRenderKeep) scratch.release();
   return rc;
 }
 

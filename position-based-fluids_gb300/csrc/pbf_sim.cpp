@@ -93,6 +93,7 @@ struct pbf_sim {
   cudaEvent_t step_done[kCountLag] = {};
   uint64_t launched = 0;  // steps launched since init or the last growth
   uint32_t list_grows = 0;
+  RenderScratch render;
   // debug views
   int32_t *d_ranges = nullptr;
 };
@@ -127,6 +128,7 @@ void free_all(pbf_sim *s) {
   s->count_stream = nullptr;
   for (cudaEvent_t e : s->events) cudaEventDestroy(e);
   s->events.clear();
+  s->render.release();
   for (void *p : s->allocations) cudaFree(p);
   s->allocations.clear();
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -814,7 +816,7 @@ int pbf_render(pbf_sim *s, const pbf_camera *cam, uint32_t width, uint32_t heigh
   if (!ready(s)) return s ? PBF_ERR_STATE : PBF_ERR_INVALID;
   if (!cam || !rgb) return PBF_ERR_INVALID;
   return render_particles(s->d.X, s->paper ? s->d.ID : nullptr, s->n, s->prm, *cam, width,
-                          height, rgb, s->stream);
+                          height, rgb, s->render, s->stream);
 }
 
 int pbf_autotune(pbf_sim *s, uint32_t trial_steps, pbf_tuning *out) {
