@@ -21,36 +21,67 @@ __device__ __forceinline__ uint32_t scene_cell(float x, float y, float z,
          (uint32_t)s.ncell[0] * ((uint32_t)cy + (uint32_t)s.ncell[1] * (uint32_t)cz);
 }
 
-// Accumulates the per-pass digit histograms (digit_bits wide, pass p's
-// histogram at p << digit_bits) of one key per lane into shared memory,
-// aggregating equal digits within the warp first.
+// One key per lane (whole warp; invalid lanes count nothing) into the per-pass
+// digit histograms in shared memory (digit_bits wide, pass p's at
+// p << digit_bits): one addition where the warp's keys agree in the digit --
+// the upper digits of keys that are nearly in order -- and one per key
+// otherwise.  (Grouping equal digits with __match_any_sync instead cost more
+// than all the rest of the histogram: 21 us of 1M keys' 82 us sort, now 6.5.)
 __device__ __forceinline__ void warp_digit_histogram(uint32_t key, bool valid,
                                                      uint32_t passes, uint32_t digit_bits,
                                                      uint32_t *s_hist) {
-  const unsigned lane = threadIdx.x & 31u;
   const uint32_t mask = (1u << digit_bits) - 1u;
+  const unsigned lanes = __ballot_sync(0xffffffffu, valid);
+  if (lanes == 0u) return;
+  const uint32_t first = __shfl_sync(0xffffffffu, key, __ffs(lanes) - 1);
   for (uint32_t p = 0; p < passes; ++p) {
-    const uint32_t d = (key >> (p * digit_bits)) & mask;
-    const unsigned peers = __match_any_sync(0xffffffffu, valid ? d : 0xffffffffu);
-    if (valid && lane == (unsigned)(__ffs(peers) - 1))
-      atomicAdd(&s_hist[(p << digit_bits) + d], (uint32_t)__popc(peers));
+    const uint32_t shift = p * digit_bits;
+    const uint32_t d = key >> shift & mask, d0 = first >> shift & mask;
+    if (__all_sync(0xffffffffu, !valid || d == d0)) {
+      if ((threadIdx.x & 31u) == 0u)
+        atomicAdd(&s_hist[(p << digit_bits) + d0], (uint32_t)__popc(lanes));
+    } else if (valid) {
+      atomicAdd(&s_hist[(p << digit_bits) + d], 1u);
+    }
   }
 }
 
-// Counts key into counts[] for the counting sort: equal keys of a warp
-// aggregated into one atomic; pos[i] = the particle's place among the
-// increments of its cell (warp lanes in order, warps in atomic order).
-__device__ __forceinline__ void count_cell_key(uint32_t key, bool valid, uint32_t i,
-                                               uint32_t *__restrict__ counts,
-                                               uint32_t *__restrict__ pos) {
+// Counts kKeys keys per lane (whole warp) into counts[] for the counting sort,
+// all their atomics in flight together: one atomic per run of equal keys in
+// neighbouring lanes; pos[i] = the particle's place among the increments of
+// its cell (a run's lanes in order, runs in atomic order).
+template <int kKeys>
+__device__ __forceinline__ void count_cell_keys(const uint32_t (&key)[kKeys],
+                                                const bool (&valid)[kKeys],
+                                                const uint32_t (&i)[kKeys],
+                                                uint32_t *__restrict__ counts,
+                                                uint32_t *__restrict__ pos) {
   const uint32_t lane = threadIdx.x & 31u;
-  const unsigned peers = __match_any_sync(0xffffffffu, valid ? key : 0xffffffffu);
-  const uint32_t leader = (uint32_t)(__ffs(peers) - 1);
-  uint32_t base = 0;
-  if (valid && lane == leader) base = atomicAdd(&counts[key], (uint32_t)__popc(peers));
-  base = __shfl_sync(0xffffffffu, base, (int)leader);
-  if (valid) pos[i] = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+  uint32_t head[kKeys], base[kKeys];
+#pragma unroll
+  for (int u = 0; u < kKeys; ++u) {
+    const uint32_t before = __shfl_up_sync(0xffffffffu, key[u], 1);
+    const bool valid_before = __shfl_up_sync(0xffffffffu, (int)valid[u], 1);
+    const unsigned heads =
+        __ballot_sync(0xffffffffu, lane == 0u || key[u] != before || valid[u] != valid_before);
+    // the caller's run: from the last head at or below its lane to the next one
+    const unsigned below = 0xffffffffu >> (31u - lane);
+    head[u] = 31u - (uint32_t)__clz((int)(heads & below));
+    const unsigned later = heads & ~below;
+    const uint32_t end = later ? (uint32_t)__ffs((int)later) - 1u : 32u;
+    base[u] = 0;
+    if (valid[u] && lane == head[u]) base[u] = atomicAdd(&counts[key[u]], end - head[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < kKeys; ++u) {
+    const uint32_t first = __shfl_sync(0xffffffffu, base[u], (int)head[u]);
+    if (valid[u]) pos[i[u]] = first + (lane - head[u]);
+  }
 }
+// Keys a thread takes at a time in the counting, predicting and scattering
+// kernels of large arrays, which wait on their loads and atomics: 4.2M keys
+// counted in 12 us instead of 18, scattered in 14 instead of 20.
+constexpr int kCountKeys = 4;
 
 // Slot of the particle in unordered slot q once its cell is back in index
 // order: cells of up to kRankCell particles are left as the scatter placed

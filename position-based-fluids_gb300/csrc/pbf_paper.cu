@@ -64,25 +64,38 @@ namespace {
 // ------------------------------------------------------------------------
 // Prediction and cell key of every particle (grid-stride, whole warps
 // iterate together), counted for the counting sort.
+template <int kKeys>
 __global__ void __launch_bounds__(256)
     k_predict_count(const float4 *__restrict__ X, const float4 *__restrict__ V, uint32_t n,
                     PaperConsts c, const SceneDesc *__restrict__ scenes,
                     const uint16_t *__restrict__ sid, uint32_t *__restrict__ keys,
                     uint32_t *__restrict__ counts, uint32_t *__restrict__ pos) {
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
-    const uint32_t k = base + threadIdx.x;
-    const bool valid = k < n;
-    uint32_t key = 0;
-    if (valid) {
-      const float4 x = X[k];
-      const float4 v1 = gravity_velocity(V[k], c.dt, c.gy);
-      const float3 p = add3(x, displacement(v1, c.dt));
-      const SceneDesc &s = scene_of(scenes, sid, k);
-      key = s.cell_base + scene_cell(p.x, p.y, p.z, s);
-      keys[k] = key;
+  const uint32_t stride = gridDim.x * blockDim.x * kKeys;
+  for (uint32_t base = blockIdx.x * blockDim.x * kKeys; base < n; base += stride) {
+    uint32_t k[kKeys], key[kKeys];
+    bool valid[kKeys];
+    float4 x[kKeys], v[kKeys];
+#pragma unroll
+    for (int u = 0; u < kKeys; ++u) {
+      k[u] = base + (uint32_t)u * blockDim.x + threadIdx.x;
+      valid[u] = k[u] < n;
+      if (valid[u]) {
+        x[u] = load_own(&X[k[u]]);
+        v[u] = load_own(&V[k[u]]);
+      }
     }
-    count_cell_key(key, valid, k, counts, pos);
+#pragma unroll
+    for (int u = 0; u < kKeys; ++u) {
+      key[u] = 0;
+      if (valid[u]) {
+        const float4 v1 = gravity_velocity(v[u], c.dt, c.gy);
+        const float3 p = add3(x[u], displacement(v1, c.dt));
+        const SceneDesc &s = scene_of(scenes, sid, k[u]);
+        key[u] = s.cell_base + scene_cell(p.x, p.y, p.z, s);
+        keys[k[u]] = key[u];
+      }
+    }
+    count_cell_keys(key, valid, k, counts, pos);
   }
 }
 
@@ -96,8 +109,8 @@ __global__ void __launch_bounds__(256)
   const uint32_t hist_words = passes << digit_bits;
   for (uint32_t i = threadIdx.x; i < hist_words; i += blockDim.x) s_hist[i] = 0;
   __syncthreads();
-  // Grid-stride over the particles (whole warps iterate together so that
-  // __match_any_sync sees every lane): one histogram flush per CTA.
+  // Grid-stride over the particles (whole warps iterate together): one
+  // histogram flush per CTA.
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
     const uint32_t k = base + threadIdx.x;
@@ -377,7 +390,10 @@ cudaError_t paper_predict_count(const float4 *X, const float4 *V, uint32_t n,
                                 const CellSortPlan &plan, uint32_t *cell_scratch,
                                 cudaStream_t st) {
   if (n == 0) return cudaSuccess;
-  k_predict_count<<<min(blocks_for(n, 256), kStrideCtas), 256, 0, st>>>(
+  // (1.05M particles 12.4 us one at a time, 13.7 four at a time; 4.2M 39 and 36)
+  const bool many = n >= kStrideCtas * 256u * kCountKeys;
+  const auto kernel = many ? k_predict_count<kCountKeys> : k_predict_count<1>;
+  kernel<<<min(blocks_for(n, many ? 256 * kCountKeys : 256), kStrideCtas), 256, 0, st>>>(
       X, V, n, c, scenes, sid, keys, cell_scratch + plan.off_counts, cell_scratch + plan.off_pos);
   return cudaGetLastError();
 }

@@ -151,11 +151,11 @@ __global__ void __launch_bounds__(256)
                        uint32_t *__restrict__ counts, uint32_t *__restrict__ pos) {
   const uint32_t stride = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
-    const uint32_t t = base + threadIdx.x;
-    const bool valid = t < n;
-    uint32_t key = 0;
-    if (valid) keys[t] = key = rc_predict(t, n, X, V, P, k, scenes[0]);
-    count_cell_key(key, valid, t, counts, pos);
+    const uint32_t t[1] = {base + threadIdx.x};
+    const bool valid[1] = {t[0] < n};
+    uint32_t key[1] = {0};
+    if (valid[0]) keys[t[0]] = key[0] = rc_predict(t[0], n, X, V, P, k, scenes[0]);
+    count_cell_keys(key, valid, t, counts, pos);
   }
 }
 

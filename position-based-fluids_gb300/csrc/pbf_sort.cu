@@ -36,6 +36,13 @@ constexpr uint32_t kLbInclusive = 2u << 30;
 constexpr uint32_t kSpinLimit = 1u << 22;
 constexpr int kSortWarps = kSortThreads / 32;
 static_assert(kSortThreads == (1 << kMinDigitBits), "at least one digit per scan thread");
+// A digit pass takes its tile with more threads of fewer keys: the ranking is a
+// serial round per key of a warp, and a tile's time is the pass's latency while
+// there are only a few tiles per SM (1M keys: 245 tiles).
+constexpr int kSweepThreads = 512;
+constexpr int kSweepItems = kSortTile / kSweepThreads;  // 8
+constexpr int kSweepWarps = kSweepThreads / 32;
+static_assert(kSweepThreads >= (1 << kMaxDigitBits), "a thread per digit");
 
 __device__ __forceinline__ uint32_t ld_volatile(const uint32_t *p) {
   return *reinterpret_cast<const volatile uint32_t *>(p);
@@ -44,7 +51,8 @@ __device__ __forceinline__ void st_volatile(uint32_t *p, uint32_t v) {
   *reinterpret_cast<volatile uint32_t *>(p) = v;
 }
 
-// Exclusive scan of one value per thread over a 256-thread block.
+// Exclusive scan of one value per thread over a block of kWarps warps.
+template <int kWarps = kSortWarps>
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v,
                                                          uint32_t *s_warp) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -57,20 +65,24 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v,
   if (lane == 31) s_warp[warp] = incl;
   __syncthreads();
   if (warp == 0) {
-    uint32_t w = lane < kSortWarps ? s_warp[lane] : 0u;
+    uint32_t w = lane < kWarps ? s_warp[lane] : 0u;
     uint32_t wi = w;
 #pragma unroll
-    for (int o = 1; o < kSortWarps; o <<= 1) {
+    for (int o = 1; o < kWarps; o <<= 1) {
       const uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
       if (lane >= o) wi += t;
     }
-    if (lane < kSortWarps) s_warp[lane] = wi - w;
+    if (lane < kWarps) s_warp[lane] = wi - w;
   }
   __syncthreads();
   return incl - v + s_warp[warp];
 }
 
-__global__ void __launch_bounds__(256)
+// Two CTAs per SM: each adds its whole histogram to the global one, so more and
+// smaller CTAs (1216 before) spend their time in those atomics.
+constexpr uint32_t kHistThreads = 512;
+constexpr uint32_t kHistCtas = 152u * 2u;
+__global__ void __launch_bounds__(kHistThreads)
     k_sort_histogram(const uint32_t *__restrict__ keys, uint32_t n,
                      uint32_t passes, uint32_t digit_bits, uint32_t *__restrict__ hist) {
   __shared__ uint32_t s_hist[kMaxHistWords];
@@ -78,8 +90,19 @@ __global__ void __launch_bounds__(256)
   for (uint32_t i = threadIdx.x; i < hist_words; i += blockDim.x) s_hist[i] = 0;
   __syncthreads();
   const uint32_t stride = gridDim.x * blockDim.x;
-  // Whole warps iterate together so that __match_any_sync sees every lane.
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
+  // Whole warps iterate together.  Four keys per thread where the keys are
+  // 16-byte aligned, then the rest one by one.
+  const uint32_t words = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0u ? n >> 2 : 0u;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < words; base += stride) {
+    const uint32_t i = base + threadIdx.x;
+    const bool valid = i < words;
+    const uint4 k = valid ? __ldg(reinterpret_cast<const uint4 *>(keys) + i) : make_uint4(0, 0, 0, 0);
+    warp_digit_histogram(k.x, valid, passes, digit_bits, s_hist);
+    warp_digit_histogram(k.y, valid, passes, digit_bits, s_hist);
+    warp_digit_histogram(k.z, valid, passes, digit_bits, s_hist);
+    warp_digit_histogram(k.w, valid, passes, digit_bits, s_hist);
+  }
+  for (uint32_t base = 4u * words + blockIdx.x * blockDim.x; base < n; base += stride) {
     const uint32_t i = base + threadIdx.x;
     const bool valid = i < n;
     warp_digit_histogram(valid ? keys[i] : 0u, valid, passes, digit_bits, s_hist);
@@ -121,25 +144,29 @@ __global__ void __launch_bounds__(kSortThreads)
 __device__ __forceinline__ uint32_t lookback_prefix(uint32_t *lookback, uint32_t radix,
                                                     uint32_t tile, uint32_t d,
                                                     uint32_t spin_limit, uint32_t *err) {
+  constexpr int kWindow = 4;  // words in flight together: the walk is a chain of L2 reads
   uint32_t excl = 0;
   int t = (int)tile - 1;
   uint32_t spins = 0;
   while (true) {
-    const uint32_t v = ld_volatile(&lookback[(size_t)t * radix + d]);
-    const uint32_t flag = v & ~kLbMask;
-    if (flag == 0u) {
-      if (++spins >= spin_limit) {
-        atomicOr(err, kDevErrLookback);
-        break;
-      }
-      if (spins > 64) __nanosleep(32);
-      continue;
+    uint32_t v[kWindow];
+#pragma unroll
+    for (int w = 0; w < kWindow; ++w)
+      v[w] = t >= w ? ld_volatile(&lookback[(size_t)(t - w) * radix + d]) : kLbInclusive;
+#pragma unroll
+    for (int w = 0; w < kWindow; ++w) {
+      const uint32_t flag = v[w] & ~kLbMask;
+      if (flag == 0u) break;
+      excl += v[w] & kLbMask;
+      if (flag == kLbInclusive) return excl;
+      --t;
     }
-    excl += v & kLbMask;
-    if (flag == kLbInclusive || t == 0) break;
-    --t;
+    if (++spins >= spin_limit) {
+      atomicOr(err, kDevErrLookback);
+      return excl;
+    }
+    if (spins > 64) __nanosleep(32);
   }
-  return excl;
 }
 
 // Runs the look-back wait of one digit against a predecessor tile that
@@ -149,14 +176,30 @@ __global__ void k_wait_selftest(uint32_t *lookback, uint32_t spin_limit, uint32_
   if (threadIdx.x == 0) lookback_prefix(lookback, 1u << kMinDigitBits, 1u, 0u, spin_limit, err);
 }
 
+// The lanes of `lanes` whose kBits-bit digit equals the caller's (whole warp),
+// from a ballot per bit: __match_any_sync takes a round per distinct value and
+// was most of a pass.  1M keys of 18 bits: 25.8 us per pass with it and 8 warps
+// per tile, 18.4 with 16 warps, 16.7 with the ballots; 8M keys 327 -> 190 us
+// for the whole sort.
+template <uint32_t kBits>
+__device__ __forceinline__ unsigned same_digit(uint32_t d, unsigned lanes) {
+#pragma unroll
+  for (uint32_t b = 0; b < kBits; ++b) {
+    const bool one = d >> b & 1u;
+    const unsigned ones = __ballot_sync(0xffffffffu, one);
+    lanes &= one ? ones : ~ones;
+  }
+  return lanes;
+}
+
 // Dynamic shared memory of one digit pass with 2^kBits digits.
 constexpr size_t onesweep_smem_bytes(uint32_t bits) {
-  return ((size_t)kSortWarps * (1u << bits) + 2u * (1u << bits) + 2u * kSortTile) *
+  return ((size_t)kSweepWarps * (1u << bits) + 2u * (1u << bits) + 2u * kSortTile) *
          sizeof(uint32_t);
 }
 
 template <uint32_t kBits, bool kIota>
-__global__ void __launch_bounds__(kSortThreads)
+__global__ void __launch_bounds__(kSweepThreads)
     k_onesweep(const uint32_t *__restrict__ keys_in,
                const uint32_t *__restrict__ vals_in,
                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out,
@@ -164,30 +207,29 @@ __global__ void __launch_bounds__(kSortThreads)
                const uint32_t *__restrict__ global_excl,
                uint32_t *lookback, uint32_t *tile_counter, uint32_t *err) {
   constexpr uint32_t R = 1u << kBits;
-  constexpr uint32_t kDig = R / kSortThreads;  // digits per thread, per-digit phases
   extern __shared__ __align__(16) uint32_t s_dyn[];
-  uint32_t(*s_wcnt)[R] = reinterpret_cast<uint32_t(*)[R]>(s_dyn);  // [kSortWarps][R]
-  uint32_t *s_dexcl = s_dyn + kSortWarps * R;
+  uint32_t(*s_wcnt)[R] = reinterpret_cast<uint32_t(*)[R]>(s_dyn);  // [kSweepWarps][R]
+  uint32_t *s_dexcl = s_dyn + kSweepWarps * R;
   uint32_t *s_gbase = s_dexcl + R;
   uint32_t *s_keys = s_gbase + R;
   uint32_t *s_vals = s_keys + kSortTile;
   __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_warp[kSortWarps];
+  __shared__ uint32_t s_warp[kSweepWarps];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
-  for (uint32_t i = tid; i < kSortWarps * R; i += kSortThreads) (&s_wcnt[0][0])[i] = 0u;
+  for (uint32_t i = tid; i < kSweepWarps * R; i += kSweepThreads) (&s_wcnt[0][0])[i] = 0u;
   __syncthreads();
 
   const uint32_t tile = s_tile;
   const uint32_t tile_base = tile * (uint32_t)kSortTile;
-  // Each warp owns a contiguous segment of 32*kSortItems keys and reads it
+  // Each warp owns a contiguous segment of 32*kSweepItems keys and reads it
   // lane-striped; the warp-local order (item, lane) is the input order.
-  const uint32_t seg = tile_base + (uint32_t)warp * (32u * kSortItems);
+  const uint32_t seg = tile_base + (uint32_t)warp * (32u * kSweepItems);
 
-  uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
+  uint32_t key[kSweepItems], val[kSweepItems], rank[kSweepItems];
 #pragma unroll
-  for (int it = 0; it < kSortItems; ++it) {
+  for (int it = 0; it < kSweepItems; ++it) {
     const uint32_t idx = seg + (uint32_t)it * 32u + lane;
     const bool ok = idx < n;
     key[it] = ok ? keys_in[idx] : 0u;
@@ -198,11 +240,11 @@ __global__ void __launch_bounds__(kSortThreads)
   // the same digit, item by item.
   const unsigned lt_mask = (1u << lane) - 1u;
 #pragma unroll
-  for (int it = 0; it < kSortItems; ++it) {
+  for (int it = 0; it < kSweepItems; ++it) {
     const uint32_t idx = seg + (uint32_t)it * 32u + lane;
     const bool ok = idx < n;
     const uint32_t d = (key[it] >> shift) & (R - 1);
-    const unsigned peers = __match_any_sync(0xffffffffu, ok ? d : 0xffffffffu);
+    const unsigned peers = same_digit<kBits>(d, __ballot_sync(0xffffffffu, ok));
     const uint32_t before = ok ? s_wcnt[warp][d] : 0u;
     __syncwarp();
     rank[it] = before + (uint32_t)__popc(peers & lt_mask);
@@ -212,54 +254,36 @@ __global__ void __launch_bounds__(kSortThreads)
   }
   __syncthreads();
 
-  // Per digit (kDig consecutive digits per thread): the tile's count, and
-  // each warp's exclusive offset.
-  uint32_t tile_count[kDig], excl[kDig];
-  uint32_t sum = 0;
+  // Per digit (one thread each): the tile's count, and each warp's exclusive
+  // offset.
+  const uint32_t d = (uint32_t)tid;
+  uint32_t tile_count = 0, excl = 0;
+  if (d < R) {
 #pragma unroll
-  for (uint32_t j = 0; j < kDig; ++j) {
-    const uint32_t d = (uint32_t)tid * kDig + j;
-    uint32_t c = 0;
-#pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
+    for (int w = 0; w < kSweepWarps; ++w) {
       const uint32_t x = s_wcnt[w][d];
-      s_wcnt[w][d] = c;
-      c += x;
+      s_wcnt[w][d] = tile_count;
+      tile_count += x;
     }
-    tile_count[j] = c;
-    excl[j] = 0;
-    sum += c;
-  }
-
-  // Decoupled look-back: publish every aggregate before waiting on any.
-  if (tile == 0) {
-#pragma unroll
-    for (uint32_t j = 0; j < kDig; ++j)
-      st_volatile(&lookback[(uint32_t)tid * kDig + j], kLbInclusive | tile_count[j]);
-  } else {
-    uint32_t *mine = lookback + (size_t)tile * R + (uint32_t)tid * kDig;
-#pragma unroll
-    for (uint32_t j = 0; j < kDig; ++j) st_volatile(&mine[j], kLbAggregate | tile_count[j]);
-#pragma unroll
-    for (uint32_t j = 0; j < kDig; ++j) {
-      excl[j] = lookback_prefix(lookback, R, tile, (uint32_t)tid * kDig + j, kSpinLimit, err);
-      st_volatile(&mine[j], kLbInclusive | ((excl[j] + tile_count[j]) & kLbMask));
+    // decoupled look-back
+    uint32_t *mine = lookback + (size_t)tile * R + d;
+    st_volatile(mine, (tile == 0 ? kLbInclusive : kLbAggregate) | tile_count);
+    if (tile != 0) {
+      excl = lookback_prefix(lookback, R, tile, d, kSpinLimit, err);
+      st_volatile(mine, kLbInclusive | ((excl + tile_count) & kLbMask));
     }
   }
-  uint32_t e = block_exclusive_scan(sum, s_warp);
-#pragma unroll
-  for (uint32_t j = 0; j < kDig; ++j) {
-    const uint32_t d = (uint32_t)tid * kDig + j;
-    s_gbase[d] = global_excl[d] + excl[j];
+  const uint32_t e = block_exclusive_scan<kSweepWarps>(tile_count, s_warp);
+  if (d < R) {
+    s_gbase[d] = global_excl[d] + excl;
     s_dexcl[d] = e;
-    e += tile_count[j];
   }
   __syncthreads();
 
   // Stage the tile in digit order in shared memory, then write it out with
   // consecutive threads on consecutive destinations.
 #pragma unroll
-  for (int it = 0; it < kSortItems; ++it) {
+  for (int it = 0; it < kSweepItems; ++it) {
     const uint32_t idx = seg + (uint32_t)it * 32u + lane;
     if (idx < n) {
       const uint32_t dg = (key[it] >> shift) & (R - 1);
@@ -270,7 +294,7 @@ __global__ void __launch_bounds__(kSortThreads)
   }
   __syncthreads();
   const uint32_t tile_n = min((uint32_t)kSortTile, n - tile_base);
-  for (uint32_t i = tid; i < tile_n; i += kSortThreads) {
+  for (uint32_t i = tid; i < tile_n; i += kSweepThreads) {
     const uint32_t k = s_keys[i];
     const uint32_t dg = (k >> shift) & (R - 1);
     const uint32_t dst = s_gbase[dg] + (i - s_dexcl[dg]);
@@ -314,10 +338,10 @@ void launch_onesweep(bool iota, uint32_t tiles, cudaStream_t stream, const uint3
                      uint32_t *err) {
   const size_t smem = onesweep_smem_bytes(kBits);
   if (iota)
-    k_onesweep<kBits, true><<<tiles, kSortThreads, smem, stream>>>(ksrc, nullptr, kdst, vdst, n,
+    k_onesweep<kBits, true><<<tiles, kSweepThreads, smem, stream>>>(ksrc, nullptr, kdst, vdst, n,
                                                                   shift, hist, lb, ctr, err);
   else
-    k_onesweep<kBits, false><<<tiles, kSortThreads, smem, stream>>>(ksrc, vsrc, kdst, vdst, n,
+    k_onesweep<kBits, false><<<tiles, kSweepThreads, smem, stream>>>(ksrc, vsrc, kdst, vdst, n,
                                                                    shift, hist, lb, ctr, err);
 }
 
@@ -567,20 +591,32 @@ __global__ void __launch_bounds__(kSortThreads)
   }
 }
 
-// Every particle at its cell's offset plus its place among the cell's.
+// Every particle at its cell's offset plus its place among the cell's (four
+// per thread where one per thread would be several waves of CTAs).
+template <int kKeys>
 __global__ void __launch_bounds__(256)
     k_count_scatter(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ pos,
                     const uint32_t *__restrict__ off, uint32_t n, uint32_t ncells,
                     uint32_t *__restrict__ skeys, uint32_t *__restrict__ perm) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t k = keys[i];
-  if (k >= ncells) return;  // not counted (error flag set)
-  const uint32_t d = off[k] + pos[i];
-  // always true unless the scan's look-back gave up (error flag set)
-  if (d < n) {
-    skeys[d] = k;
-    perm[d] = i;
+  // kKeys keys per thread, their loads in flight together
+  const uint32_t first = blockIdx.x * blockDim.x * kKeys + threadIdx.x;
+  uint32_t k[kKeys], place[kKeys], d[kKeys];
+#pragma unroll
+  for (int u = 0; u < kKeys; ++u) {
+    const uint32_t i = first + (uint32_t)u * blockDim.x;
+    k[u] = i < n ? __ldg(&keys[i]) : 0xffffffffu;
+    place[u] = i < n ? __ldg(&pos[i]) : 0u;
+  }
+#pragma unroll
+  for (int u = 0; u < kKeys; ++u)  // a key not below ncells was not counted (error flag set)
+    d[u] = k[u] < ncells ? __ldg(&off[k[u]]) + place[u] : 0xffffffffu;
+#pragma unroll
+  for (int u = 0; u < kKeys; ++u) {
+    // always true unless the scan's look-back gave up (error flag set)
+    if (d[u] < n) {
+      skeys[d[u]] = k[u];
+      perm[d[u]] = first + (uint32_t)u * blockDim.x;
+    }
   }
 }
 
@@ -589,13 +625,21 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_count_keys(const uint32_t *__restrict__ keys, uint32_t n, uint32_t ncells,
                  uint32_t *__restrict__ counts, uint32_t *__restrict__ pos, uint32_t *err) {
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
-    const uint32_t i = base + threadIdx.x;
-    const uint32_t key = i < n ? keys[i] : 0u;
-    const bool valid = i < n && key < ncells;
-    if (i < n && !valid) atomicOr(err, kDevErrKey);
-    count_cell_key(key, valid, i, counts, pos);
+  const uint32_t stride = gridDim.x * blockDim.x * kCountKeys;
+  for (uint32_t base = blockIdx.x * blockDim.x * kCountKeys; base < n; base += stride) {
+    uint32_t i[kCountKeys], key[kCountKeys];
+    bool valid[kCountKeys];
+#pragma unroll
+    for (int u = 0; u < kCountKeys; ++u) {
+      i[u] = base + (uint32_t)u * blockDim.x + threadIdx.x;
+      key[u] = i[u] < n ? keys[i[u]] : 0u;
+    }
+#pragma unroll
+    for (int u = 0; u < kCountKeys; ++u) {
+      valid[u] = i[u] < n && key[u] < ncells;
+      if (i[u] < n && !valid[u]) atomicOr(err, kDevErrKey);
+    }
+    count_cell_keys(key, valid, i, counts, pos);
   }
 }
 
@@ -655,16 +699,19 @@ __global__ void __launch_bounds__(256)
     }
     return;
   }
+  // four indices in flight at a time (past the cell's end its last one)
   uint32_t prev = perm[a];
   bool sorted = true;
 #pragma unroll 1
-  for (uint32_t j = 1; j < m; ++j) {
-    const uint32_t x = perm[a + j];
-    if (x < prev) {
-      sorted = false;
-      break;
+  for (uint32_t j = 1; j < m && sorted; j += 4) {
+    uint32_t x[4];
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) x[e] = perm[a + min(j + e, m - 1u)];
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) {
+      sorted = sorted && x[e] >= prev;
+      prev = x[e];
     }
-    prev = x;
   }
   if (sorted) return;
   if (kSortHere) {
@@ -820,8 +867,8 @@ cudaError_t sort_clear(const SortPlan &plan, uint32_t *scratch,
 cudaError_t sort_histogram(const SortPlan &plan, const uint32_t *keys,
                            uint32_t *scratch, cudaStream_t stream) {
   if (plan.n == 0) return cudaSuccess;
-  const uint32_t blocks = min(blocks_for(plan.n, 256), kStrideCtas);
-  k_sort_histogram<<<blocks, 256, 0, stream>>>(keys, plan.n, plan.passes, plan.digit_bits,
+  const uint32_t blocks = min(blocks_for(plan.n, kHistThreads), kHistCtas);
+  k_sort_histogram<<<blocks, kHistThreads, 0, stream>>>(keys, plan.n, plan.passes, plan.digit_bits,
                                                scratch + plan.off_hist);
   return cudaGetLastError();
 }
@@ -995,7 +1042,9 @@ static cudaError_t scan_and_scatter(const CellSortPlan &plan, const uint32_t *ke
       scratch + plan.off_big, plan.big_cap, scratch + plan.off_huge, plan.huge_cap);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || plan.n == 0) return e;
-  k_count_scatter<<<blocks_for(plan.n, 256), 256, 0, stream>>>(
+  const bool many = plan.n > kStrideCtas * 256u;
+  const auto scatter = many ? k_count_scatter<kCountKeys> : k_count_scatter<1>;
+  scatter<<<blocks_for(plan.n, many ? 256 * kCountKeys : 256), 256, 0, stream>>>(
       keys, scratch + plan.off_pos, offsets, plan.n, plan.ncells, skeys, perm);
   return cudaGetLastError();
 }
@@ -1046,7 +1095,7 @@ cudaError_t cell_sort_finish(const CellSortPlan &plan, const uint32_t *keys, uin
 cudaError_t cell_sort_count(const CellSortPlan &plan, const uint32_t *keys, uint32_t *scratch,
                             uint32_t *err, cudaStream_t stream) {
   if (plan.n == 0) return cudaSuccess;
-  k_count_keys<<<min(blocks_for(plan.n, 256), kStrideCtas), 256, 0, stream>>>(
+  k_count_keys<<<min(blocks_for(plan.n, 256 * kCountKeys), kStrideCtas), 256, 0, stream>>>(
       keys, plan.n, plan.ncells, scratch + plan.off_counts, scratch + plan.off_pos, err);
   return cudaGetLastError();
 }
