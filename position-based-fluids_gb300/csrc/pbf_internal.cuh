@@ -466,6 +466,15 @@ constexpr uint32_t kGroupParticles = 16384;
 inline bool use_groups(const DeviceState &d, const PaperConsts &c) {
   return d.tune.grouped && c.n <= kGroupParticles;
 }
+// The whole step as one launch of one cluster, for scenes of up to
+// kTinyParticles particles in kTinyCells cells (everything its passes gather
+// lies in shared memory).  tiny_cluster: how many particles the device's
+// largest cluster takes (0: the step is run pass by pass).
+constexpr uint32_t kTinyParticles = 1024;
+constexpr uint32_t kTinyCells = 6144;
+uint32_t tiny_cluster();
+cudaError_t tiny_step(const DeviceState &d, const PaperConsts &c, uint32_t ncells,
+                      uint32_t iterations, uint32_t *host_max, cudaStream_t st);
 cudaError_t group_nbr_lambda(const DeviceState &d, const PaperConsts &c, const uint16_t *sid,
                              cudaStream_t st);
 cudaError_t group_lambda(const DeviceState &d, const PaperConsts &c, const uint16_t *sid,

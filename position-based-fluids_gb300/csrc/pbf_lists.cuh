@@ -91,6 +91,21 @@ __device__ __forceinline__ void for_each_listed(const uint4 *__restrict__ nbr4, 
   }
 }
 
+// How a pass loads what it gathers: through the read-only path when an earlier
+// kernel wrote it, from L2 when an earlier phase of the same kernel did.
+struct EarlierKernel {
+  template <typename T>
+  __device__ __forceinline__ static T ld(const T *p) {
+    return __ldg(p);
+  }
+};
+struct EarlierPhase {
+  template <typename T>
+  __device__ __forceinline__ static T ld(const T *p) {
+    return __ldcg(p);
+  }
+};
+
 // Positions as three planes (x, y, z), four values per 16-byte word, each plane
 // padded to whole words: the list builds test four candidates per three loads
 // in 23 instructions (12 of them packed), where the scalar test of one float4
@@ -135,7 +150,7 @@ __device__ __forceinline__ uint32_t four_mask(const float4 &x, const float4 &y, 
 
 // Bit 31 - e of the result: candidate c0 + e of [a, b) has low <= r^2 < h2
 // (kLow) or r^2 < h2.  c0 is a multiple of 4, less than b, and a - c0 < 32.
-template <bool kLow>
+template <bool kLow, typename Mem = EarlierKernel>
 __device__ __forceinline__ uint32_t row_mask(const Planes &p, uint32_t c0, uint32_t a, uint32_t b,
                                              float2 nx, float2 ny, float2 nz, float low,
                                              float h2) {
@@ -144,7 +159,7 @@ __device__ __forceinline__ uint32_t row_mask(const Planes &p, uint32_t c0, uint3
 #pragma unroll
   for (uint32_t g = 0; g < 8; ++g) {
     if (c0 + 4u * g >= b) break;
-    const float4 x = __ldg(p.x + w0 + g), y = __ldg(p.y + w0 + g), z = __ldg(p.z + w0 + g);
+    const float4 x = Mem::ld(p.x + w0 + g), y = Mem::ld(p.y + w0 + g), z = Mem::ld(p.z + w0 + g);
     m |= four_mask<kLow>(x, y, z, nx, ny, nz, low, h2) >> (4 * g);
   }
   if (a > c0) m &= ~0u >> (a - c0);

@@ -57,8 +57,9 @@ __device__ __forceinline__ float3 add3(float4 x, float3 d) {
 }
 
 // Step-start predicted position of slot j (as written by the reorder).
+template <typename Mem = EarlierKernel>
 __device__ __forceinline__ float3 start_position(const NbrCtx &c, uint32_t j) {
-  return add3(__ldg(&c.X2[j]), displacement(__ldg(&c.V2[j]), c.dt));
+  return add3(Mem::ld(&c.X2[j]), displacement(Mem::ld(&c.V2[j]), c.dt));
 }
 
 // Particles j != k closer than h form a pair.  Distances below
@@ -93,7 +94,7 @@ __device__ __forceinline__ Sep separation(const float3 &a, const float3 &b) {
 
 // Visits the 9 rows around the cell with key `key` (order: dz, dy, slot);
 // f(q, j) gets the row index q = (dz+1)*3 + (dy+1) and the slot j != k.
-template <typename F>
+template <typename Mem = EarlierKernel, typename F>
 __device__ __forceinline__ void scan_rows(uint32_t k, uint32_t key, const SceneDesc &s,
                                           const uint32_t *__restrict__ off, F &&f) {
   const int nx = s.ncell[0], ny = s.ncell[1], nz = s.ncell[2];
@@ -112,8 +113,8 @@ __device__ __forceinline__ void scan_rows(uint32_t k, uint32_t key, const SceneD
       if (y < 0 || y >= ny) continue;
       const int q = (dz + 1) * 3 + (dy + 1);
       const uint32_t row = s.cell_base + (uint32_t)nx * ((uint32_t)y + (uint32_t)ny * (uint32_t)z);
-      const uint32_t a = __ldg(&off[row + x0]);
-      const uint32_t b = __ldg(&off[row + x1 + 1]);
+      const uint32_t a = Mem::ld(&off[row + x0]);
+      const uint32_t b = Mem::ld(&off[row + x1 + 1]);
       for (uint32_t j = a; j < b; ++j)
         if (j != k) f(q, j);
     }
@@ -121,12 +122,12 @@ __device__ __forceinline__ void scan_rows(uint32_t k, uint32_t key, const SceneD
 }
 
 // Re-derives N_k from the cells and the step-start positions (global loads).
-template <typename F>
+template <typename Mem = EarlierKernel, typename F>
 __device__ __forceinline__ void visit_fallback(const NbrCtx &c, uint32_t k, F &&f) {
   const SceneDesc &sc = scene_of(c.scenes, c.sid, k);
-  const float3 pk = start_position(c, k);
-  scan_rows(k, __ldg(&c.skeys[k]), sc, c.off, [&](int, uint32_t j) {
-    if (is_pair(separation(pk, start_position(c, j)).r2, c.h2)) f(j);
+  const float3 pk = start_position<Mem>(c, k);
+  scan_rows<Mem>(k, Mem::ld(&c.skeys[k]), sc, c.off, [&](int, uint32_t j) {
+    if (is_pair(separation(pk, start_position<Mem>(c, j)).r2, c.h2)) f(j);
   });
 }
 
@@ -265,7 +266,7 @@ __device__ __forceinline__ void scan_members(const float4 &pk, uint32_t key, con
 // zero as well.  The candidate loop is 23 instructions per four candidates
 // (12 of them packed), where one candidate at a time with its member work
 // inside took about 18 each.
-template <typename Word>
+template <typename Mem = EarlierKernel, typename Word>
 __device__ __forceinline__ uint32_t scan_members_planes(const float4 &pk, uint32_t k, uint32_t key,
                                                         const SceneDesc &s,
                                                         const uint32_t *__restrict__ off,
@@ -290,13 +291,13 @@ __device__ __forceinline__ uint32_t scan_members_planes(const float4 &pk, uint32
       const int y = cy + dy;
       if (y < 0 || y >= ny) continue;
       const uint32_t row = s.cell_base + (uint32_t)nx * ((uint32_t)y + (uint32_t)ny * (uint32_t)z);
-      const uint32_t a = __ldg(&off[row + x0]);
-      const uint32_t b = __ldg(&off[row + x1 + 1]);
+      const uint32_t a = Mem::ld(&off[row + x0]);
+      const uint32_t b = Mem::ld(&off[row + x1 + 1]);
       const bool own = (dz | dy) == 0;
       for (uint32_t c0 = a & ~3u; c0 < b; c0 += 32u) {
         const uint32_t m =
-            own ? row_mask<true>(planes, c0, a, b, px, py, pz, kMinPair2, c.h2)
-                : row_mask<false>(planes, c0, a, b, px, py, pz, 0.f, c.h2);
+            own ? row_mask<true, Mem>(planes, c0, a, b, px, py, pz, kMinPair2, c.h2)
+                : row_mask<false, Mem>(planes, c0, a, b, px, py, pz, 0.f, c.h2);
         cnt += (uint32_t)__popc(m);
         list.add(m, c0, word);
       }
@@ -341,18 +342,15 @@ struct DeltaAcc {
 // delta-p, collision response (clamp to the admissible box with the moving
 // x-min wall), Jacobi update of d and p; the last iteration also writes the
 // velocity d/dt and 1/rho for the velocity passes.
-// (x, d0, rho: the particle's step-start position, displacement and density;
-// rho is only used by the last iteration.)
-template <typename Rho>
-__device__ __forceinline__ void delta_store(uint32_t k, const DeltaAcc &a, const float4 &x,
-                                            const float4 &d0, Rho &&rho, const NbrCtx &nc,
-                                            const PaperConsts &c, float4 *__restrict__ D,
-                                            float4 *__restrict__ P, float4 *__restrict__ U,
-                                            int last) {
+struct Moved {
+  float3 d, p;
+};
+// (x, d0: the particle's step-start position and displacement.)
+__device__ __forceinline__ Moved delta_moved(const DeltaAcc &a, const float4 &x, const float4 &d0,
+                                             const SceneDesc &sc, const PaperConsts &c) {
   float3 d = make_float3(__fmaf_rn(a.sx, c.inv_rho0, d0.x), __fmaf_rn(a.sy, c.inv_rho0, d0.y),
                          __fmaf_rn(a.sz, c.inv_rho0, d0.z));
   float3 p = add3(x, d);
-  const SceneDesc &sc = scene_of(nc.scenes, nc.sid, k);
   const float lo_x = __fadd_rn(sc.lo[0], sc.wave);
   if (p.x < lo_x) { d.x = __fsub_rn(lo_x, x.x); p.x = __fadd_rn(x.x, d.x); }
   else if (p.x > sc.hi[0]) { d.x = __fsub_rn(sc.hi[0], x.x); p.x = __fadd_rn(x.x, d.x); }
@@ -360,11 +358,23 @@ __device__ __forceinline__ void delta_store(uint32_t k, const DeltaAcc &a, const
   else if (p.y > sc.hi[1]) { d.y = __fsub_rn(sc.hi[1], x.y); p.y = __fadd_rn(x.y, d.y); }
   if (p.z < sc.lo[2]) { d.z = __fsub_rn(sc.lo[2], x.z); p.z = __fadd_rn(x.z, d.z); }
   else if (p.z > sc.hi[2]) { d.z = __fsub_rn(sc.hi[2], x.z); p.z = __fadd_rn(x.z, d.z); }
-  D[k] = make_float4(d.x, d.y, d.z, 0.0f);
-  P[k] = make_float4(p.x, p.y, p.z, 0.0f);
-  if (last)
-    U[k] = make_float4(__fdiv_rn(d.x, c.dt), __fdiv_rn(d.y, c.dt), __fdiv_rn(d.z, c.dt),
-                       __fdiv_rn(1.0f, rho()));
+  return Moved{d, p};
+}
+// Velocity d/dt and 1/rho.
+__device__ __forceinline__ float4 delta_velocity(const float3 &d, float rho, const PaperConsts &c) {
+  return make_float4(__fdiv_rn(d.x, c.dt), __fdiv_rn(d.y, c.dt), __fdiv_rn(d.z, c.dt),
+                     __fdiv_rn(1.0f, rho));
+}
+template <typename Rho>
+__device__ __forceinline__ void delta_store(uint32_t k, const DeltaAcc &a, const float4 &x,
+                                            const float4 &d0, Rho &&rho, const NbrCtx &nc,
+                                            const PaperConsts &c, float4 *__restrict__ D,
+                                            float4 *__restrict__ P, float4 *__restrict__ U,
+                                            int last) {
+  const Moved m = delta_moved(a, x, d0, scene_of(nc.scenes, nc.sid, k), c);
+  D[k] = make_float4(m.d.x, m.d.y, m.d.z, 0.0f);
+  P[k] = make_float4(m.p.x, m.p.y, m.p.z, 0.0f);
+  if (last) U[k] = delta_velocity(m.d, rho(), c);
 }
 __device__ __forceinline__ void delta_commit(uint32_t k, const DeltaAcc &a, const NbrCtx &nc,
                                              const PaperConsts &c, float4 *__restrict__ D,

@@ -94,6 +94,7 @@ struct pbf_sim {
   uint64_t launched = 0;  // steps launched since init or the last growth
   uint32_t list_grows = 0;
   RenderScratch render;
+  uint32_t tiny_particles = 0;  // paper: scenes up to this size step in one launch
   // debug views
   int32_t *d_ranges = nullptr;
 };
@@ -196,8 +197,22 @@ cudaError_t join_count_copy(pbf_sim *s) {
   return cudaStreamWaitEvent(s->stream, s->count_join, 0);
 }
 
+// Whether the step runs as one launch (pbf_group.cu).  Timed steps report the
+// time of each pass and run them one by one; the bits are the same.
+bool use_tiny(const pbf_sim *s) {
+  const GatherTuning &t = s->d.tune;
+  return s->paper && t.grouped && !t.radix_sort && !s->timing && !s->timed_capture &&
+         s->n <= s->tiny_particles && s->ncells <= kTinyCells;
+}
+
 int launch_step(pbf_sim *s) {
   DeviceState &d = s->d;
+  if (use_tiny(s)) {
+    PBF_TRY(tiny_step(d, s->pc, s->ncells, s->prm.solver_iterations, s->nbr_max_host,
+                      s->stream));
+    s->events_used = 0;
+    return PBF_OK;
+  }
   const cudaStream_t st = s->stream;
   const uint32_t n = s->n;
   const uint32_t passes = s->plan.passes;
@@ -594,6 +609,7 @@ int pbf_init(pbf_sim *s) {
   }
   if (rc == PBF_OK && s->paper) {
     cudaError_t te = tile_init();
+    if (s->n <= kTinyParticles) s->tiny_particles = tiny_cluster();
     if (te == cudaSuccess) te = cudaMallocHost(&s->nbr_max_host, sizeof(uint32_t));
     for (cudaEvent_t &e : s->step_done)
       if (te == cudaSuccess) te = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
@@ -800,6 +816,10 @@ int pbf_set_graph(pbf_sim *s, int enable) {
 int pbf_launches_per_step(const pbf_sim *s, uint32_t *launches) {
   if (!s || !launches) return PBF_ERR_INVALID;
   const uint32_t it = s->prm.solver_iterations;
+  if (use_tiny(s)) {
+    *launches = 1u;
+    return PBF_OK;
+  }
   const uint32_t sort = (s->paper ? !s->d.tune.radix_sort : s->rc_count_sort)
                             ? kCellPlaceLaunches
                             : 1u /*scan*/ + s->plan.passes + (s->offset_runs ? 2u : 1u) /*offsets*/;
