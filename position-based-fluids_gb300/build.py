@@ -39,7 +39,7 @@ CU_SOURCES = ["pbf_sort.cu", "pbf_paper.cu", "pbf_group.cu", "pbf_tile.cu", "pbf
 CPP_SOURCES = ["pbf_params.cpp", "pbf_scenario.cpp", "pbf_sim.cpp", "pbf_batch.cpp", "pbf_server.cpp",
                "Simulation.cpp"]
 RUNNER_SOURCES = ["pbf_run.cpp"]
-HEADERS = ["pbf_internal.cuh", "pbf_device.cuh", "pbf_lists.cuh", "pbf_paper.cuh", "pbf_host.hpp", "Simulation.hpp"]
+HEADERS = ["pbf_internal.cuh", "pbf_device.cuh", "pbf_lists.cuh", "pbf_group.cuh", "pbf_paper.cuh", "pbf_host.hpp", "Simulation.hpp"]
 
 
 def _run(cmd: list[str]) -> str:

@@ -524,6 +524,11 @@ cudaError_t rc_gather(const DeviceState &d, uint32_t n, const StepClear *clear, 
 // The passes read neighbours by sorted slot (PS, the planes, SS, VS) and write
 // their own slot's values there; lambda leaves the lists that delta-p walks,
 // and the last delta-p pass also writes P and V by input index for the commit.
+// Scenes of up to this many particles take eight threads per particle.  Per
+// step, one thread against eight: 1,000 particles 219 and 116 us alone (61 and
+// 27 with three scenes at once), 8,000 251 / 157 (68 / 41), 17,576 253 / 201
+// (75 / 74), 32,768 279 / 267 (89 / 125).
+constexpr uint32_t kRefGroupParticles = 16384;
 cudaError_t rc_lambda(float4 *PS, const float4 *planes, float *SS, const uint32_t *offsets,
                       uint32_t n, const RefConsts &k, uint32_t maxn, uint4 *nbr,
                       uint32_t *nbr_cnt, cudaStream_t st);

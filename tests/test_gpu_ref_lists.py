@@ -65,3 +65,25 @@ def test_both_sorts(pbf, oracle_mod, cells):
     p = pbf.scenes.base_params(tuple(0.1 * c for c in cells), cells, mode=pbf.MODE_REF_COMPAT)
     ps = pbf.generate_block((0.12, 0.14, 0.13), 11, 9, 10, 0.05, 0.002, 0.125, 9)
     check(pbf, oracle_mod, p, ps, 2)
+
+
+# eight threads per particle up to 16,384 particles, one beyond: both with lists
+# that hold every set, some, and almost none
+@pytest.mark.parametrize("nz,max_neighbours", [(16, 128), (16, 32), (17, 128), (17, 32), (17, 8)])
+def test_threads_per_particle(pbf, oracle_mod, nz, max_neighbours):
+    p = pbf.scenes.base_params((1.9, 1.9, 1.2), (19, 19, 12), mode=pbf.MODE_REF_COMPAT)
+    p.max_neighbours = max_neighbours
+    ps = pbf.generate_block((0.15, 0.15, 0.15), 32, 32, nz, 0.048, 0.008, 0.125, 31)
+    check(pbf, oracle_mod, p, ps, 2, wave=0.004)
+
+
+# rows of hundreds of candidates and sets of hundreds of members, in either form
+@pytest.mark.parametrize("count", [700, 17000])
+def test_crushed(pbf, oracle_mod, count):
+    p = pbf.scenes.base_params((1.0, 1.0, 1.0), (10, 10, 10), mode=pbf.MODE_REF_COMPAT)
+    rng = np.random.default_rng(count)
+    ps = np.zeros(count, pbf.PARTICLE_DTYPE)
+    side = 0.05 * (count / 6.0) ** (1 / 3)
+    ps["x"] = (0.15 + rng.uniform(0, side, (count, 3))).astype(np.float32)
+    ps["m"] = 0.125
+    check(pbf, oracle_mod, p, ps, 1)
