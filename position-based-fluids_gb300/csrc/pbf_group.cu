@@ -350,6 +350,7 @@ __global__ void __launch_bounds__(kGroupThreads)
                  const float4 *__restrict__ SS, NbrCtx nc, PaperConsts c,
                  const uint32_t *__restrict__ ID2, float4 *__restrict__ X,
                  float4 *__restrict__ V, uint32_t *__restrict__ ID) {
+  report_count(nc);
   __shared__ __align__(16) float s_terms[Terms<4>::kStride * kCtaParticles];
   group_xsph_of<EarlierKernel>(cta_particle(), PW, U, Wv, XS, SS, nc, c, ID2, X, V, ID,
                                s_terms + threadIdx.x / kGroup * Terms<4>::kStride);
@@ -399,7 +400,6 @@ struct TinyStep {
   float4 *X, *V, *X2, *V2;
   float *R;
   uint32_t *ID, *skeys, *off, *nbr_cnt, *cnt_max;
-  uint32_t *host_max;  // page-locked: the step's largest count for the host
   uint32_t ncells, iterations;
 };
 
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
       m = __reduce_max_sync(kAll, m);
       if (threadIdx.x == 0) {
         *t.cnt_max = m;
-        *t.host_max = m;
+        *t.nc.host_max = m;
       }
     }
     const float4 qk = make_float4(pk.x, pk.y, pk.z, lambda);
@@ -761,7 +761,7 @@ uint32_t tiny_cluster() {
 }
 
 cudaError_t tiny_step(const DeviceState &d, const PaperConsts &c, uint32_t ncells,
-                      uint32_t iterations, uint32_t *host_max, cudaStream_t st) {
+                      uint32_t iterations, cudaStream_t st) {
   TinyStep t;
   t.nc = make_ctx(d, c, nullptr);
   t.c = c;
@@ -775,7 +775,6 @@ cudaError_t tiny_step(const DeviceState &d, const PaperConsts &c, uint32_t ncell
   t.off = d.offsets;
   t.nbr_cnt = d.nbr_cnt;
   t.cnt_max = d.nbr_max;
-  t.host_max = host_max;
   t.ncells = ncells;
   t.iterations = iterations;
   // as many CTAs as the particles need, a power of two of them

@@ -354,6 +354,7 @@ struct DeviceState {
   uint4 *nbr = nullptr;                // neighbour lists, 4 slots or 8 staged indices per word
   uint32_t *nbr_cnt = nullptr;         // neighbour counts
   uint32_t *nbr_max = nullptr;         // largest neighbour count of the step (paper)
+  uint32_t *nbr_max_host = nullptr;    // the same in page-locked memory (single scenes)
   uint32_t *sort_scratch = nullptr;
   uint32_t *cell_scratch = nullptr;    // counting sort by cell
   uint32_t *err = nullptr;             // device error flag word
@@ -474,7 +475,7 @@ constexpr uint32_t kTinyParticles = 1024;
 constexpr uint32_t kTinyCells = 6144;
 uint32_t tiny_cluster();
 cudaError_t tiny_step(const DeviceState &d, const PaperConsts &c, uint32_t ncells,
-                      uint32_t iterations, uint32_t *host_max, cudaStream_t st);
+                      uint32_t iterations, cudaStream_t st);
 cudaError_t group_nbr_lambda(const DeviceState &d, const PaperConsts &c, const uint16_t *sid,
                              cudaStream_t st);
 cudaError_t group_lambda(const DeviceState &d, const PaperConsts &c, const uint16_t *sid,

@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(kBlock)
                   const float4 *__restrict__ SS, NbrCtx nc, PaperConsts c,
                   const uint32_t *__restrict__ ID2, float4 *__restrict__ X,
                   float4 *__restrict__ V, uint32_t *__restrict__ ID) {
+  report_count(nc);
   const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
   if (k >= c.n) return;
   const float4 pk = PW[k];

@@ -24,7 +24,8 @@ struct NbrCtx {
   const SceneDesc *__restrict__ scenes;
   const uint16_t *__restrict__ sid;
   uint32_t *err;
-  uint32_t *cnt_max;  // largest neighbour count of the step (may be null)
+  uint32_t *cnt_max;   // largest neighbour count of the step (may be null)
+  uint32_t *host_max;  // where the host reads it (may be null)
   uint32_t n, maxn;
   float dt, h2;
 };
@@ -35,6 +36,11 @@ __device__ __forceinline__ void record_count(uint32_t *cnt_max, uint32_t cnt) {
   const unsigned m = __activemask();
   const uint32_t mx = __reduce_max_sync(m, cnt);
   if (cnt_max && (threadIdx.x & 31u) == (unsigned)(__ffs(m) - 1)) atomicMax(cnt_max, mx);
+}
+
+// The step's last kernel: its largest count to the host.
+__device__ __forceinline__ void report_count(const NbrCtx &c) {
+  if (c.host_max && blockIdx.x == 0 && threadIdx.x == 0) *c.host_max = *c.cnt_max;
 }
 
 __device__ __forceinline__ const SceneDesc &scene_of(const SceneDesc *scenes,
@@ -514,6 +520,7 @@ inline NbrCtx make_ctx(const DeviceState &d, const PaperConsts &c, const uint16_
   nc.sid = sid;
   nc.err = d.err;
   nc.cnt_max = d.nbr_max;
+  nc.host_max = d.nbr_max_host;
   nc.n = c.n;
   nc.maxn = c.maxn;
   nc.dt = c.dt;

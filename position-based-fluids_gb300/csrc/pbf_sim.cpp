@@ -79,17 +79,13 @@ struct pbf_sim {
   bool have_times = false;
   bool stepped = false;
   bool scene_dirty = false;
-  // adaptive neighbour-list capacity (paper): the largest count of each
-  // step lands in page-locked memory; before launching a step the host
-  // looks at the count of the step kCountLag back, or of a later one that has
-  // run (the first step's right after it), and grows the lists when it came
-  // within 1/8 of the capacity
+  // adaptive neighbour-list capacity (paper): each step's last kernel writes
+  // the step's largest count to page-locked memory (a copy of the one word,
+  // even on a side branch, was a graph node more per step); before launching a
+  // step the host looks at the count of the step kCountLag back, or of a later
+  // one that has run (the first step's right after it), and grows the lists
+  // when it came within 1/8 of the capacity
   uint32_t *nbr_max_host = nullptr;
-  // the copy of that count runs on a side branch of the step (forked after
-  // the list build, joined at the step's end) so the solver passes do not
-  // wait for it
-  cudaStream_t count_stream = nullptr;
-  cudaEvent_t count_fork = nullptr, count_join = nullptr;
   cudaEvent_t step_done[kCountLag] = {};
   uint64_t launched = 0;  // steps launched since init or the last growth
   uint32_t list_grows = 0;
@@ -122,11 +118,6 @@ void free_all(pbf_sim *s) {
   }
   if (s->nbr_max_host) cudaFreeHost(s->nbr_max_host);
   s->nbr_max_host = nullptr;
-  if (s->count_fork) cudaEventDestroy(s->count_fork);
-  if (s->count_join) cudaEventDestroy(s->count_join);
-  if (s->count_stream) cudaStreamDestroy(s->count_stream);
-  s->count_fork = s->count_join = nullptr;
-  s->count_stream = nullptr;
   for (cudaEvent_t e : s->events) cudaEventDestroy(e);
   s->events.clear();
   s->render.release();
@@ -180,23 +171,6 @@ cudaError_t step_offsets(pbf_sim *s) {
   return cell_offsets(d.skeys, s->n, s->ncells, d.offsets, s->stream);
 }
 
-// Copies the step's largest neighbour count (complete once the list build
-// has run) to page-locked host memory on the side stream; join_count_copy
-// at the end of the step makes the step wait for it.
-cudaError_t fork_count_copy(pbf_sim *s) {
-  cudaError_t e = cudaEventRecord(s->count_fork, s->stream);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(s->count_stream, s->count_fork, 0);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(s->nbr_max_host, s->d.nbr_max, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                        s->count_stream);
-  if (e == cudaSuccess) e = cudaEventRecord(s->count_join, s->count_stream);
-  return e;
-}
-
-cudaError_t join_count_copy(pbf_sim *s) {
-  return cudaStreamWaitEvent(s->stream, s->count_join, 0);
-}
-
 // Whether the step runs as one launch (pbf_group.cu).  Timed steps report the
 // time of each pass and run them one by one; the bits are the same.
 bool use_tiny(const pbf_sim *s) {
@@ -208,8 +182,7 @@ bool use_tiny(const pbf_sim *s) {
 int launch_step(pbf_sim *s) {
   DeviceState &d = s->d;
   if (use_tiny(s)) {
-    PBF_TRY(tiny_step(d, s->pc, s->ncells, s->prm.solver_iterations, s->nbr_max_host,
-                      s->stream));
+    PBF_TRY(tiny_step(d, s->pc, s->ncells, s->prm.solver_iterations, s->stream));
     s->events_used = 0;
     return PBF_OK;
   }
@@ -251,7 +224,6 @@ int launch_step(pbf_sim *s) {
       for (uint32_t it = 0; it < iters; ++it) {
         if (it == 0) {
           PBF_TRY(tile_nbr_build(d, s->pc, nullptr, 1, st));
-          PBF_TRY(fork_count_copy(s));
           PBF_TRY_STATUS(mark(s, 1, "nbr_build", 1, &ev));
         }
         PBF_TRY(tile_lambda(d, s->pc, nullptr, 1, st));
@@ -263,17 +235,14 @@ int launch_step(pbf_sim *s) {
       PBF_TRY_STATUS(mark(s, 3, "vorticity", 1, &ev));
       PBF_TRY(tile_xsph_commit(d, s->pc, nullptr, 1, st));
       PBF_TRY_STATUS(mark(s, 3, "xsph_commit", 1, &ev));
-      PBF_TRY(join_count_copy(s));
     } else {
       for (uint32_t it = 0; it < iters; ++it) {
         if (it == 0 && d.tune.fuse_first) {
           PBF_TRY(paper_nbr_lambda(d, s->pc, nullptr, st));
-          PBF_TRY(fork_count_copy(s));
           PBF_TRY_STATUS(mark(s, 1, "nbr_lambda", 1, &ev));
         } else {
           if (it == 0) {
             PBF_TRY(paper_nbr_build(d, s->pc, nullptr, st));
-            PBF_TRY(fork_count_copy(s));
             PBF_TRY_STATUS(mark(s, 1, "nbr_build", 1, &ev));
           }
           PBF_TRY(paper_lambda(d, s->pc, nullptr, st));
@@ -286,7 +255,6 @@ int launch_step(pbf_sim *s) {
       PBF_TRY_STATUS(mark(s, 3, "vorticity", 1, &ev));
       PBF_TRY(paper_xsph_commit(d, s->pc, nullptr, st));
       PBF_TRY_STATUS(mark(s, 3, "xsph_commit", 1, &ev));
-      PBF_TRY(join_count_copy(s));
     }
   } else {
     if (s->rc_count_sort) {
@@ -613,11 +581,8 @@ int pbf_init(pbf_sim *s) {
     if (te == cudaSuccess) te = cudaMallocHost(&s->nbr_max_host, sizeof(uint32_t));
     for (cudaEvent_t &e : s->step_done)
       if (te == cudaSuccess) te = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-    if (te == cudaSuccess) te = cudaStreamCreateWithFlags(&s->count_stream, cudaStreamNonBlocking);
-    if (te == cudaSuccess) te = cudaEventCreateWithFlags(&s->count_fork, cudaEventDisableTiming);
-    if (te == cudaSuccess) te = cudaEventCreateWithFlags(&s->count_join, cudaEventDisableTiming);
     if (te != cudaSuccess) rc = cuda_status(te, "pbf_init");
-    else *s->nbr_max_host = 0;
+    else *(d.nbr_max_host = s->nbr_max_host) = 0;
   }
   if (rc != PBF_OK) {
     free_all(s);

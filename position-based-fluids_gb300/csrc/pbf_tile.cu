@@ -549,6 +549,7 @@ __global__ void __launch_bounds__(kThreads, kCtasOne)
                        const float4 *__restrict__ SS, NbrCtx nc, BlockCtx bc, PaperConsts c,
                        const uint32_t *__restrict__ ID2, float4 *__restrict__ X,
                        float4 *__restrict__ V, uint32_t *__restrict__ ID) {
+  report_count(nc);
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const BlockSmem sm{smem_raw};
   const float4 *const src[1] = {PW};
