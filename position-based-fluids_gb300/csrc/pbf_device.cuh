@@ -84,14 +84,15 @@ __device__ __forceinline__ void count_cell_keys(const uint32_t (&key)[kKeys],
 constexpr int kCountKeys = 4;
 
 // Slot of the particle in unordered slot q once its cell is back in index
-// order: cells of up to kRankCell particles are left as the scatter placed
+// order: cells of up to rank_cell particles are left as the scatter placed
 // them, and each particle finds its place by counting the smaller indices
 // (larger cells are already in order: k_cell_fix_big).
 __device__ __forceinline__ uint32_t ordered_slot(const uint32_t *__restrict__ perm,
                                                  const uint32_t *__restrict__ off, uint32_t key,
-                                                 uint32_t q, uint32_t index, uint32_t n) {
+                                                 uint32_t q, uint32_t index, uint32_t n,
+                                                 uint32_t rank_cell) {
   const uint32_t a = __ldg(&off[key]), b = min(__ldg(&off[key + 1]), n);
-  if (b - a > kRankCell || a > q) return q;  // (a <= q < b unless the sort reported an error)
+  if (b - a > rank_cell || a > q) return q;  // (a <= q < b unless the sort reported an error)
   uint32_t rank = 0;
   for (uint32_t t = a; t < b; ++t) rank += perm[t] < index ? 1u : 0u;
   return min(a + rank, n - 1u);

@@ -184,11 +184,20 @@ uint32_t sort_pass_launches(const SortPlan &plan);
 // puts each cell back in index order, so skeys / perm are the stable sort's.
 // Layout of its scratch (32-bit words):
 // The step's own order of the particles in a cell is left to the kernel that
-// gathers the state (ordered_slot) for cells of up to this many.
+// gathers the state (ordered_slot) for cells of up to kRankCell particles, and
+// for any cell of a scene (a batch: of a capacity) of up to kRankAllParticles,
+// where the launch for the larger cells takes longer than what it does (steps
+// of 32,768 particles 93.5 -> 92.0 us).  The neighbour passes over a crowded
+// cell each test the pairs that ranking it reads, with more work per pair, so
+// the ranks never bound a step.
 constexpr uint32_t kRankCell = 64;
+constexpr uint32_t kRankAllParticles = 65536;
 struct CellSortPlan {
   uint32_t n = 0, ncells = 0, tiles = 0;
   uint32_t scan_chunks = 0;  // chunks of 2048 counts per scan tile (1 or 4)
+  // cells of any size are ordered by the gather (by the capacity, so that a
+  // batch's launches do not change with its scenes)
+  bool rank_all = false;
   uint32_t small_cap = 0, med_cap = 0, big_cap = 0, huge_cap = 0;
   uint32_t bm_words = 0;   // words of a bitmap over the n particle indices
   uint32_t bm_stride = 0;  // words from one CTA's bitmap to the next
@@ -218,22 +227,26 @@ cudaError_t cell_sort_finish(const CellSortPlan &plan, const uint32_t *keys, uin
                              uint32_t *offsets, uint32_t *skeys, uint32_t *perm, uint32_t *err,
                              cudaStream_t stream);
 // The same for a step, whose gather of the state orders the cells of up to
-// kRankCell particles (ordered_slot): perm holds those in the order their
-// counts were taken.  The control words must be zero (cell_sort_clear once;
-// the gather leaves them so).
+// kRankCell particles, or all (ordered_slot): perm holds those in the order
+// their counts were taken.  The control words must be zero (cell_sort_clear
+// once; the gather leaves them so).
 cudaError_t cell_sort_place(const CellSortPlan &plan, const uint32_t *keys, uint32_t *scratch,
                             uint32_t *offsets, uint32_t *skeys, uint32_t *perm, uint32_t *err,
                             cudaStream_t stream);
-constexpr uint32_t kCellPlaceLaunches = 3;
+inline uint32_t cell_place_launches(const CellSortPlan &plan) {
+  return plan.rank_all ? 2u : 3u;
+}
 // The words a step's gather zeroes for the next step (ctl, words) and for the
 // rest of this one (one word, may be null).
 struct StepClear {
   uint32_t *ctl;
   uint32_t words;
   uint32_t *also;
+  uint32_t rank_cell;
 };
 inline StepClear step_clear(const CellSortPlan &plan, uint32_t *scratch, uint32_t *also) {
-  return StepClear{scratch + plan.off_ctl, (uint32_t)plan.ctl_words, also};
+  return StepClear{scratch + plan.off_ctl, (uint32_t)plan.ctl_words, also,
+                   plan.rank_all ? UINT32_MAX : kRankCell};
 }
 // The predict kernel's counting from a key array; a key outside
 // [0, plan.ncells) is left out and sets kDevErrKey in *err.

@@ -131,10 +131,10 @@ __global__ void __launch_bounds__(256)
     if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
-// The state in slot order: slot k of `perm` (kRanked: cells of up to kRankCell
-// particles still unordered, each particle finding its slot in its cell --
-// about eight indices its cell-mates read as well, where a pass over the
-// cells that put them in order took 5 us at 1M particles and a launch).
+// The state in slot order: slot k of `perm` (kRanked: cells of up to
+// clear.rank_cell particles still unordered, each particle finding its slot in
+// its cell -- about eight indices its cell-mates read as well, where a pass
+// over the cells that put them in order took 5 us at 1M particles and a launch).
 // kRanked also leaves the sort's control words and the step's largest
 // neighbour count zero.
 template <bool kRanked>
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256)
   const float4 x = X[src];
   const float4 v1 = gravity_velocity(V[src], c.dt, c.gy);
   const uint32_t id = ID[src];
-  const uint32_t k = kRanked ? ordered_slot(perm, off, skeys[q], q, src, n) : q;
+  const uint32_t k = kRanked ? ordered_slot(perm, off, skeys[q], q, src, n, clear.rank_cell) : q;
   const float3 d = displacement(v1, c.dt);
   const float3 p = add3(x, d);
   X2[k] = x;

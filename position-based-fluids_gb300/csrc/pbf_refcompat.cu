@@ -188,8 +188,8 @@ __global__ void __launch_bounds__(256)
 }
 
 // Predicted positions by slot (PS, planes) and each slot's input index.
-// kRanked: as k_reorder (pbf_paper.cu), the cells of up to kRankCell particles
-// are put in order here, and the sort's control words left zero.
+// kRanked: as k_reorder (pbf_paper.cu), the cells of up to clear.rank_cell
+// particles are put in order here, and the sort's control words left zero.
 template <bool kRanked>
 __global__ void __launch_bounds__(256)
     k_rc_gather(const float4 *__restrict__ P, const uint32_t *__restrict__ perm,
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256)
   if (t >= n) return;
   // perm is a permutation of [0, n) unless the sort reported an error.
   const uint32_t element = min(perm[t], n - 1u);
-  const uint32_t q = kRanked ? ordered_slot(perm, off, skeys[t], t, element, n) : t;
+  const uint32_t q = kRanked ? ordered_slot(perm, off, skeys[t], t, element, n, clear.rank_cell) : t;
   const uint32_t i = n - 1u - element;
   const float4 p = P[i];
   PS[q] = p;

@@ -199,7 +199,7 @@ int launch_step(pbf_sim *s) {
                                 d.cell_scratch, st));
     PBF_TRY_STATUS(mark(s, 0, "predict_hash", 1, &ev));
     PBF_TRY(cell_sort_place(s->cplan, d.keys, d.cell_scratch, d.offsets, d.skeys, d.perm, d.err, st));
-    PBF_TRY_STATUS(mark(s, 0, "cell_sort", kCellPlaceLaunches, &ev));
+    PBF_TRY_STATUS(mark(s, 0, "cell_sort", cell_place_launches(s->cplan), &ev));
   } else if (s->paper) {
     PBF_TRY(sort_clear(s->plan, d.sort_scratch, st));
     PBF_TRY(cudaMemsetAsync(d.nbr_max, 0, sizeof(uint32_t), st));
@@ -262,7 +262,7 @@ int launch_step(pbf_sim *s) {
                                d.cell_scratch, st));
       PBF_TRY_STATUS(mark(s, 0, "rc_predict_hash", 1, &ev));
       PBF_TRY(cell_sort_place(s->cplan, d.keys, d.cell_scratch, d.offsets, d.skeys, d.perm, d.err, st));
-      PBF_TRY_STATUS(mark(s, 0, "cell_sort", kCellPlaceLaunches, &ev));
+      PBF_TRY_STATUS(mark(s, 0, "cell_sort", cell_place_launches(s->cplan), &ev));
     } else {
       PBF_TRY(sort_clear(s->plan, d.sort_scratch, st));
       PBF_TRY(rc_predict_hash(d.X, d.V, d.P, n, s->rc, d.scenes, d.keys, s->plan,
@@ -786,7 +786,7 @@ int pbf_launches_per_step(const pbf_sim *s, uint32_t *launches) {
     return PBF_OK;
   }
   const uint32_t sort = (s->paper ? !s->d.tune.radix_sort : s->rc_count_sort)
-                            ? kCellPlaceLaunches
+                            ? cell_place_launches(s->cplan)
                             : 1u /*scan*/ + s->plan.passes + (s->offset_runs ? 2u : 1u) /*offsets*/;
   if (s->paper)
     *launches = 1u /*predict+hash*/ + sort + 1u /*reorder*/ + paper_first_launches(s->d) +

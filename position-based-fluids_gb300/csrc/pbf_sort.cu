@@ -977,6 +977,7 @@ CellSortPlan make_cell_sort_plan(uint32_t n, uint32_t ncells) {
   p.n = n;
   p.ncells = ncells;
   set_scan_tiles(p);
+  p.rank_all = n <= kRankAllParticles;
   p.small_cap = (uint32_t)std::min<uint64_t>(ncells, (uint64_t)n / 2 + 1);
   p.med_cap = (uint32_t)std::min<uint64_t>(ncells, (uint64_t)n / (kSmallCell + 1) + 1);
   p.big_cap = (uint32_t)std::min<uint64_t>(ncells, (uint64_t)n / (kWarpCell + 1) + 1);
@@ -1063,7 +1064,7 @@ cudaError_t cell_sort_place(const CellSortPlan &plan, const uint32_t *keys, uint
                             cudaStream_t stream) {
   const cudaError_t e = scan_and_scatter<true>(plan, keys, scratch, offsets, skeys, perm, err,
                                                stream);
-  if (e != cudaSuccess || plan.n == 0) return e;
+  if (e != cudaSuccess || plan.rank_all || plan.n == 0) return e;
   // at most n / (kRankCell + 1) cells are listed
   const uint32_t ctas = min(kStrideCtas / 4u, max(kHugeCtas, plan.n / (kRankCell + 1u) + 1u));
   return fix_big(plan, scratch, offsets, perm, ctas, stream);
