@@ -33,3 +33,35 @@ def test_sizes(pbf, n):
             img = sim.render(cam, width, height)
             want = oracle_render.render(pos, p, cam, width, height)
             assert np.array_equal(img, want), (width, height, near, cap)
+
+
+def picture(pbf, p, pos, width, height, near, cap):
+    ps = np.zeros(len(pos), pbf.PARTICLE_DTYPE)
+    ps["x"] = 0.5
+    ps["m"] = 0.125
+    with pbf.Simulation(p, ps) as sim:
+        sim.init()
+        sim.set_state(pos, np.zeros_like(pos))
+        cam = pbf.default_camera(p)
+        cam.distance *= near
+        cam.max_point_size = cap
+        return sim.render(cam, width, height)
+
+
+# 81,919 sprites are drawn in one part; with particles outside the view added,
+# which draw nothing, in two, the second taking the image in blocks of eight by
+# eight pixels, of which these images hold whole ones, cut ones and less than one
+@pytest.mark.parametrize("width, height, near, cap", [(133, 81, 1.0, 12.0), (640, 512, 0.35, 64.0),
+                                                      (96, 64, 40.0, 12.0), (5, 3, 1.0, 200.0)])
+def test_two_parts_draw_what_one_does(pbf, width, height, near, cap):
+    p = pbf.scenes.base_params((1.0, 1.0, 1.0), (10, 10, 10))
+    n = 81919
+    rng = np.random.default_rng(width)
+    pos = rng.uniform(0.0, 1.0, (n, 4)).astype(np.float32)
+    pos[1::2, 2] = 0.5  # depths that many share
+    want = picture(pbf, p, pos, width, height, near, cap)
+    assert len(np.unique(want)) > 2
+    for more in (1, 33, 5000):
+        outside = np.full((more, 4), 1e6, np.float32)
+        for both in (np.concatenate([pos, outside]), np.insert(pos, n // 3, outside, axis=0)):
+            assert np.array_equal(picture(pbf, p, both, width, height, near, cap), want)
