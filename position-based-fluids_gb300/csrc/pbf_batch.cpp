@@ -150,7 +150,6 @@ int launch_batch_step(pbf_batch *b) {
     PBF_TRY(sort_clear(b->plan, d.sort_scratch, st));
     PBF_TRY(paper_predict_hash(d.X, d.V, n, pc, d.scenes, d.sid, d.keys, b->plan,
                                d.sort_scratch, st));
-    PBF_TRY(sort_scan(b->plan, d.sort_scratch, st));
     PBF_TRY(sort_passes(b->plan, d.keys, nullptr, d.skeys, d.perm, d.sort_scratch, d.err, st));
     PBF_TRY(cell_offsets_runs(d.skeys, n, b->cells_total, d.offsets, d.runs, d.runs_count, st));
   }
@@ -481,9 +480,9 @@ int pbf_batch_launches_per_step(const pbf_batch *b, uint32_t *launches) {
   if (!b || !launches) return PBF_ERR_INVALID;
   const SortPlan plan = make_sort_plan(std::max<uint32_t>(b->n_total, 1),
                                        bits_for(std::max<uint32_t>(b->cells_total, 1)));
-  // predict + hash, the sort (counting: 2 or 3 launches; radix: scan, digit
+  // predict + hash, the sort (counting: 2 or 3 launches; radix: digit
   // passes, two for the offsets), reorder, the solver, the velocity passes
-  const uint32_t sort = b->d.tune.radix_sort ? 1u + plan.passes + 2u : cell_place_launches(b->cplan);
+  const uint32_t sort = b->d.tune.radix_sort ? plan.passes + 2u : cell_place_launches(b->cplan);
   *launches = 1u + sort + 1u + paper_first_launches(b->d) +
               2u * b->solver.solver_iterations - 1u + 2u;
   return PBF_OK;

@@ -91,7 +91,7 @@ constexpr uint32_t sort_passes_for(uint32_t key_bits) {
 struct SortPlan {
   uint32_t n = 0, key_bits = 0, passes = 0, tiles = 0;
   uint32_t digit_bits = 0, radix = 0;
-  size_t off_hist = 0;      // passes * radix: digit histograms, then prefixes
+  size_t off_hist = 0;      // passes * radix: digit histograms
   size_t off_counter = 0;   // 32 words: per-pass tile counters
   size_t off_lookback = 0;  // passes * tiles * radix
   size_t clear_words = 0;   // words from off_hist that must start at zero
@@ -142,10 +142,7 @@ cudaError_t sort_clear(const SortPlan &plan, uint32_t *scratch,
 // Digit histograms of keys (all passes); expects sort_clear first.
 cudaError_t sort_histogram(const SortPlan &plan, const uint32_t *keys,
                            uint32_t *scratch, cudaStream_t stream);
-// Exclusive prefix of each pass histogram, in place.
-cudaError_t sort_scan(const SortPlan &plan, uint32_t *scratch,
-                      cudaStream_t stream);
-// The digit passes (histograms must be scanned).  vals_in may be null
+// The digit passes.  vals_in may be null
 // (values = index).  Results land in keys_out / vals_out; inputs are left
 // untouched.
 cudaError_t sort_passes(const SortPlan &plan, const uint32_t *keys_in,

@@ -120,7 +120,6 @@ extern "C" int pbf_op_sort_pairs_noalloc(const uint32_t *d_keys_in,
   const cudaStream_t st = (cudaStream_t)stream;
   cudaError_t e = sort_clear(plan, scratch, st);
   if (e == cudaSuccess) e = sort_histogram(plan, d_keys_in, scratch, st);
-  if (e == cudaSuccess) e = sort_scan(plan, scratch, st);
   if (e == cudaSuccess)
     e = sort_passes(plan, d_keys_in, d_vals_in, d_keys_out, d_vals_out, scratch,
                     err, st);

@@ -206,10 +206,9 @@ int launch_step(pbf_sim *s) {
     PBF_TRY(paper_predict_hash(d.X, d.V, n, s->pc, d.scenes, nullptr, d.keys,
                                s->plan, d.sort_scratch, st));
     PBF_TRY_STATUS(mark(s, 0, "predict_hash", 1, &ev));
-    PBF_TRY(sort_scan(s->plan, d.sort_scratch, st));
     PBF_TRY(sort_passes(s->plan, d.keys, nullptr, d.skeys, d.perm,
                         d.sort_scratch, d.err, st));
-    PBF_TRY_STATUS(mark(s, 0, "sort_onesweep", 1 + passes, &ev));
+    PBF_TRY_STATUS(mark(s, 0, "sort_onesweep", passes, &ev));
     PBF_TRY(step_offsets(s));
     PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
   }
@@ -268,9 +267,8 @@ int launch_step(pbf_sim *s) {
       PBF_TRY(rc_predict_hash(d.X, d.V, d.P, n, s->rc, d.scenes, d.keys, s->plan,
                               d.sort_scratch, st));
       PBF_TRY_STATUS(mark(s, 0, "rc_predict_hash", 1, &ev));
-      PBF_TRY(sort_scan(s->plan, d.sort_scratch, st));
       PBF_TRY(sort_passes(s->plan, d.keys, nullptr, d.skeys, d.perm, d.sort_scratch, d.err, st));
-      PBF_TRY_STATUS(mark(s, 0, "sort_onesweep", 1 + passes, &ev));
+      PBF_TRY_STATUS(mark(s, 0, "sort_onesweep", passes, &ev));
       PBF_TRY(step_offsets(s));
       PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
     }
@@ -787,7 +785,7 @@ int pbf_launches_per_step(const pbf_sim *s, uint32_t *launches) {
   }
   const uint32_t sort = (s->paper ? !s->d.tune.radix_sort : s->rc_count_sort)
                             ? cell_place_launches(s->cplan)
-                            : 1u /*scan*/ + s->plan.passes + (s->offset_runs ? 2u : 1u) /*offsets*/;
+                            : s->plan.passes + (s->offset_runs ? 2u : 1u) /*offsets*/;
   if (s->paper)
     *launches = 1u /*predict+hash*/ + sort + 1u /*reorder*/ + paper_first_launches(s->d) +
                 2u * it - 1u + 2u;
@@ -944,7 +942,6 @@ int pbf_op_sort_pairs(const uint32_t *d_keys_in, const uint32_t *d_vals_in,
   const cudaStream_t st = (cudaStream_t)stream;
   PBF_TRY(sort_clear(plan, scratch, st));
   PBF_TRY(sort_histogram(plan, d_keys_in, scratch, st));
-  PBF_TRY(sort_scan(plan, scratch, st));
   PBF_TRY(sort_passes(plan, d_keys_in, d_vals_in, d_keys_out, d_vals_out,
                       scratch, err, st));
   return PBF_OK;

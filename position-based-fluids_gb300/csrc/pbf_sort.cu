@@ -112,89 +112,77 @@ __global__ void __launch_bounds__(kHistThreads)
     if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
-// Exclusive prefix of each pass histogram, in place: each thread owns
-// radix / 256 consecutive digits.
-__global__ void __launch_bounds__(kSortThreads)
-    k_sort_scan(uint32_t passes, uint32_t digit_bits, uint32_t *__restrict__ hist) {
-  __shared__ uint32_t s_warp[kSortWarps];
-  constexpr uint32_t kMaxPer = 1u << (kMaxDigitBits - kMinDigitBits);
-  const uint32_t per = 1u << (digit_bits - kMinDigitBits);
-  for (uint32_t p = 0; p < passes; ++p) {
-    uint32_t *h = hist + (p << digit_bits) + threadIdx.x * per;
-    uint32_t v[kMaxPer], sum = 0;
-#pragma unroll
-    for (uint32_t j = 0; j < kMaxPer; ++j) {
-      v[j] = j < per ? h[j] : 0u;
-      sum += v[j];
-    }
-    uint32_t e = block_exclusive_scan(sum, s_warp);
-#pragma unroll
-    for (uint32_t j = 0; j < kMaxPer; ++j) {
-      if (j < per) h[j] = e;
-      e += v[j];
-    }
-    __syncthreads();
-  }
-}
+// Look-back over groups of kLookGroup tiles.  A tile's word is its count
+// (kLbAggregate), then the count of everything up to it (kLbInclusive); the last
+// tile of a group gives its whole group's count instead of its own, which no
+// other tile needs.  So a tile adds up to kLookGroup - 1 words of its own group,
+// all in flight together, then the groups' words, again as many in flight: two
+// or three L2 round trips after the last of them has its counts, where tiles
+// that all start at once -- a sort of one wave -- walked up to 244 words behind
+// each other, four at a time.  Sort of 1M keys of 18 bits 47.0 -> 43.2 us.
+constexpr uint32_t kLookGroup = 16;
 
-// Exclusive prefix of digit d over tiles [0, tile) from the look-back
-// words, waiting for predecessors that have not published yet.  A wait of
-// more than spin_limit polls sets kDevErrLookback in *err and gives up
-// (returning what it has), so a kernel never spins without bound.
-__device__ __forceinline__ uint32_t lookback_prefix(uint32_t *lookback, uint32_t radix,
-                                                    uint32_t tile, uint32_t d,
-                                                    uint32_t spin_limit, uint32_t *err) {
-  constexpr int kWindow = 4;  // words in flight together: the walk is a chain of L2 reads
-  uint32_t excl = 0;
-  int t = (int)tile - 1;
-  uint32_t spins = 0;
-  while (true) {
-    uint32_t v[kWindow];
+// Adds `count` words from `at` downwards, `step` words apart, as they are
+// published; true when one of them was inclusive, or the wait gave up.
+__device__ __forceinline__ bool look_back(const uint32_t *at, size_t step, uint32_t count,
+                                          uint32_t &excl, uint32_t &spins, uint32_t spin_limit,
+                                          uint32_t *err) {
+  while (count > 0u) {
+    uint32_t v[kLookGroup];
 #pragma unroll
-    for (int w = 0; w < kWindow; ++w)
-      v[w] = t >= w ? ld_volatile(&lookback[(size_t)(t - w) * radix + d]) : kLbInclusive;
+    for (uint32_t w = 0; w < kLookGroup; ++w) v[w] = w < count ? ld_volatile(at - w * step) : 0u;
+    uint32_t taken = 0;
 #pragma unroll
-    for (int w = 0; w < kWindow; ++w) {
-      const uint32_t flag = v[w] & ~kLbMask;
-      if (flag == 0u) break;
+    for (uint32_t w = 0; w < kLookGroup; ++w) {
+      if (taken != w || (v[w] & ~kLbMask) == 0u) continue;
       excl += v[w] & kLbMask;
-      if (flag == kLbInclusive) return excl;
-      --t;
+      if ((v[w] & ~kLbMask) == kLbInclusive) return true;
+      ++taken;
     }
-    if (++spins >= spin_limit) {
+    at -= taken * step;
+    count -= taken;
+    if (count == 0u) break;
+    if (taken == 0u && ++spins >= spin_limit) {
       atomicOr(err, kDevErrLookback);
-      return excl;
+      return true;
     }
     if (spins > 64) __nanosleep(32);
   }
+  return false;
+}
+
+// Publishes tile `tile`'s count of digit d and returns the count of all tiles
+// before it.  Gives up (and reports through *err) after spin_limit polls without
+// a new word, so a missing one cannot hang the GPU.
+__device__ __forceinline__ uint32_t lookback_prefix(uint32_t *lookback, uint32_t radix,
+                                                    uint32_t tile, uint32_t d, uint32_t count,
+                                                    uint32_t spin_limit, uint32_t *err) {
+  const uint32_t group = tile / kLookGroup, place = tile % kLookGroup;
+  const bool leads = place == kLookGroup - 1u;
+  uint32_t *mine = lookback + (size_t)tile * radix + d;
+  uint32_t excl = 0, spins = 0;
+  if (!leads) st_volatile(mine, (tile == 0 ? kLbInclusive : kLbAggregate) | count);
+  if (tile == 0) return 0u;
+  bool done = look_back(mine - radix, radix, place, excl, spins, spin_limit, err);
+  if (!done && group > 0u) {
+    if (leads) st_volatile(mine, kLbAggregate | (excl + count));
+    look_back(lookback + ((size_t)group * kLookGroup - 1u) * radix + d,
+              (size_t)kLookGroup * radix, group, excl, spins, spin_limit, err);
+  }
+  st_volatile(mine, kLbInclusive | ((excl + count) & kLbMask));
+  return excl;
 }
 
 // Runs the look-back wait of one digit against a predecessor tile that
 // never publishes (the words are zero): the wait must give up after
 // spin_limit polls and report through *err.
 __global__ void k_wait_selftest(uint32_t *lookback, uint32_t spin_limit, uint32_t *err) {
-  if (threadIdx.x == 0) lookback_prefix(lookback, 1u << kMinDigitBits, 1u, 0u, spin_limit, err);
-}
-
-// The lanes of `lanes` whose kBits-bit digit equals the caller's (whole warp),
-// from a ballot per bit: __match_any_sync takes a round per distinct value and
-// was most of a pass.  1M keys of 18 bits: 25.8 us per pass with it and 8 warps
-// per tile, 18.4 with 16 warps, 16.7 with the ballots; 8M keys 327 -> 190 us
-// for the whole sort.
-template <uint32_t kBits>
-__device__ __forceinline__ unsigned same_digit(uint32_t d, unsigned lanes) {
-#pragma unroll
-  for (uint32_t b = 0; b < kBits; ++b) {
-    const bool one = d >> b & 1u;
-    const unsigned ones = __ballot_sync(0xffffffffu, one);
-    lanes &= one ? ones : ~ones;
-  }
-  return lanes;
+  if (threadIdx.x == 0) lookback_prefix(lookback, 1u << kMinDigitBits, 1u, 0u, 0u, spin_limit, err);
 }
 
 // Dynamic shared memory of one digit pass with 2^kBits digits.
 constexpr size_t onesweep_smem_bytes(uint32_t bits) {
-  return ((size_t)kSweepWarps * (1u << bits) + 2u * (1u << bits) + 2u * kSortTile) *
+  return ((size_t)2u * kSweepWarps * (1u << bits) + 2u * (1u << bits) + 2u * kSortTile) *
          sizeof(uint32_t);
 }
 
@@ -204,12 +192,13 @@ __global__ void __launch_bounds__(kSweepThreads)
                const uint32_t *__restrict__ vals_in,
                uint32_t *__restrict__ keys_out, uint32_t *__restrict__ vals_out,
                uint32_t n, uint32_t shift,
-               const uint32_t *__restrict__ global_excl,
+               const uint32_t *__restrict__ hist,
                uint32_t *lookback, uint32_t *tile_counter, uint32_t *err) {
   constexpr uint32_t R = 1u << kBits;
   extern __shared__ __align__(16) uint32_t s_dyn[];
   uint32_t(*s_wcnt)[R] = reinterpret_cast<uint32_t(*)[R]>(s_dyn);  // [kSweepWarps][R]
-  uint32_t *s_dexcl = s_dyn + kSweepWarps * R;
+  uint32_t(*s_match)[R] = s_wcnt + kSweepWarps;
+  uint32_t *s_dexcl = s_dyn + 2u * kSweepWarps * R;
   uint32_t *s_gbase = s_dexcl + R;
   uint32_t *s_keys = s_gbase + R;
   uint32_t *s_vals = s_keys + kSortTile;
@@ -218,7 +207,10 @@ __global__ void __launch_bounds__(kSweepThreads)
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) s_tile = atomicAdd(tile_counter, 1u);
-  for (uint32_t i = tid; i < kSweepWarps * R; i += kSweepThreads) (&s_wcnt[0][0])[i] = 0u;
+  for (uint32_t i = tid; i < 2u * kSweepWarps * R / 4u; i += kSweepThreads)
+    reinterpret_cast<uint4 *>(s_dyn)[i] = make_uint4(0u, 0u, 0u, 0u);
+  const uint32_t d = (uint32_t)tid;  // the digit this thread sees to after the ranks
+  const uint32_t total = d < R ? __ldg(&hist[d]) : 0u;
   __syncthreads();
 
   const uint32_t tile = s_tile;
@@ -236,46 +228,64 @@ __global__ void __launch_bounds__(kSweepThreads)
     val[it] = ok ? (kIota ? idx : vals_in[idx]) : 0u;
   }
 
+  // Keys of lower digits in all tiles, while this tile's keys are on their way
+  // (a launch of its own for this scan took 3.4 us and its gap).
+  const uint32_t global_excl = block_exclusive_scan<kSweepWarps>(total, s_warp);
+
   // Warp-level multisplit: stable rank of each key among the warp's keys of
-  // the same digit, item by item.
+  // the same digit, item by item; the lanes of a digit find each other through
+  // a word of shared memory.  (With a ballot per digit bit the ranks took 3,640
+  // cycles of a tile, 6,500 with two tiles on the SM: 12 cycles a ballot.  1M
+  // keys of 18 bits 43.2 -> 39.0 us, 4M 111 -> 100; __match_any_sync, a round
+  // per distinct value, was slower still.)
   const unsigned lt_mask = (1u << lane) - 1u;
 #pragma unroll
   for (int it = 0; it < kSweepItems; ++it) {
     const uint32_t idx = seg + (uint32_t)it * 32u + lane;
     const bool ok = idx < n;
-    const uint32_t d = (key[it] >> shift) & (R - 1);
-    const unsigned peers = same_digit<kBits>(d, __ballot_sync(0xffffffffu, ok));
-    const uint32_t before = ok ? s_wcnt[warp][d] : 0u;
+    const uint32_t dg = (key[it] >> shift) & (R - 1);
+    // one digit throughout (keys in order): known without 32 turns at one word
+    // (4M equal keys 109 -> 85 us, random ones 100 -> 101)
+    const uint32_t dg0 = __shfl_sync(0xffffffffu, dg, 0);
+    if (__all_sync(0xffffffffu, ok && dg == dg0)) {
+      const uint32_t before = s_wcnt[warp][dg];
+      __syncwarp();
+      rank[it] = before + (uint32_t)lane;
+      if (lane == 31) s_wcnt[warp][dg] = before + 32u;
+      __syncwarp();
+      continue;
+    }
+    if (ok) atomicOr(&s_match[warp][dg], 1u << lane);
+    __syncwarp();
+    const unsigned peers = s_match[warp][dg];
+    const uint32_t before = s_wcnt[warp][dg];
     __syncwarp();
     rank[it] = before + (uint32_t)__popc(peers & lt_mask);
-    if (ok && lane == 31 - __clz(peers))
-      s_wcnt[warp][d] = before + (uint32_t)__popc(peers);
+    if (ok && lane == 31 - __clz(peers)) {
+      s_match[warp][dg] = 0u;
+      s_wcnt[warp][dg] = before + (uint32_t)__popc(peers);
+    }
     __syncwarp();
   }
   __syncthreads();
 
   // Per digit (one thread each): the tile's count, and each warp's exclusive
   // offset.
-  const uint32_t d = (uint32_t)tid;
   uint32_t tile_count = 0, excl = 0;
   if (d < R) {
+    uint32_t x[kSweepWarps];
+#pragma unroll
+    for (int w = 0; w < kSweepWarps; ++w) x[w] = s_wcnt[w][d];
 #pragma unroll
     for (int w = 0; w < kSweepWarps; ++w) {
-      const uint32_t x = s_wcnt[w][d];
       s_wcnt[w][d] = tile_count;
-      tile_count += x;
+      tile_count += x[w];
     }
-    // decoupled look-back
-    uint32_t *mine = lookback + (size_t)tile * R + d;
-    st_volatile(mine, (tile == 0 ? kLbInclusive : kLbAggregate) | tile_count);
-    if (tile != 0) {
-      excl = lookback_prefix(lookback, R, tile, d, kSpinLimit, err);
-      st_volatile(mine, kLbInclusive | ((excl + tile_count) & kLbMask));
-    }
+    excl = lookback_prefix(lookback, R, tile, d, tile_count, kSpinLimit, err);
   }
   const uint32_t e = block_exclusive_scan<kSweepWarps>(tile_count, s_warp);
   if (d < R) {
-    s_gbase[d] = global_excl[d] + excl;
+    s_gbase[d] = global_excl + excl;
     s_dexcl[d] = e;
   }
   __syncthreads();
@@ -294,15 +304,20 @@ __global__ void __launch_bounds__(kSweepThreads)
   }
   __syncthreads();
   const uint32_t tile_n = min((uint32_t)kSortTile, n - tile_base);
-  for (uint32_t i = tid; i < tile_n; i += kSweepThreads) {
-    const uint32_t k = s_keys[i];
-    const uint32_t dg = (k >> shift) & (R - 1);
-    const uint32_t dst = s_gbase[dg] + (i - s_dexcl[dg]);
-    // Always true unless a look-back wait gave up (error flag set).
-    if (dst < n) {
-      keys_out[dst] = k;
-      vals_out[dst] = s_vals[i];
-    }
+#pragma unroll
+  for (uint32_t it = 0; it < kSweepItems; ++it) {
+    const uint32_t i = it * kSweepThreads + tid;
+    key[it] = i < tile_n ? s_keys[i] : 0u;
+    val[it] = i < tile_n ? s_vals[i] : 0u;
+    const uint32_t dg = (key[it] >> shift) & (R - 1);
+    rank[it] = i < tile_n ? s_gbase[dg] + (i - s_dexcl[dg]) : n;
+  }
+#pragma unroll
+  for (uint32_t it = 0; it < kSweepItems; ++it) {
+    // (also when a look-back wait gave up: error flag set)
+    if (rank[it] >= n) continue;
+    keys_out[rank[it]] = key[it];
+    vals_out[rank[it]] = val[it];
   }
 }
 
@@ -850,7 +865,7 @@ uint32_t bits_for(uint32_t max_key_exclusive) {
   return b;
 }
 
-uint32_t sort_pass_launches(const SortPlan &plan) { return 2u + plan.passes; }
+uint32_t sort_pass_launches(const SortPlan &plan) { return 1u + plan.passes; }
 
 cudaError_t wait_selftest(uint32_t *scratch, uint32_t spin_limit, uint32_t *err,
                           cudaStream_t stream) {
@@ -870,13 +885,6 @@ cudaError_t sort_histogram(const SortPlan &plan, const uint32_t *keys,
   const uint32_t blocks = min(blocks_for(plan.n, kHistThreads), kHistCtas);
   k_sort_histogram<<<blocks, kHistThreads, 0, stream>>>(keys, plan.n, plan.passes, plan.digit_bits,
                                                scratch + plan.off_hist);
-  return cudaGetLastError();
-}
-
-cudaError_t sort_scan(const SortPlan &plan, uint32_t *scratch,
-                      cudaStream_t stream) {
-  k_sort_scan<<<1, kSortThreads, 0, stream>>>(plan.passes, plan.digit_bits,
-                                              scratch + plan.off_hist);
   return cudaGetLastError();
 }
 

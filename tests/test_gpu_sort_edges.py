@@ -54,6 +54,27 @@ def test_sort_pairs(pbf, n, bits, kind, shift):
         assert np.array_equal(ov.cpu().numpy().view(np.uint32), want)
 
 
+# tiles of 4,096 keys in groups of 16: the last, the first and the only tile of a
+# group, one group and several, a warp of one digit and a part of a warp at the end
+@pytest.mark.parametrize("tiles", [2, 15, 16, 17, 31, 32, 33, 256, 257, 513])
+@pytest.mark.parametrize("more", [-4095, -33, -1, 0])
+@pytest.mark.parametrize("bits,kind", [(8, "random"), (18, "equal"), (18, "runs"), (24, "nearly")])
+def test_tiles_and_groups(pbf, tiles, more, bits, kind):
+    n = 4096 * tiles + more
+    rng = np.random.default_rng(n + bits)
+    k = keys_of(kind, n, 1 << bits, rng)
+    keys = dev(k)
+    size = pbf.op_sort_scratch_bytes(n, bits)
+    scratch = torch.empty(size, dtype=torch.uint8, device="cuda")
+    ok, ov = torch.empty_like(keys), torch.empty_like(keys)
+    order = np.argsort(k, kind="stable")
+    st = torch.cuda.current_stream().cuda_stream
+    pbf.op_sort_pairs(keys.data_ptr(), None, n, bits, ok.data_ptr(), ov.data_ptr(), scratch.data_ptr(), size, st)
+    pbf.op_sort_status(scratch.data_ptr(), n, bits, st)
+    assert np.array_equal(ok.cpu().numpy().view(np.uint32), k[order])
+    assert np.array_equal(ov.cpu().numpy().view(np.uint32), order)
+
+
 @pytest.mark.parametrize("n", SIZES)
 @pytest.mark.parametrize("ncells,kind", [(1, "equal"), (2048, "runs"), (114688, "nearly"), (114689, "random"), (600000, "nearly")])
 def test_sort_cells(pbf, n, ncells, kind):
