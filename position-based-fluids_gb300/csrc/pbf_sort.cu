@@ -516,17 +516,18 @@ __global__ void __launch_bounds__(kSortThreads)
   constexpr uint32_t kScanTile = kScanChunk * kScanChunks;
   __shared__ uint32_t s_tile, s_excl;
   __shared__ uint32_t s_chunk[kScanChunks];
-  __shared__ uint32_t s_warp[kSortWarps];
+  __shared__ uint32_t s_warp[kScanChunks][kSortWarps];
   uint32_t *lookback = ctl + kCtlHeader;
-  const uint32_t tid = threadIdx.x;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   if (tid == 0) s_tile = atomicAdd(&ctl[0], 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
-  uint32_t v[kScanChunks][kScanItems], texcl[kScanChunks];
+  // every chunk's counts on their way together, then one scan of all chunks (a
+  // step's cell sort at 1M 22.4 -> 20.8 us, at 4M 30.2 -> 28.4)
+  uint32_t v[kScanChunks][kScanItems], sum[kScanChunks], texcl[kScanChunks];
 #pragma unroll
   for (uint32_t q = 0; q < kScanChunks; ++q) {
     const uint32_t base = tile * kScanTile + q * kScanChunk + tid * kScanItems;
-    uint32_t sum = 0;
     // two 16-byte loads where the counts are 16-byte aligned (base is a
     // multiple of 8)
     if (base + kScanItems <= ncells && (reinterpret_cast<uintptr_t>(counts + base) & 15u) == 0u) {
@@ -534,21 +535,36 @@ __global__ void __launch_bounds__(kSortThreads)
       const uint4 b = *reinterpret_cast<const uint4 *>(counts + base + 4);
       v[q][0] = a.x; v[q][1] = a.y; v[q][2] = a.z; v[q][3] = a.w;
       v[q][4] = b.x; v[q][5] = b.y; v[q][6] = b.z; v[q][7] = b.w;
-      if (a.x | a.y | a.z | a.w) *reinterpret_cast<uint4 *>(counts + base) = make_uint4(0, 0, 0, 0);
-      if (b.x | b.y | b.z | b.w)
-        *reinterpret_cast<uint4 *>(counts + base + 4) = make_uint4(0, 0, 0, 0);
     } else {
 #pragma unroll
-      for (uint32_t j = 0; j < kScanItems; ++j) {
-        const uint32_t idx = base + j;
-        v[q][j] = idx < ncells ? counts[idx] : 0u;
-        if (v[q][j]) counts[idx] = 0u;
-      }
+      for (uint32_t j = 0; j < kScanItems; ++j) v[q][j] = base + j < ncells ? counts[base + j] : 0u;
     }
+  }
+#pragma unroll
+  for (uint32_t q = 0; q < kScanChunks; ++q) {
+    const uint32_t base = tile * kScanTile + q * kScanChunk + tid * kScanItems;
+    uint32_t any = 0;
+    sum[q] = 0;
 #pragma unroll
     for (uint32_t j = 0; j < kScanItems; ++j) {
-      sum += v[q][j];
-      if (kList && v[q][j] > kRankCell) {
+      any |= v[q][j];
+      sum[q] += v[q][j];
+    }
+    if (any) {
+      if (base + kScanItems <= ncells &&
+          (reinterpret_cast<uintptr_t>(counts + base) & 15u) == 0u) {
+        *reinterpret_cast<uint4 *>(counts + base) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4 *>(counts + base + 4) = make_uint4(0, 0, 0, 0);
+      } else {
+#pragma unroll
+        for (uint32_t j = 0; j < kScanItems; ++j)
+          if (v[q][j]) counts[base + j] = 0u;
+      }
+    }
+    if (kList) {
+#pragma unroll
+      for (uint32_t j = 0; j < kScanItems; ++j) {
+        if (v[q][j] <= kRankCell) continue;
         if (v[q][j] <= kBigCell) {
           const uint32_t at = atomicAdd(&ctl[1], 1u);
           if (at < big_cap) big[at] = base + j;
@@ -558,10 +574,29 @@ __global__ void __launch_bounds__(kSortThreads)
         }
       }
     }
-    texcl[q] = block_exclusive_scan(sum, s_warp);
-    if (tid == kSortThreads - 1) s_chunk[q] = texcl[q] + sum;
-    __syncthreads();
+    texcl[q] = sum[q];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, texcl[q], o);
+      if (lane >= (uint32_t)o) texcl[q] += t;
+    }
+    if (lane == 31u) s_warp[q][warp] = texcl[q];
   }
+  __syncthreads();
+  if (warp < kScanChunks) {  // a chunk's warps by one warp
+    const uint32_t w = lane < (uint32_t)kSortWarps ? s_warp[warp][lane] : 0u;
+    uint32_t wi = w;
+#pragma unroll
+    for (int o = 1; o < kSortWarps; o <<= 1) {
+      const uint32_t t = __shfl_up_sync(0xffffffffu, wi, o);
+      if (lane >= (uint32_t)o) wi += t;
+    }
+    if (lane < (uint32_t)kSortWarps) s_warp[warp][lane] = wi - w;
+    if (lane == (uint32_t)kSortWarps - 1u) s_chunk[warp] = wi;
+  }
+  __syncthreads();
+#pragma unroll
+  for (uint32_t q = 0; q < kScanChunks; ++q) texcl[q] += s_warp[q][warp] - sum[q];
   if (tid < 32) {
     uint32_t tot = 0;
 #pragma unroll
