@@ -94,3 +94,25 @@ def test_sort_cells(pbf, n, ncells, kind):
     assert np.array_equal(ok.cpu().numpy().view(np.uint32), k[order])
     want = np.concatenate([[0], np.cumsum(np.bincount(k, minlength=ncells))])
     assert np.array_equal(off.cpu().numpy(), want)
+
+
+# cells of every size around the half and the whole of a small cell's network,
+# their particles in any order
+@pytest.mark.parametrize("largest", [2, 7, 8, 9, 15, 16, 17])
+def test_small_cells_of_every_size(pbf, largest):
+    rng = np.random.default_rng(largest)
+    sizes = np.concatenate([np.arange(largest + 1), rng.integers(largest // 2, largest + 1, 9000)])
+    k = rng.permutation(np.repeat(np.arange(len(sizes)), sizes)).astype(np.uint32)
+    n, ncells = len(k), len(sizes)
+    keys = dev(k)
+    size = pbf.op_sort_cells_scratch_bytes(n, ncells)
+    scratch = torch.empty(max(16, size), dtype=torch.uint8, device="cuda")
+    off = torch.empty(ncells + 1, dtype=torch.int32, device="cuda")
+    skeys, perm = torch.empty_like(keys), torch.empty_like(keys)
+    st = torch.cuda.current_stream().cuda_stream
+    pbf.op_sort_cells(keys.data_ptr(), n, ncells, off.data_ptr(), skeys.data_ptr(), perm.data_ptr(), scratch.data_ptr(),
+                      size, st)
+    order = np.argsort(k, kind="stable")
+    assert np.array_equal(perm.cpu().numpy().view(np.uint32), order)
+    assert np.array_equal(skeys.cpu().numpy().view(np.uint32), k[order])
+    assert np.array_equal(off.cpu().numpy(), np.concatenate([[0], np.cumsum(sizes)]))
