@@ -237,7 +237,8 @@ int pbf_launches_per_step(const pbf_sim *sim, uint32_t *launches);
  * membership mask and store the members from the mask afterwards; 0 stores
  * each member as it is found.  With every field at its default, scenes of up
  * to 16,384 particles run their gather passes with eight threads per
- * particle instead; any other setting is taken as given.  No choice changes
+ * particle instead, and those of up to 1,024 (in at most 6,144 cells) the
+ * whole step in one launch; any other setting is taken as given.  No choice changes
  * a result bit.  trial_ms is the tuner's best time per launch of each pass (0 when
  * untuned). */
 typedef struct pbf_tuning {
@@ -274,10 +275,10 @@ int pbf_neighbour_stats(pbf_sim *sim, uint32_t *max_count, uint32_t *overflow);
  * neighbour count, and when that comes within 1/8 of the capacity the lists
  * are reallocated to 1.5x the count (at most 1024) before the next step is
  * launched, unless pbf_params.grow_lists is 0.  (Batches and servers keep
- * the capacity they were created with.)  (pbf_step therefore keeps at most 16 steps queued: before
- * launching a step it waits for the step 16 back -- for the first step's
- * count right after that step -- and looks at the latest count there is.)  No
- * reference counterpart; grows may be NULL. */
+ * the capacity they were created with.)  (pbf_step therefore keeps at most 16
+ * steps queued: before launching a step it waits for the step 16 back -- for
+ * the first step's count right after that step -- and looks at the latest
+ * count there is.)  No reference counterpart; grows may be NULL. */
 int pbf_list_capacity(const pbf_sim *sim, uint32_t *capacity, uint32_t *grows);
 /* Staged cell blocks of the last step (PAPER mode with staged = 1 in the
  * tuning): how many occupied blocks of 4 x 4 x 4 cells staged their

@@ -179,7 +179,7 @@ uint32_t sort_pass_launches(const SortPlan &plan);
 // cell's in `pos`; cell_sort_finish turns the counts into the cell offsets
 // (leaving the counts zero for the next step), scatters the particles and
 // puts each cell back in index order, so skeys / perm are the stable sort's.
-// Layout of its scratch (32-bit words):
+//
 // The step's own order of the particles in a cell is left to the kernel that
 // gathers the state (ordered_slot) for cells of up to kRankCell particles, and
 // for any cell of a scene (a batch: of a capacity) of up to kRankAllParticles,
@@ -189,6 +189,7 @@ uint32_t sort_pass_launches(const SortPlan &plan);
 // the ranks never bound a step.
 constexpr uint32_t kRankCell = 64;
 constexpr uint32_t kRankAllParticles = 65536;
+// Layout of the sort's scratch (32-bit words).
 struct CellSortPlan {
   uint32_t n = 0, ncells = 0, tiles = 0;
   uint32_t scan_chunks = 0;  // chunks of 2048 counts per scan tile (1 or 4)
