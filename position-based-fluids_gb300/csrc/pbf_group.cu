@@ -367,11 +367,11 @@ __global__ void __launch_bounds__(kGroupThreads)
 // in its own shared memory; a particle's group keeps its own state in
 // registers and writes each pass's value into every CTA's copy (distributed
 // shared memory).  Every CTA sorts the scene for itself at the start, so the
-// sort ends in shared memory as well.  1,000 particles: 39.5 us a step alone, and
-// three such scenes at once 14 us a step where the launches allowed 20.  Of its
-// 75,000 clocks the sort takes 6,700, the scan for neighbours 7,300, each pass
+// sort ends in shared memory as well.  1,000 particles: 36.9 us a step alone, and
+// three such scenes at once 13.8 us a step where the launches allowed 20.  Of its
+// 71,000 clocks the sort takes 6,700, the scan for neighbours 7,300, each pass
 // about 3,400 (four warps per scheduler of some 450 instructions) and each
-// barrier with the stores it waits for about 2,700.
+// barrier with the stores it waits for about 2,300.
 constexpr int kTinyThreads = 512;
 constexpr int kTinyGroups = kTinyThreads / kGroup;  // 64 per CTA
 constexpr uint32_t kTinyMaxCtas = kTinyParticles / kTinyGroups;
@@ -437,15 +437,25 @@ __device__ __forceinline__ uint32_t peer_address(uint32_t address, uint32_t rank
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(address), "r"(rank));
   return r;
 }
-// One particle's value into every CTA's copy: the group's threads take the
-// CTAs in turn.
-__device__ __forceinline__ void store_copies(float4 *own, const float4 &v, bool live) {
-  if (!live) return;
-  const uint32_t at = shared_address(own), ctas = cluster_size();
-  for (uint32_t r = lane_of_group(); r < ctas; r += kGroup)
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(peer_address(at, r)),
-                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-                 : "memory");
+// The CTA's particles' values into every CTA's copy of `array`: gathered in
+// `stage`, then a warp for each CTA, its lanes' stores side by side.  (Each
+// group's threads storing its own value to the CTAs in turn, 64 bytes to eight
+// CTAs per instruction: 38.9 us a step instead of 36.9.)
+__device__ __forceinline__ void store_copies(float4 *array, uint32_t first, uint32_t n,
+                                             const float4 &v, float4 *stage) {
+  if (lane_of_group() == 0) stage[threadIdx.x / kGroup] = v;
+  __syncthreads();
+  const uint32_t ctas = cluster_size(), lane = threadIdx.x & 31u;
+  for (uint32_t r = threadIdx.x / 32u; r < ctas; r += kTinyWarps)
+#pragma unroll
+    for (uint32_t i = lane; i < (uint32_t)kTinyGroups; i += 32u) {
+      if (first + i >= n) continue;
+      const float4 w = stage[i];
+      asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(
+                       peer_address(shared_address(array + first + i), r)),
+                   "f"(w.x), "f"(w.y), "f"(w.z), "f"(w.w)
+                   : "memory");
+    }
 }
 
 // Prediction and cell sort of the whole scene into the CTA's shared memory:
@@ -543,6 +553,8 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
   cluster_arrive();  // waited for before the first store into another CTA
   const uint32_t rank = cluster_rank(), group = threadIdx.x / kGroup;
   const PaperConsts &c = t.c;
+  __shared__ float4 s_stage[2][kTinyGroups];
+  const uint32_t first = rank * (uint32_t)kTinyGroups;
   float *terms = reinterpret_cast<float *>(s_tiny) + group * Terms<10>::kStride;
   uint16_t *list = reinterpret_cast<uint16_t *>(s_tiny + kTinyList) + group * kBuildList;
   float4 *A = reinterpret_cast<float4 *>(s_tiny + kTinyA);
@@ -608,7 +620,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
       }
       lambda = acc.lambda(c);
       rho = acc.rho;
-      store_copies(&B[k], make_float4(pk.x, pk.y, pk.z, lambda), g.live);
+      store_copies(B, first, c.n, make_float4(pk.x, pk.y, pk.z, lambda), s_stage[0]);
     }
     cluster_arrive();
     cluster_wait();
@@ -637,8 +649,9 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
       const Moved m = delta_moved(acc, x, make_float4(d.x, d.y, d.z, 0.f), sc, c);
       d = m.d;
       pk = make_float4(m.p.x, m.p.y, m.p.z, 0.f);
-      store_copies(&A[k], pk, g.live);
-      if (it + 1u == t.iterations) store_copies(&U[k], delta_velocity(d, rho, c), g.live);
+      store_copies(A, first, c.n, pk, s_stage[1]);
+      if (it + 1u == t.iterations)
+        store_copies(U, first, c.n, delta_velocity(d, rho, c), s_stage[0]);
     }
     cluster_arrive();
     cluster_wait();
@@ -660,7 +673,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
   }
   const float wn = norm3(w.wx, w.wy, w.wz);
   const float4 pw = make_float4(pk.x, pk.y, pk.z, __fmul_rn(wn, own.u.w));
-  store_copies(&B[k], pw, g.live);
+  store_copies(B, first, c.n, pw, s_stage[1]);
   cluster_arrive();
   cluster_wait();  // the last stores into another CTA lie behind it
   XsphAcc e;
