@@ -171,8 +171,6 @@ cudaError_t cell_hash(const float4 *pred, uint32_t n, const SceneDesc &scene,
 // after spin_limit polls.
 cudaError_t wait_selftest(uint32_t *scratch, uint32_t spin_limit, uint32_t *err,
                           cudaStream_t stream);
-// Number of kernel launches of one sort (histogram not included).
-uint32_t sort_pass_launches(const SortPlan &plan);
 
 // Counting sort of cell keys (paper path): the predict kernel counts every
 // cell's particles into `counts` and keeps each particle's place among its

@@ -925,8 +925,6 @@ uint32_t bits_for(uint32_t max_key_exclusive) {
   return b;
 }
 
-uint32_t sort_pass_launches(const SortPlan &plan) { return 1u + plan.passes; }
-
 cudaError_t wait_selftest(uint32_t *scratch, uint32_t spin_limit, uint32_t *err,
                           cudaStream_t stream) {
   k_wait_selftest<<<1, 32, 0, stream>>>(scratch, spin_limit, err);
