@@ -299,7 +299,7 @@ int pbf_batch_create(const pbf_params *solver, uint32_t max_scenes, uint32_t max
     return rc;
   }
   e = cudaMemsetAsync(d.err, 0, sizeof(uint32_t), b->stream);
-  if (e == cudaSuccess) e = cell_sort_clear(b->cplan_cap, d.cell_scratch, true, b->stream);
+  if (e == cudaSuccess) e = cell_sort_clear(b->cplan_cap, d.cell_scratch, b->stream);
   if (e == cudaSuccess)
     e = cudaMemsetAsync(d.offsets, 0, ((size_t)max_cells + 1) * sizeof(uint32_t), b->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);

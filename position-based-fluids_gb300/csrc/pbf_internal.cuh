@@ -213,10 +213,8 @@ CellSortPlan make_cell_sort_plan(uint32_t n, uint32_t ncells);
 // n particles over ncells cells: a batch keeps one layout of its scratch
 // while its scenes change.
 CellSortPlan resize_cell_sort_plan(const CellSortPlan &cap, uint32_t n, uint32_t ncells);
-// Zeroes the control words (and, with counts = true, the counts: once after
-// allocation).
-cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, bool counts,
-                            cudaStream_t stream);
+// Zeroes the counts and the control words (one launch).
+cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, cudaStream_t stream);
 // Offsets, scatter and in-cell order after the predict kernel has counted
 // (4 launches).
 cudaError_t cell_sort_finish(const CellSortPlan &plan, const uint32_t *keys, uint32_t *scratch,

@@ -595,7 +595,7 @@ int pbf_init(pbf_sim *s) {
   }
   PBF_TRY(cudaMemsetAsync(d.err, 0, sizeof(uint32_t), s->stream));
   if (s->paper || s->rc_count_sort)
-    PBF_TRY(cell_sort_clear(s->cplan, d.cell_scratch, true, s->stream));
+    PBF_TRY(cell_sort_clear(s->cplan, d.cell_scratch, s->stream));
   PBF_TRY(cudaMemsetAsync(d.P, 0, n * sizeof(float4), s->stream));
   PBF_TRY(cudaMemsetAsync(d.offsets, 0, ((size_t)s->ncells + 1) * sizeof(uint32_t),
                           s->stream));
@@ -978,7 +978,7 @@ int pbf_op_sort_cells(const uint32_t *d_keys, uint32_t n, uint32_t ncells, uint3
   uint32_t *scratch = static_cast<uint32_t *>(d_scratch);
   const cudaStream_t st = (cudaStream_t)stream;
   // the control words hold the error word (ctl[3]); the counts start at zero
-  PBF_TRY(cell_sort_clear(plan, scratch, true, st));
+  PBF_TRY(cell_sort_clear(plan, scratch, st));
   PBF_TRY(cell_sort_count(plan, d_keys, scratch, scratch + plan.off_ctl + 3, st));
   PBF_TRY(cell_sort_finish(plan, d_keys, scratch, d_offsets, d_sorted_keys, d_perm,
                            scratch + plan.off_ctl + 3, st));

