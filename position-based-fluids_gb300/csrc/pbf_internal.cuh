@@ -200,7 +200,7 @@ struct CellSortPlan {
   size_t off_counts = 0;  // ncells: per-cell counts (zero between steps)
   size_t off_pos = 0;     // n: each particle's place among its cell's
   size_t off_ctl = 0;     // 8 control words (list counts, an error word), then the
-  size_t ctl_words = 0;   //     scan's look-back words (zeroed before every step)
+  size_t ctl_words = 0;   //     scan's look-back words (zero between steps)
   size_t off_small = 0;   // cells of 2..16 particles out of index order
   size_t off_med = 0;     // cells of 17..64 particles
   size_t off_big = 0;     // cells of 65..8192 particles
@@ -213,6 +213,12 @@ CellSortPlan make_cell_sort_plan(uint32_t n, uint32_t ncells);
 // n particles over ncells cells: a batch keeps one layout of its scratch
 // while its scenes change.
 CellSortPlan resize_cell_sort_plan(const CellSortPlan &cap, uint32_t n, uint32_t ncells);
+// The control words from off_ctl on that cell_sort_clear zeroes: those of every
+// layout within the plan's capacity.  (A step leaves the words of its own layout
+// zero; one of fewer cells can take smaller scan tiles, and more of them.)
+inline size_t cell_sort_clear_words(const CellSortPlan &plan) {
+  return plan.off_small - plan.off_ctl;
+}
 // Zeroes the counts and the control words (one launch).
 cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, cudaStream_t stream);
 // Offsets, scatter and in-cell order after the predict kernel has counted

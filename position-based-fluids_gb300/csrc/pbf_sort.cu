@@ -1100,7 +1100,7 @@ CellSortPlan resize_cell_sort_plan(const CellSortPlan &cap, uint32_t n, uint32_t
 }
 
 cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, cudaStream_t stream) {
-  const uint32_t ctl = (uint32_t)plan.ctl_words;
+  const uint32_t ctl = (uint32_t)cell_sort_clear_words(plan);
   k_cell_clear<<<min(blocks_for(max(plan.ncells, ctl), 1024), kStrideCtas), 256, 0, stream>>>(
       scratch + plan.off_counts, plan.ncells, scratch + plan.off_ctl, ctl);
   return cudaGetLastError();

@@ -1,0 +1,46 @@
+"""Sizes and rules the host decides for the kernels (csrc/pbf_internal.cuh),
+evaluated on the CPU: small C++ programs against the library, over the sizes
+where a rule can go wrong."""
+from __future__ import annotations
+
+import subprocess
+
+from conftest import ROOT
+
+
+def evaluate(pbf, tmp_path, code: str) -> list[str]:
+    """Lines printed by a program whose main() is `code`."""
+    import importlib
+
+    build = importlib.import_module(pbf.__name__ + ".build")
+    src, exe = tmp_path / "rule.cpp", tmp_path / "rule"
+    src.write_text('#include <algorithm>\n#include <cstdint>\n#include <cstdio>\n'
+                   '#include "pbf_internal.cuh"\nusing namespace pbf;\n'
+                   f'int main() {{\n{code}\n}}\n')
+    pkg = pbf.LIB_PATH.parent
+    subprocess.run([build.CXX, *build.CXX_FLAGS, "-I", str(pkg / "csrc"), str(src), "-o", str(exe),
+                    f"-L{pkg}", "-lpbf_gb300", f"-Wl,-rpath,{pkg}"], check=True, cwd=ROOT)
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True,
+                          timeout=60).stdout.split("\n")[:-1]
+
+
+def test_cleared_control_words_hold_every_layout(pbf, tmp_path):
+    """A batch's control words are zeroed once, for its capacity: that has to
+    cover those of every layout within it (fewer cells can mean smaller scan
+    tiles, and more of them)."""
+    lines = evaluate(pbf, tmp_path, r"""
+  const uint32_t chunk = 2048;
+  for (uint32_t c = 1; c < 1200; ++c)
+    for (uint32_t cells : {c * chunk - 1, c * chunk, c * chunk + 1}) {
+      const CellSortPlan cap = make_cell_sort_plan(100000, cells);
+      const size_t zeroed = cell_sort_clear_words(cap);
+      if (cap.off_ctl + zeroed > cap.off_small) std::printf("past the words: %u\n", cells);
+      for (uint32_t k = 0; k <= c; k = k < 60 ? k + 1 : k * 2) {
+        const CellSortPlan p = resize_cell_sort_plan(cap, 1000, std::min(cells, k * chunk));
+        if (p.ctl_words > zeroed)
+          std::printf("%u of %u cells: %zu words, %zu zeroed\n", p.ncells, cells, p.ctl_words,
+                      zeroed);
+      }
+    }
+""")
+    assert lines == []
