@@ -7,6 +7,12 @@
 
 #include <cstddef>
 
+#ifdef __CUDACC__
+#define PBF_HOST_DEVICE __host__ __device__
+#else
+#define PBF_HOST_DEVICE
+#endif
+
 namespace pbf {
 
 // ---------------------------------------------------------------- errors --
@@ -219,6 +225,11 @@ CellSortPlan resize_cell_sort_plan(const CellSortPlan &cap, uint32_t n, uint32_t
 inline size_t cell_sort_clear_words(const CellSortPlan &plan) {
   return plan.off_small - plan.off_ctl;
 }
+// The index `stride` after i in a loop up to `end`, or `end` (a count of cells can
+// be so near 2^32 that i + stride is past it).  i < end.
+PBF_HOST_DEVICE inline uint32_t stride_next(uint32_t i, uint32_t stride, uint32_t end) {
+  return end - i > stride ? i + stride : end;
+}
 // Zeroes the counts and the control words (one launch).
 cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, cudaStream_t stream);
 // Offsets, scatter and in-cell order after the predict kernel has counted
@@ -395,11 +406,6 @@ cudaError_t iota_range(uint32_t *dst, uint32_t n, cudaStream_t st);
 // The staged gather passes (pbf_tile.cu) work on blocks of kBlockCells^3
 // cells of each scene's grid.
 constexpr int kBlockCells = 4;
-#ifdef __CUDACC__
-#define PBF_HOST_DEVICE __host__ __device__
-#else
-#define PBF_HOST_DEVICE
-#endif
 PBF_HOST_DEVICE inline uint32_t blocks_along(int32_t cells) {
   return (uint32_t)((cells + kBlockCells - 1) / kBlockCells);
 }

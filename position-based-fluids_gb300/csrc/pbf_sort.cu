@@ -685,8 +685,8 @@ __global__ void __launch_bounds__(256)
     k_cell_clear(uint32_t *__restrict__ counts, uint32_t cells, uint32_t *__restrict__ ctl,
                  uint32_t words) {
   const uint32_t first = blockIdx.x * 256u + threadIdx.x, stride = gridDim.x * 256u;
-  for (uint32_t i = first; i < cells; i += stride) counts[i] = 0u;
-  for (uint32_t i = first; i < words; i += stride) ctl[i] = 0u;
+  for (uint32_t i = first; i < cells; i = stride_next(i, stride, cells)) counts[i] = 0u;
+  for (uint32_t i = first; i < words; i = stride_next(i, stride, words)) ctl[i] = 0u;
 }
 
 // The counting of the predict kernel, from a key array (the operator).

@@ -44,3 +44,26 @@ def test_cleared_control_words_hold_every_layout(pbf, tmp_path):
     }
 """)
     assert lines == []
+
+
+def test_grid_stride_ends_at_the_largest_counts(pbf, tmp_path):
+    """The strided loops over cells visit every index once and end, also where
+    the index after the last one is past 32 bits."""
+    lines = evaluate(pbf, tmp_path, r"""
+  const uint32_t stride = kStrideCtas * 256u;
+  for (uint32_t end : {0u, 1u, 255u, stride - 1, stride, stride + 1, 3 * stride + 7,
+                       0xffffffffu - stride, 0xffffffffu - 1, 0xffffffffu})
+    for (uint32_t first : {0u, 1u, 255u, stride / 2, stride - 1}) {
+      const uint64_t want = first < end ? ((uint64_t)end - first + stride - 1) / stride : 0;
+      uint64_t trips = 0;
+      uint64_t at = first;
+      for (uint32_t i = first; i < end && trips <= want; i = stride_next(i, stride, end)) {
+        if (i != at) std::printf("%u of %u\n", i, end);
+        at += stride;
+        ++trips;
+      }
+      if (trips != want) std::printf("%u to %u: %llu trips, not %llu\n", first, end,
+                                     (unsigned long long)trips, (unsigned long long)want);
+    }
+""")
+    assert lines == []
