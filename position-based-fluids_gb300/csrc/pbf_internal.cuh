@@ -230,6 +230,10 @@ inline size_t cell_sort_clear_words(const CellSortPlan &plan) {
 PBF_HOST_DEVICE inline uint32_t stride_next(uint32_t i, uint32_t stride, uint32_t end) {
   return end - i > stride ? i + stride : end;
 }
+// Whether `items` from index `at` on lie below `end` (at + items may be past 2^32).
+PBF_HOST_DEVICE inline bool whole_items(uint32_t at, uint32_t items, uint32_t end) {
+  return at < end && end - at >= items;
+}
 // Zeroes the counts and the control words (one launch).
 cudaError_t cell_sort_clear(const CellSortPlan &plan, uint32_t *scratch, cudaStream_t stream);
 // Offsets, scatter and in-cell order after the predict kernel has counted

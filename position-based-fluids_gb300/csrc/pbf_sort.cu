@@ -539,7 +539,8 @@ __global__ void __launch_bounds__(kSortThreads)
     const uint32_t base = tile * kScanTile + q * kScanChunk + tid * kScanItems;
     // two 16-byte loads where the counts are 16-byte aligned (base is a
     // multiple of 8)
-    if (base + kScanItems <= ncells && (reinterpret_cast<uintptr_t>(counts + base) & 15u) == 0u) {
+    if (whole_items(base, kScanItems, ncells) &&
+        (reinterpret_cast<uintptr_t>(counts + base) & 15u) == 0u) {
       const uint4 a = *reinterpret_cast<const uint4 *>(counts + base);
       const uint4 b = *reinterpret_cast<const uint4 *>(counts + base + 4);
       v[q][0] = a.x; v[q][1] = a.y; v[q][2] = a.z; v[q][3] = a.w;
@@ -560,7 +561,7 @@ __global__ void __launch_bounds__(kSortThreads)
       sum[q] += v[q][j];
     }
     if (any) {
-      if (base + kScanItems <= ncells &&
+      if (whole_items(base, kScanItems, ncells) &&
           (reinterpret_cast<uintptr_t>(counts + base) & 15u) == 0u) {
         *reinterpret_cast<uint4 *>(counts + base) = make_uint4(0, 0, 0, 0);
         *reinterpret_cast<uint4 *>(counts + base + 4) = make_uint4(0, 0, 0, 0);
@@ -638,7 +639,8 @@ __global__ void __launch_bounds__(kSortThreads)
       o[j] = run;
       run += v[q][j];
     }
-    if (base + kScanItems <= ncells && (reinterpret_cast<uintptr_t>(off + base) & 15u) == 0u) {
+    if (whole_items(base, kScanItems, ncells) &&
+        (reinterpret_cast<uintptr_t>(off + base) & 15u) == 0u) {
       *reinterpret_cast<uint4 *>(off + base) = make_uint4(o[0], o[1], o[2], o[3]);
       *reinterpret_cast<uint4 *>(off + base + 4) = make_uint4(o[4], o[5], o[6], o[7]);
     } else {

@@ -67,3 +67,16 @@ def test_grid_stride_ends_at_the_largest_counts(pbf, tmp_path):
     }
 """)
     assert lines == []
+
+
+def test_items_within_the_largest_counts(pbf, tmp_path):
+    """Whether a thread's eight cells lie below the end, also where the index
+    after the eighth is past 32 bits."""
+    lines = evaluate(pbf, tmp_path, r"""
+  for (uint64_t end : {0ull, 1ull, 7ull, 8ull, 9ull, 2048ull, 0xfffffff7ull, 0xfffffff8ull,
+                       0xfffffff9ull, 0xffffffffull})
+    for (uint64_t at : {0ull, 8ull, 2040ull, 0xffffffe8ull, 0xfffffff0ull, 0xfffffff8ull})
+      if (whole_items((uint32_t)at, 8, (uint32_t)end) != (at + 8 <= end))
+        std::printf("%llu of %llu\n", (unsigned long long)at, (unsigned long long)end);
+""")
+    assert lines == []
