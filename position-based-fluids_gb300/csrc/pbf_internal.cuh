@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstddef>
 
 #ifdef __CUDACC__
@@ -22,6 +23,24 @@ enum DeviceError : uint32_t {
   kDevErrLookback = 1u,  // a sort's look-back wait hit its bound
   kDevErrStage = 2u,     // a tile's bulk copies did not complete within the bounded wait
   kDevErrKey = 4u,       // the cell-sort operator got a key not below its cell count
+};
+
+// A setting of the current device's kernels, made the first time each device
+// needs it (a process can hold several): run(device, set) calls set() unless it
+// has succeeded on that device.  Two threads may both call it, and devices from
+// the 64th on call it every time.
+class OncePerDevice {
+  std::atomic<uint64_t> done{0};
+
+ public:
+  template <typename F>
+  cudaError_t run(int device, F &&set) {
+    const uint64_t bit = device >= 0 && device < 64 ? 1ull << device : 0ull;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    const cudaError_t e = set();
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+  }
 };
 
 // ------------------------------------------------------------ grid / scene --

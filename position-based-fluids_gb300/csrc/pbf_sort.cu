@@ -22,7 +22,6 @@
 // are already resident; every wait is additionally bounded, and a wait that
 // runs out sets a device error bit instead of spinning on.
 #include <algorithm>
-#include <mutex>
 
 #include "pbf_device.cuh"
 
@@ -322,9 +321,9 @@ __global__ void __launch_bounds__(kSweepThreads)
 }
 
 // Every instantiation takes its tile's shared memory dynamically (above the
-// 48 KB static limit with 9-bit digits); the limit is raised once.
-std::once_flag g_onesweep_once;
-cudaError_t g_onesweep_status = cudaSuccess;
+// 48 KB static limit: 66 KB with 8-bit digits, 100 KB with 9-bit ones); the limit
+// is raised once on each device.
+OncePerDevice g_onesweep_once;
 
 template <uint32_t kBits>
 cudaError_t allow_onesweep_smem() {
@@ -338,12 +337,13 @@ cudaError_t allow_onesweep_smem() {
 }
 
 cudaError_t onesweep_init() {
-  std::call_once(g_onesweep_once, [] {
-    cudaError_t e = allow_onesweep_smem<8>();
-    if (e == cudaSuccess) e = allow_onesweep_smem<9>();
-    g_onesweep_status = e;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return g_onesweep_once.run(device, [] {
+    const cudaError_t e = allow_onesweep_smem<8>();
+    return e == cudaSuccess ? allow_onesweep_smem<9>() : e;
   });
-  return g_onesweep_status;
 }
 
 template <uint32_t kBits>

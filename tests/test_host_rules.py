@@ -80,3 +80,24 @@ def test_items_within_the_largest_counts(pbf, tmp_path):
         std::printf("%llu of %llu\n", (unsigned long long)at, (unsigned long long)end);
 """)
     assert lines == []
+
+
+def test_kernel_attributes_once_per_device(pbf, tmp_path):
+    """A setting that belongs to a device is made on each of them, once, and
+    again after a failure."""
+    lines = evaluate(pbf, tmp_path, r"""
+  OncePerDevice once;
+  int calls = 0;
+  const auto good = [&] { ++calls; return cudaSuccess; };
+  const auto bad = [&] { ++calls; return cudaErrorInvalidValue; };
+  for (int device : {0, 0, 1, 0, 1, 63, 63}) once.run(device, good);
+  if (calls != 3) std::printf("%d calls on three devices\n", calls);
+  calls = 0;
+  if (once.run(2, bad) != cudaErrorInvalidValue) std::printf("failure lost\n");
+  if (once.run(2, good) != cudaSuccess || once.run(2, bad) != cudaSuccess || calls != 2)
+    std::printf("after a failure: %d calls\n", calls);
+  calls = 0;
+  for (int device : {64, 64, 1000}) once.run(device, good);  // beyond what it remembers
+  if (calls != 3) std::printf("%d calls beyond the table\n", calls);
+""")
+    assert lines == []
