@@ -235,11 +235,13 @@ int pbf_launches_per_step(const pbf_sim *sim, uint32_t *launches);
  * default); both give the stable permutation.  masked_build = 1 (the
  * default) has the list build (0 and 1) test each row of candidates into a
  * membership mask and store the members from the mask afterwards; 0 stores
- * each member as it is found.  With every field at its default, scenes of up
- * to 16,384 particles run their gather passes with eight threads per
- * particle instead, and those of up to 1,024 (in at most 6,144 cells) the
- * whole step in one launch; any other setting is taken as given.  No choice changes
- * a result bit.  trial_ms is the tuner's best time per launch of each pass (0 when
+ * each member as it is found.  With threads, batch, fuse_first, staged and
+ * masked_build at their defaults and one_thread = 0 (the default), scenes of
+ * up to 16,384 particles run their gather passes with eight threads per
+ * particle instead, and those of up to 1,024 (in at most 6,144 cells, with
+ * radix_sort = 0) the whole step in one launch; any other setting, and
+ * one_thread = 1, is taken as given.  No choice changes a result bit.
+ * trial_ms is the tuner's best time per launch of each pass (0 when
  * untuned). */
 typedef struct pbf_tuning {
   uint32_t threads[6];
@@ -249,6 +251,7 @@ typedef struct pbf_tuning {
   uint32_t staged;
   uint32_t radix_sort;
   uint32_t masked_build;
+  uint32_t one_thread;
 } pbf_tuning;
 /* Times every shape over `trial_steps` steps (1..32) of this simulation
  * from its current state, keeps the fastest per pass and restores the state

@@ -300,8 +300,8 @@ enum GatherKind : int {
 };
 
 // Launch shape of each gather pass.  No choice changes a result bit: every
-// variant computes each particle in one thread with the same operations in
-// the same order.
+// variant sums a particle's components with the same operations in the same
+// order, in one thread or, with eight threads per particle, a component each.
 struct GatherTuning {
   // threads per CTA, 64 << code: 128, except 256 for lambda and vorticity
   // (fastest over the 1M-particle dam break's 500 steps)
@@ -320,10 +320,18 @@ struct GatherTuning {
   // stores the members from it afterwards (same lists; 3% faster build, 6%
   // faster fused build on the 1M-particle dam break)
   uint8_t masked_build = 1;
-  // 1: scenes of few particles take eight threads per particle (pbf_group.cu)
-  // instead of these shapes.  Not part of pbf_tuning: a caller that sets any
-  // shape but the defaults gets that shape.
-  uint8_t grouped = 1;
+  // 1: these shapes for scenes of any size; 0: scenes of few particles take
+  // eight threads per particle (pbf_group.cu), unless a shape is not its default
+  uint8_t one_thread = 0;
+  bool grouped() const {
+    const GatherTuning standard;
+    if (one_thread || staged || fuse_first != standard.fuse_first ||
+        masked_build != standard.masked_build)
+      return false;
+    for (int k = 0; k < kGatherKinds; ++k)
+      if (block[k] != standard.block[k] || batch[k] != standard.batch[k]) return false;
+    return true;
+  }
 };
 constexpr int kBlockCodes = 3;  // 64, 128, 256
 constexpr int kBatchCodes = 2;  // 4, 8
@@ -507,7 +515,7 @@ cudaError_t paper_xsph_commit(const DeviceState &d, const PaperConsts &c,
 // once gain as well.
 constexpr uint32_t kGroupParticles = 16384;
 inline bool use_groups(const DeviceState &d, const PaperConsts &c) {
-  return d.tune.grouped && c.n <= kGroupParticles;
+  return d.tune.grouped() && c.n <= kGroupParticles;
 }
 // The whole step as one launch of one cluster, for scenes of up to
 // kTinyParticles particles in kTinyCells cells (everything its passes gather

@@ -5,7 +5,6 @@
 // compute_scaling.cl:16, XSPH c = 0.01 at apply_vorticity_and_viscosity.cl:103,
 // gravity -9.81 at predict_positions.cl:8, 4 iterations at
 // src/Simulation.cpp:503).
-#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -243,6 +242,7 @@ void to_pbf_tuning(const GatherTuning &g, const double trial_ms[kGatherKinds], p
   out->staged = g.staged;
   out->radix_sort = g.radix_sort;
   out->masked_build = g.masked_build;
+  out->one_thread = g.one_thread;
 }
 
 int to_gather_tuning(const pbf_tuning &t, GatherTuning *out) {
@@ -280,11 +280,11 @@ int to_gather_tuning(const pbf_tuning &t, GatherTuning *out) {
     return PBF_ERR_INVALID;
   }
   g.masked_build = (uint8_t)t.masked_build;
-  const GatherTuning standard;
-  g.grouped = !g.staged && g.fuse_first == standard.fuse_first &&
-              g.masked_build == standard.masked_build &&
-              std::equal(g.block, g.block + kGatherKinds, standard.block) &&
-              std::equal(g.batch, g.batch + kGatherKinds, standard.batch);
+  if (t.one_thread > 1) {
+    set_error_message("tuning: one_thread must be 0 or 1");
+    return PBF_ERR_INVALID;
+  }
+  g.one_thread = (uint8_t)t.one_thread;
   *out = g;
   return PBF_OK;
 }

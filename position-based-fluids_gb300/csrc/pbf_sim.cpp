@@ -175,7 +175,7 @@ cudaError_t step_offsets(pbf_sim *s) {
 // time of each pass and run them one by one; the bits are the same.
 bool use_tiny(const pbf_sim *s) {
   const GatherTuning &t = s->d.tune;
-  return s->paper && t.grouped && !t.radix_sort && !s->timing && !s->timed_capture &&
+  return s->paper && t.grouped() && !t.radix_sort && !s->timing && !s->timed_capture &&
          s->n <= s->tiny_particles && s->ncells <= kTinyCells;
 }
 

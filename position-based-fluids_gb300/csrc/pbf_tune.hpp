@@ -17,11 +17,12 @@ namespace pbf {
 // the shortest launches.  Then it times whole steps of that choice against
 // the staged tiles (pbf_tile.cu) from the same state and keeps the staged
 // passes when their steps are more than kTuneMargin faster, and for small
-// scenes against the passes with eight threads per particle (pbf_group.cu).  The current shapes are timed first and a pass
-// moves to another shape only when that one is more than kTuneMargin
-// faster: on a near-tie the pick would follow timing noise, and the
-// defaults are the shapes measured fastest over a whole dam break, where
-// later states separate shapes that tie on the starting lattice.  X, V and
+// scenes against the passes with eight threads per particle (pbf_group.cu).
+// The current shapes are timed first and a pass moves to another shape only
+// when that one is more than kTuneMargin faster: on a near-tie the pick would
+// follow timing noise, and the defaults are the shapes measured fastest over
+// a whole dam break, where later states separate shapes that tie on the
+// starting lattice.  X, V and
 // ID of the first n slots are saved before and restored after, so the
 // caller's state is unchanged; since no shape changes a result bit, later
 // steps are the ones an untuned run would take.
@@ -60,12 +61,13 @@ int paper_autotune(DeviceState &d, uint32_t n, cudaStream_t st, uint32_t trials,
       t.batch[k] = (uint8_t)batch;
     }
     t.fuse_first = (uint8_t)fuse;
-    t.grouped = 0;
+    t.one_thread = 1;
     return t;
   };
   const GatherTuning before = d.tune;
   GatherTuning best = before;
-  best.staged = best.grouped = 0;
+  best.staged = 0;
+  best.one_thread = 1;
   double best_ms[kGatherKinds];
   for (int k = 0; k < kGatherKinds; ++k) best_ms[k] = std::numeric_limits<double>::infinity();
   // Runs `trials` steps (one, untimed, when !timed) with shapes t from the
@@ -105,7 +107,8 @@ int paper_autotune(DeviceState &d, uint32_t n, cudaStream_t st, uint32_t trials,
       const bool timed = pass == 1;
       if (timed) {
         GatherTuning cur = before;
-        cur.staged = cur.grouped = 0;
+        cur.staged = 0;
+        cur.one_thread = 1;
         for (int fuse = 0; fuse < 2 && rc == PBF_OK; ++fuse) {
           cur.fuse_first = (uint8_t)fuse;
           if (!trial(cur, true, true)) break;
@@ -150,6 +153,8 @@ int paper_autotune(DeviceState &d, uint32_t n, cudaStream_t st, uint32_t trials,
         int pick = step_ms[1] < step_ms[0] * (1.0 - kTuneMargin) ? 1 : 0;
         if (count == 3 && step_ms[pick] >= step_ms[2] * (1.0 - kTuneMargin)) pick = 2;
         best = variants[pick];
+        // (not compared at this size: a batch can hold fewer particles later)
+        if (count == 2) best.one_thread = before.one_thread;
       }
     }
     if (e0) cudaEventDestroy(e0);

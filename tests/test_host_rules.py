@@ -15,7 +15,7 @@ def evaluate(pbf, tmp_path, code: str) -> list[str]:
     build = importlib.import_module(pbf.__name__ + ".build")
     src, exe = tmp_path / "rule.cpp", tmp_path / "rule"
     src.write_text('#include <algorithm>\n#include <cstdint>\n#include <cstdio>\n'
-                   '#include "pbf_internal.cuh"\nusing namespace pbf;\n'
+                   '#include "pbf_host.hpp"\nusing namespace pbf;\n'
                    f'int main() {{\n{code}\n}}\n')
     pkg = pbf.LIB_PATH.parent
     subprocess.run([build.CXX, *build.CXX_FLAGS, "-I", str(pkg / "csrc"), str(src), "-o", str(exe),
@@ -99,5 +99,40 @@ def test_kernel_attributes_once_per_device(pbf, tmp_path):
   calls = 0;
   for (int device : {64, 64, 1000}) once.run(device, good);  // beyond what it remembers
   if (calls != 3) std::printf("%d calls beyond the table\n", calls);
+""")
+    assert lines == []
+
+
+def test_tuning_survives_the_round_trip(pbf, tmp_path):
+    """What pbf_get_tuning reports selects, set again, the passes it was read
+    from: for every field, also one thread per particle in the default shapes,
+    which the tuner can pick for a small scene."""
+    lines = evaluate(pbf, tmp_path, r"""
+  int grouped = 0;
+  for (uint32_t bits = 0; bits < 128; ++bits) {
+    GatherTuning g, back;
+    g.one_thread = bits & 1;
+    g.fuse_first = bits >> 1 & 1;
+    g.staged = bits >> 2 & 1;
+    g.radix_sort = bits >> 3 & 1;
+    g.masked_build = bits >> 4 & 1;
+    if (bits >> 5 & 1) g.block[kKindDelta] = 0;
+    if (bits >> 6 & 1) g.batch[kKindXsph] = 1;
+    pbf_tuning t;
+    to_pbf_tuning(g, nullptr, &t);
+    if (to_gather_tuning(t, &back) != PBF_OK) std::printf("%u refused\n", bits);
+    if (back.grouped() != g.grouped() || back.one_thread != g.one_thread ||
+        back.fuse_first != g.fuse_first || back.staged != g.staged ||
+        back.radix_sort != g.radix_sort || back.masked_build != g.masked_build ||
+        !std::equal(g.block, g.block + kGatherKinds, back.block) ||
+        !std::equal(g.batch, g.batch + kGatherKinds, back.batch))
+      std::printf("%u comes back as another\n", bits);
+    grouped += g.grouped();
+    t.one_thread = 2;
+    if (to_gather_tuning(t, &back) != PBF_ERR_INVALID) std::printf("%u: one_thread = 2\n", bits);
+  }
+  if (grouped != 2) std::printf("eight threads in %d of them\n", grouped);  // either sort
+  const pbf_tuning zero{};  // a caller that leaves the field out: as the other fields say
+  if (zero.one_thread != GatherTuning().one_thread) std::printf("not the default\n");
 """)
     assert lines == []
