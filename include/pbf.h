@@ -100,6 +100,10 @@ typedef struct {
   float gravity_y;                /* [gravity_y] paper mode               */
   float wall_margin;              /* [wall_margin] paper mode, in metres  */
   uint32_t max_neighbours;        /* [max_neighbours] stored per particle */
+                                  /* (REF_COMPAT: 128 at most, and fewer  */
+                                  /* or none when the lists would take    */
+                                  /* more than 1/16 of the device's       */
+                                  /* memory or half of what is free)      */
   uint32_t grow_lists;            /* [grow_lists] 1: a simulation's list  */
                                   /* capacity grows with its scene (see   */
                                   /* pbf_list_capacity); 0: fixed         */

@@ -393,22 +393,21 @@ int collect_times(pbf_sim *s) {
   return PBF_OK;
 }
 
-// Neighbour lists of the reference-equation passes: max_neighbours entries
-// per particle (8 to 128), halved until they take at most half of the free
-// memory; a scene so large that not even 8 entries fit runs without lists.
+// Neighbour lists of the reference-equation passes (ref_list_entries); a scene
+// with no room for them runs without.
 int alloc_ref_lists(pbf_sim *s) {
   size_t free_bytes = 0, total = 0;
   PBF_TRY(cudaMemGetInfo(&free_bytes, &total));
-  uint32_t maxn = std::min(128u, std::max(8u, s->prm.max_neighbours / 8u * 8u));
   s->rc_maxn = 0;
-  for (; maxn >= 8u; maxn = maxn / 16u * 8u) {
+  uint64_t room = ref_list_room(free_bytes, total);
+  while (const uint32_t maxn = ref_list_entries(s->prm.max_neighbours, s->n, room)) {
     const size_t count = (size_t)paper_list_words(maxn) * s->n;
-    if (count * sizeof(uint4) > free_bytes / 2) continue;
     if (dalloc(s, &s->d.nbr, count) == PBF_OK) {
       s->rc_maxn = maxn;
       return PBF_OK;
     }
-    cudaGetLastError();  // try fewer entries
+    cudaGetLastError();
+    room = count * sizeof(uint4) - 1;  // try fewer entries
   }
   return PBF_OK;
 }

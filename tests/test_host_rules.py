@@ -136,3 +136,36 @@ def test_tuning_survives_the_round_trip(pbf, tmp_path):
   if (zero.one_thread != GatherTuning().one_thread) std::printf("not the default\n");
 """)
     assert lines == []
+
+
+def test_reference_lists_leave_the_memory(pbf, tmp_path):
+    """Neighbour lists of the reference's equations take a bounded share of the
+    device whatever its size and the scene's, do not depend on what else is
+    allocated while that leaves twice the share, and are dropped where only lists
+    too short to hold a set at rest would fit."""
+    lines = evaluate(pbf, tmp_path, r"""
+  const uint64_t gib = 1ull << 30;
+  for (uint64_t total : {8 * gib, 80 * gib, 280 * gib})
+    for (uint64_t n : {1ull, 1000ull, 1048576ull, 17000000ull, 34000000ull, 100000000ull,
+                       300000000ull, 1073741823ull})
+      for (uint32_t maxn : {1u, 8u, 9u, 16u, 24u, 31u, 32u, 40u, 64u, 100u, 128u, 1024u}) {
+        const uint32_t all = ref_list_entries(maxn, n, ref_list_room(total, total));
+        for (uint64_t eighths = 0; eighths <= 8; ++eighths) {
+          const uint64_t left = total / 8 * eighths;
+          const uint32_t e = ref_list_entries(maxn, n, ref_list_room(left, total));
+          const uint64_t bytes = (uint64_t)paper_list_words(e) * sizeof(uint4) * n;
+          const uint32_t most = std::min(128u, std::max(8u, maxn / 8 * 8));
+          const char *wrong = nullptr;
+          if (bytes > total / 16 || bytes > left / 2) wrong = "too much";
+          else if (e % 8 || e > most || (e && e < std::min(most, 32u))) wrong = "entries";
+          else if (eighths && e != all) wrong = "depends on the rest";
+          else if (e != most && 4 * n * most <= std::min(left / 2, total / 16)) wrong = "too few";
+          if (wrong) std::printf("%s: %u of %u, n %llu, %llu of %llu GiB\n", wrong, e, maxn,
+                                 (unsigned long long)n, (unsigned long long)(left / gib),
+                                 (unsigned long long)(total / gib));
+        }
+      }
+  if (ref_list_entries(128, 4194304, ref_list_room(280 * gib, 280 * gib)) != 128)
+    std::printf("4,194,304 particles without whole lists\n");
+""")
+    assert lines == []
