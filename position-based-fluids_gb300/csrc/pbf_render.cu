@@ -352,19 +352,7 @@ void render_view_matrix(const pbf_camera &cam, float aspect, float out[16]) {
   mat_mul(proj, view, out);
 }
 
-// Sprites drawn in two parts, the second without what the first hides
-// (k_render_splat_rest): images of many sprites that hide each other.  Frames in
-// one part and in two: 152k particles at 1280 x 720 185 and 151 us, at 320 x 200
-// 142 and 101, 1M at 1920 x 1080 401 and 299; with fewer sprites the two parts
-// do not fill the GPU (69k at 1280 x 720 162 and 175, 33k at 640 x 360 105 and
-// 143), in larger images fewer lie behind others (91k at 1920 x 1080 259 and
-// 293), and small sprites take less time than placing them twice (134k of five
-// pixels across 113 and 127, 160k of ten 97 and 89).  Between a quarter and a
-// sixteenth of the sprites first, an eighth was best.
-constexpr uint32_t kCullSprites = 81920;
-constexpr uint32_t kCullPixels = 14;       // of the image per sprite, at most
-constexpr float kCullDrawn = 10485760.0f;  // pixels of all sprites, at least
-constexpr uint32_t kFirstSprites = 8;      // one in so many
+constexpr uint32_t kFirstSprites = 8;  // of two parts, the first: one sprite in so many
 
 // More scratch than this is not kept from one image to the next.
 constexpr size_t kRenderKeep = (size_t)256 << 20;
@@ -404,8 +392,7 @@ int render_particles(const float4 *X, const uint32_t *ID, uint32_t n, const pbf_
                                                                                 n, slot_of);
   // (a sprite's size at the camera's target)
   const float size = std::fmin(200.0f / std::fabs(cam.distance), v.max_size);
-  const bool cull = n >= kCullSprites && (uint64_t)n * kCullPixels >= pixels &&
-                    (float)n * size * size >= kCullDrawn;
+  const bool cull = draws_in_two_parts(n, pixels, size);
   const uint32_t drawn = cull ? n / kFirstSprites : n;
   if (n)
     k_render_splat<<<(uint32_t)(((uint64_t)drawn * kSpriteThreads + 127u) / 128u), 128, 0, st>>>(
