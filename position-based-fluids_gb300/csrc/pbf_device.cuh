@@ -49,33 +49,53 @@ __device__ __forceinline__ void warp_digit_histogram(uint32_t key, bool valid,
 // Counts kKeys keys per lane (whole warp) into counts[] for the counting sort,
 // all their atomics in flight together: one atomic per run of equal keys in
 // neighbouring lanes; pos[i] = the particle's place among the increments of
-// its cell (a run's lanes in order, runs in atomic order).
-template <int kKeys>
+// its cell (a group's lanes in order, groups in atomic order).
+// kScattered: keys in any order, so a warp in which some lanes 2, 4, 8 or 16 apart
+// hold the same key joins all equal ones: the atomics on one word wait for each
+// other, about 1 ns each.  1M random keys of 2 cells are counted in 24 us (a run at
+// a time 181), of 8 cells 22 (125), 4.2M of which half are the same 192 (288), 4.2M
+// nearly in order 23 (31; all warps through __match_any_sync, a round per distinct
+// key, 33).  A step's kernels count by runs alone: with so many particles per cell
+// its passes over the pairs take a thousand times as long.
+template <bool kScattered, int kKeys>
 __device__ __forceinline__ void count_cell_keys(const uint32_t (&key)[kKeys],
                                                 const bool (&valid)[kKeys],
                                                 const uint32_t (&i)[kKeys],
                                                 uint32_t *__restrict__ counts,
                                                 uint32_t *__restrict__ pos) {
+  constexpr unsigned kWarp = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31u;
-  uint32_t head[kKeys], base[kKeys];
+  unsigned group[kKeys];  // lanes counted by one atomic, the caller among them
+  uint32_t base[kKeys];
 #pragma unroll
   for (int u = 0; u < kKeys; ++u) {
-    const uint32_t before = __shfl_up_sync(0xffffffffu, key[u], 1);
-    const bool valid_before = __shfl_up_sync(0xffffffffu, (int)valid[u], 1);
+    const uint32_t before = __shfl_up_sync(kWarp, key[u], 1);
+    const bool valid_before = __shfl_up_sync(kWarp, (int)valid[u], 1);
     const unsigned heads =
-        __ballot_sync(0xffffffffu, lane == 0u || key[u] != before || valid[u] != valid_before);
+        __ballot_sync(kWarp, lane == 0u || key[u] != before || valid[u] != valid_before);
     // the caller's run: from the last head at or below its lane to the next one
-    const unsigned below = 0xffffffffu >> (31u - lane);
-    head[u] = 31u - (uint32_t)__clz((int)(heads & below));
+    const unsigned below = kWarp >> (31u - lane);
+    const uint32_t head = 31u - (uint32_t)__clz((int)(heads & below));
     const unsigned later = heads & ~below;
     const uint32_t end = later ? (uint32_t)__ffs((int)later) - 1u : 32u;
+    group[u] = kWarp >> (32u - (end - head)) << head;
+    if (kScattered && __popc(heads) > 4) {
+      bool apart = false;  // the caller's key in another run
+#pragma unroll
+      for (uint32_t o = 2; o <= 16; o <<= 1) {
+        const uint32_t other = __shfl_xor_sync(kWarp, key[u], (int)o);  // every lane
+        apart |= other == key[u] && !(group[u] >> (lane ^ o) & 1u);
+      }
+      if (__any_sync(kWarp, apart)) group[u] = __match_any_sync(kWarp, valid[u] ? key[u] : kWarp);
+    }
     base[u] = 0;
-    if (valid[u] && lane == head[u]) base[u] = atomicAdd(&counts[key[u]], end - head[u]);
+    if (valid[u] && lane == (uint32_t)__ffs((int)group[u]) - 1u)
+      base[u] = atomicAdd(&counts[key[u]], (uint32_t)__popc(group[u]));
   }
 #pragma unroll
   for (int u = 0; u < kKeys; ++u) {
-    const uint32_t first = __shfl_sync(0xffffffffu, base[u], (int)head[u]);
-    if (valid[u]) pos[i[u]] = first + (lane - head[u]);
+    const uint32_t first = __shfl_sync(kWarp, base[u], __ffs((int)group[u]) - 1);
+    if (valid[u]) pos[i[u]] = first + (uint32_t)__popc(group[u] & ((1u << lane) - 1u));
   }
 }
 // Keys a thread takes at a time in the counting, predicting and scattering

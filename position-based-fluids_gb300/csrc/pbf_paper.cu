@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(256)
         keys[k[u]] = key[u];
       }
     }
-    count_cell_keys(key, valid, k, counts, pos);
+    count_cell_keys<false>(key, valid, k, counts, pos);
   }
 }
 

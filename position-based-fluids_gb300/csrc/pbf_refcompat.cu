@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256)
     const bool valid[1] = {t[0] < n};
     uint32_t key[1] = {0};
     if (valid[0]) keys[t[0]] = key[0] = rc_predict(t[0], n, X, V, P, k, scenes[0]);
-    count_cell_keys(key, valid, t, counts, pos);
+    count_cell_keys<false>(key, valid, t, counts, pos);
   }
 }
 

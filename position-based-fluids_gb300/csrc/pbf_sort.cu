@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(256)
       valid[u] = i[u] < n && key[u] < ncells;
       if (i[u] < n && !valid[u]) atomicOr(err, kDevErrKey);
     }
-    count_cell_keys(key, valid, i, counts, pos);
+    count_cell_keys<true>(key, valid, i, counts, pos);
   }
 }
 
