@@ -467,6 +467,10 @@ constexpr uint32_t kScanChunks = 4;    // chunks per scan tile, where there are 
 // the look-back over at most these tiles (they fit the control words).
 constexpr uint32_t kFewTiles = 56;
 constexpr uint32_t kSmallCell = 16;
+// Cells of up to this many particles are sorted where sparse grids test them:
+// listing a cell is an atomic on one word.  1M random keys in 2M cells 28.3 ->
+// 11.9 us, 4.2M in 4.2M cells nearly in order 76 -> 22.
+constexpr uint32_t kLightCell = 4;
 constexpr uint32_t kWarpCell = 64;  // cells of 17..64 particles: one warp each
 // control words: [0] scan tiles started, [1] big cells, [2] huge cells,
 // [3] the operator's error word, [4] out-of-order small cells, [5] cells
@@ -731,38 +735,38 @@ __device__ __forceinline__ void merge_steps(uint32_t *v) {
         }
 }
 
-// The m <= kSmallCell indices from perm[a] in order, in registers: all loaded
+// The m <= kMost indices from perm[a] in order, in registers: all loaded
 // together, none stored when they were in order, the upper half of the network
 // left out where it is empty.  Cells of 4.2M particles in 15.2 -> 11 us against
 // four loads at a time and a bitonic network of 80 exchanges (this one has 19
 // for 8 indices, 63 for 16); bounded by its instructions, and slower with fewer
 // than its 62 registers.
-__device__ __forceinline__ void sort_small_cell(uint32_t *__restrict__ perm, uint32_t a,
-                                                uint32_t m) {
-  constexpr uint32_t kHalf = kSmallCell / 2;
-  uint32_t v[kSmallCell];
+template <uint32_t kMost>
+__device__ __forceinline__ void sort_cell(uint32_t *__restrict__ perm, uint32_t a, uint32_t m) {
+  constexpr uint32_t kHalf = kMost / 2;
+  uint32_t v[kMost];
 #pragma unroll
-  for (uint32_t j = 0; j < kSmallCell; ++j) v[j] = j < m ? perm[a + j] : 0xffffffffu;
+  for (uint32_t j = 0; j < kMost; ++j) v[j] = j < m ? perm[a + j] : 0xffffffffu;
   bool sorted = true;
 #pragma unroll
-  for (uint32_t j = 1; j < kSmallCell; ++j) sorted = sorted && v[j] >= v[j - 1];
+  for (uint32_t j = 1; j < kMost; ++j) sorted = sorted && v[j] >= v[j - 1];
   if (sorted) return;
   merge_steps<1, kHalf>(v);
   if (m > kHalf) {
     merge_steps<1, kHalf>(v + kHalf);
-    merge_steps<kHalf, kSmallCell>(v);
+    merge_steps<kHalf, kMost>(v);
   }
 #pragma unroll
-  for (uint32_t j = 0; j < kSmallCell; ++j)
+  for (uint32_t j = 0; j < kMost; ++j)
     if (j < m) perm[a + j] = v[j];
 }
 
 // One thread per cell.  A cell of 2..kSmallCell particles whose indices are
 // out of order (most are in order: their particles were counted by one warp)
 // is sorted here (kSortHere, on grids with at least two particles per cell)
-// or listed for k_cell_fix_big (sparse grids, where this kernel runs over
-// mostly empty cells and is kept light in registers); larger cells are
-// listed by size.
+// or, on sparse grids, where this kernel runs over mostly empty cells and is
+// kept light in registers, sorted here up to kLightCell particles and listed
+// for k_cell_fix_big above; larger cells are listed by size.
 template <bool kSortHere>
 __global__ void __launch_bounds__(256)
     k_cell_fix(const uint32_t *__restrict__ off, uint32_t ncells, uint32_t *__restrict__ perm,
@@ -787,7 +791,11 @@ __global__ void __launch_bounds__(256)
     return;
   }
   if (kSortHere) {
-    sort_small_cell(perm, a, m);
+    sort_cell<kSmallCell>(perm, a, m);
+    return;
+  }
+  if (m <= kLightCell) {
+    sort_cell<kLightCell>(perm, a, m);
     return;
   }
   // four indices in flight at a time (past the cell's end its last one)
@@ -862,7 +870,7 @@ __global__ void __launch_bounds__(kSortThreads)
   for (uint32_t w = blockIdx.x * kSortThreads + tid; w < nsmall; w += gridDim.x * kSortThreads) {
     const uint32_t c = small[w];
     const uint32_t a = off[c];
-    sort_small_cell(perm, a, off[c + 1] - a);
+    sort_cell<kSmallCell>(perm, a, off[c + 1] - a);
   }
   // cells of 17..64: one warp each
   const uint32_t nmed = min(ctl[5], med_cap);
