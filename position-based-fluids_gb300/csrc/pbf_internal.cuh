@@ -611,6 +611,10 @@ cudaError_t rc_delta(const float4 *PS, float4 *PS2, const float *SS, const RefLi
 cudaError_t rc_xsph(const float4 *PS, const float4 *planes, const float4 *VS, float4 *DV,
                     const uint32_t *input, const uint32_t *offsets, uint32_t n, const RefConsts &k,
                     cudaStream_t st);
+// Cell of every particle by input index in the reference's numbering (x
+// fastest), from the step's keys (z fastest, descending input index).
+cudaError_t rc_view_keys(const uint32_t *keys, uint32_t n, const SceneDesc &scene, uint32_t *out,
+                         cudaStream_t st);
 cudaError_t rc_commit(float4 *X, float4 *V, const float4 *P, const float4 *DV,
                       uint32_t n, cudaStream_t st);
 

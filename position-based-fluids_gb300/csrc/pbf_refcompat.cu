@@ -610,6 +610,18 @@ __global__ void __launch_bounds__(kGroupThreads)
   DV[input[q]] = make_float4(0.01f * s[0], 0.01f * s[1], 0.01f * s[2], 0.0f);
 }
 
+// Keys of the sort elements (cells with z fastest, descending input index) as the
+// cells of the particles with x fastest.
+__global__ void __launch_bounds__(256)
+    k_rc_view_keys(const uint32_t *__restrict__ keys, uint32_t n, uint32_t nx, uint32_t ny,
+                   uint32_t nz, uint32_t *__restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t k = keys[n - 1u - i];
+  const uint32_t z = k % nz, y = k / nz % ny, x = k / nz / ny;
+  out[i] = x + nx * (y + ny * z);
+}
+
 __global__ void __launch_bounds__(256)
     k_rc_commit(float4 *__restrict__ X, float4 *__restrict__ V,
                 const float4 *__restrict__ P, const float4 *__restrict__ DV,
@@ -693,6 +705,14 @@ cudaError_t rc_xsph(const float4 *PS, const float4 *planes, const float4 *VS, fl
   else
     k_rc_xsph<<<blocks_for(n, kThreads), kThreads, 0, st>>>(PS, make_planes(planes, n), VS, DV,
                                                             input, offsets, n, k);
+  return cudaGetLastError();
+}
+
+cudaError_t rc_view_keys(const uint32_t *keys, uint32_t n, const SceneDesc &scene, uint32_t *out,
+                         cudaStream_t st) {
+  k_rc_view_keys<<<blocks_for(n, 256), 256, 0, st>>>(keys, n, (uint32_t)scene.ncell[0],
+                                                     (uint32_t)scene.ncell[1],
+                                                     (uint32_t)scene.ncell[2], out);
   return cudaGetLastError();
 }
 

@@ -164,11 +164,12 @@ int mark(pbf_sim *s, int stage, const char *name, uint32_t launches,
   return PBF_OK;
 }
 
-cudaError_t step_offsets(pbf_sim *s) {
+// The cell offsets from the sorted keys.
+cudaError_t step_offsets(pbf_sim *s, const uint32_t *skeys) {
   DeviceState &d = s->d;
   if (s->offset_runs)
-    return cell_offsets_runs(d.skeys, s->n, s->ncells, d.offsets, d.runs, d.runs_count, s->stream);
-  return cell_offsets(d.skeys, s->n, s->ncells, d.offsets, s->stream);
+    return cell_offsets_runs(skeys, s->n, s->ncells, d.offsets, d.runs, d.runs_count, s->stream);
+  return cell_offsets(skeys, s->n, s->ncells, d.offsets, s->stream);
 }
 
 // Whether the step runs as one launch (pbf_group.cu).  Timed steps report the
@@ -209,7 +210,7 @@ int launch_step(pbf_sim *s) {
     PBF_TRY(sort_passes(s->plan, d.keys, nullptr, d.skeys, d.perm,
                         d.sort_scratch, d.err, st));
     PBF_TRY_STATUS(mark(s, 0, "sort_onesweep", passes, &ev));
-    PBF_TRY(step_offsets(s));
+    PBF_TRY(step_offsets(s, d.skeys));
     PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
   }
   if (s->paper) {
@@ -269,7 +270,7 @@ int launch_step(pbf_sim *s) {
       PBF_TRY_STATUS(mark(s, 0, "rc_predict_hash", 1, &ev));
       PBF_TRY(sort_passes(s->plan, d.keys, nullptr, d.skeys, d.perm, d.sort_scratch, d.err, st));
       PBF_TRY_STATUS(mark(s, 0, "sort_onesweep", passes, &ev));
-      PBF_TRY(step_offsets(s));
+      PBF_TRY(step_offsets(s, d.skeys));
       PBF_TRY_STATUS(mark(s, 0, "cell_offsets", 1, &ev));
     }
     const StepClear clear = step_clear(s->cplan, d.cell_scratch, nullptr);
@@ -414,35 +415,37 @@ int alloc_ref_lists(pbf_sim *s) {
 
 bool ready(const pbf_sim *s) { return s && s->inited; }
 
+// The first and last slot of every cell, from the offsets, to the host.
+int copy_ranges(pbf_sim *s, int32_t *ranges) {
+  if (!s->d_ranges) PBF_TRY_STATUS(dalloc(s, &s->d_ranges, 2 * (size_t)s->ncells));
+  PBF_TRY(find_cells(s->d.offsets, s->ncells, s->d_ranges, s->stream));
+  PBF_TRY(cudaMemcpyAsync(ranges, s->d_ranges, (size_t)s->ncells * 8, cudaMemcpyDeviceToHost,
+                          s->stream));
+  return PBF_OK;
+}
+
 // pbf_get_cells in REF_COMPAT mode, in the reference's numbering (x fastest,
 // ties by input index): the step's own structure numbers the cells with z
-// fastest and runs over descending input index, so the views are counted out
-// here from each particle's cell.
+// fastest and runs over descending input index, so the views are sorted out
+// here from each particle's cell, in io_vel (which this mode's state transfers
+// do not use) and the offsets (which every step writes anew).
 int ref_cells(pbf_sim *s, uint32_t *hash, uint32_t *perm, int32_t *ranges) {
+  DeviceState &d = s->d;
   const size_t n = s->n;
-  std::vector<uint32_t> key(n);
-  PBF_TRY(cudaMemcpyAsync(key.data(), s->d.keys, n * 4, cudaMemcpyDeviceToHost, s->stream));
-  PBF_TRY(cudaStreamSynchronize(s->stream));
-  std::reverse(key.begin(), key.end());
-  const uint32_t nx = (uint32_t)s->scene.ncell[0], ny = (uint32_t)s->scene.ncell[1],
-                 nz = (uint32_t)s->scene.ncell[2];
-  for (uint32_t &k : key) {
-    const uint32_t z = k % nz, y = k / nz % ny, x = k / nz / ny;
-    k = x + nx * (y + ny * z);
+  uint32_t *key = reinterpret_cast<uint32_t *>(d.io_vel), *skeys = key + n, *order = skeys + n;
+  PBF_TRY(rc_view_keys(d.keys, s->n, s->scene, key, s->stream));
+  if (hash) PBF_TRY(cudaMemcpyAsync(hash, key, n * 4, cudaMemcpyDeviceToHost, s->stream));
+  if (perm || ranges) {
+    PBF_TRY(sort_clear(s->plan, d.sort_scratch, s->stream));
+    PBF_TRY(sort_histogram(s->plan, key, d.sort_scratch, s->stream));
+    PBF_TRY(sort_passes(s->plan, key, nullptr, skeys, order, d.sort_scratch, d.err, s->stream));
   }
-  if (hash) std::memcpy(hash, key.data(), n * 4);
-  if (!perm && !ranges) return PBF_OK;
-  std::vector<uint32_t> start((size_t)s->ncells + 1, 0u);
-  for (const uint32_t k : key) ++start[(size_t)k + 1];
-  for (size_t c = 0; c < s->ncells; ++c) start[c + 1] += start[c];
-  if (ranges)
-    for (size_t c = 0; c < s->ncells; ++c) {
-      const bool any = start[c] < start[c + 1];
-      ranges[2 * c] = any ? (int32_t)start[c] : -1;
-      ranges[2 * c + 1] = any ? (int32_t)start[c + 1] - 1 : -1;
-    }
-  if (perm)
-    for (size_t i = 0; i < n; ++i) perm[start[key[i]]++] = (uint32_t)i;
+  if (perm) PBF_TRY(cudaMemcpyAsync(perm, order, n * 4, cudaMemcpyDeviceToHost, s->stream));
+  if (ranges) {
+    PBF_TRY(step_offsets(s, skeys));
+    PBF_TRY_STATUS(copy_ranges(s, ranges));
+  }
+  PBF_TRY(cudaStreamSynchronize(s->stream));
   return PBF_OK;
 }
 
@@ -891,12 +894,7 @@ int pbf_get_cells(pbf_sim *s, uint32_t *hash, uint32_t *perm, int32_t *ranges) {
   std::vector<uint32_t> skeys(n), p(n);
   PBF_TRY(cudaMemcpyAsync(skeys.data(), s->d.skeys, n * 4, cudaMemcpyDeviceToHost, s->stream));
   PBF_TRY(cudaMemcpyAsync(p.data(), s->d.ID, n * 4, cudaMemcpyDeviceToHost, s->stream));
-  if (ranges) {
-    if (!s->d_ranges) PBF_TRY_STATUS(dalloc(s, &s->d_ranges, 2 * (size_t)s->ncells));
-    PBF_TRY(find_cells(s->d.offsets, s->ncells, s->d_ranges, s->stream));
-    PBF_TRY(cudaMemcpyAsync(ranges, s->d_ranges, (size_t)s->ncells * 8,
-                            cudaMemcpyDeviceToHost, s->stream));
-  }
+  if (ranges) PBF_TRY_STATUS(copy_ranges(s, ranges));
   PBF_TRY(cudaStreamSynchronize(s->stream));
   if (hash)
     for (size_t q = 0; q < n; ++q) hash[p[q]] = skeys[q];
