@@ -83,6 +83,16 @@ inline bool draws_in_two_parts(uint32_t n, uint32_t pixels, float size) {
          (float)n * size * size >= kCullDrawn;
 }
 
+// Threads per sprite and per CTA, the CTAs of `count` sprites, and the sprite of a
+// thread (eight threads per sprite number past 2^32 at 2^29 sprites).
+constexpr uint32_t kSpriteThreads = 8, kSpriteCta = 128;
+inline uint32_t sprite_ctas(uint32_t count) {
+  return (uint32_t)(((uint64_t)count * kSpriteThreads + kSpriteCta - 1u) / kSpriteCta);
+}
+PBF_HOST_DEVICE inline uint32_t sprite_of_thread(uint32_t block, uint32_t thread) {
+  return block * (kSpriteCta / kSpriteThreads) + thread / kSpriteThreads;
+}
+
 // Renders n particles (X: position, .w = |v|; ID: input index of each slot,
 // or null when slot = input index) of the box of `prm` into rgb (host).
 int render_particles(const float4 *X, const uint32_t *ID, uint32_t n, const pbf_params &prm,

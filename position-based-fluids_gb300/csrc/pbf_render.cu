@@ -92,13 +92,12 @@ __global__ void k_render_clear(unsigned long long *__restrict__ zbuf, uint32_t p
 // 322 -> 91 us (99 in slot order), bound by its instructions, 37 per warp and
 // pixel row.  An eighth of them takes 28 us: with every sprite in flight at
 // once most of their pixels are atomics.
-constexpr uint32_t kSpriteThreads = 8;
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(kSpriteCta)
     k_render_splat(const float4 *__restrict__ X, const uint32_t *__restrict__ ID, uint32_t n,
                    uint32_t count, uint32_t stride, RenderView v, unsigned long long *zbuf) {
   const uint32_t lane = threadIdx.x & (kSpriteThreads - 1u);
   const unsigned group = 0xffu << (threadIdx.x & 31u & ~(kSpriteThreads - 1u));
-  const uint32_t i = (blockIdx.x * 128u + threadIdx.x) / kSpriteThreads;
+  const uint32_t i = sprite_of_thread(blockIdx.x, threadIdx.x);
   if (i >= count) return;
   const uint32_t k = (uint32_t)((uint64_t)i * stride % n);
   const float4 p = X[k];
@@ -395,7 +394,7 @@ int render_particles(const float4 *X, const uint32_t *ID, uint32_t n, const pbf_
   const bool cull = draws_in_two_parts(n, pixels, size);
   const uint32_t drawn = cull ? n / kFirstSprites : n;
   if (n)
-    k_render_splat<<<(uint32_t)(((uint64_t)drawn * kSpriteThreads + 127u) / 128u), 128, 0, st>>>(
+    k_render_splat<<<sprite_ctas(drawn), kSpriteCta, 0, st>>>(
         X, ID, n, drawn, sprite_stride(n), v, zbuf);
   if (cull) {
     k_render_far<<<(blocks * 8u + 255u) / 256u, 256, 0, st>>>(zbuf, (int)width, (int)height,

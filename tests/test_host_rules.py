@@ -169,3 +169,22 @@ def test_reference_lists_leave_the_memory(pbf, tmp_path):
     std::printf("4,194,304 particles without whole lists\n");
 """)
     assert lines == []
+
+
+def test_every_sprite_is_drawn(pbf, tmp_path):
+    """The threads of the sprites' kernel hold every sprite's number, also where
+    the threads number past 2^32."""
+    lines = evaluate(pbf, tmp_path, r"""
+  for (uint32_t count : {1u, 15u, 16u, 17u, 81920u, (1u << 29) - 1u, 1u << 29, (1u << 29) + 1u,
+                         (1u << 30) - 1u}) {
+    const uint32_t ctas = sprite_ctas(count);
+    if ((uint64_t)ctas * kSpriteCta < (uint64_t)count * kSpriteThreads)
+      std::printf("%u: too few CTAs\n", count);
+    for (uint32_t block : {0u, ctas / 2u, ctas - 1u})
+      for (uint32_t t = 0; t < kSpriteCta; ++t)
+        if (sprite_of_thread(block, t) != ((uint64_t)block * kSpriteCta + t) / kSpriteThreads)
+          std::printf("%u: thread %u of CTA %u draws %u\n", count, t, block,
+                      sprite_of_thread(block, t));
+  }
+""")
+    assert lines == []
