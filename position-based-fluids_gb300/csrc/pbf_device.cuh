@@ -46,56 +46,104 @@ __device__ __forceinline__ void warp_digit_histogram(uint32_t key, bool valid,
   }
 }
 
+// Counts a warp's keys (four per lane, key u of the lane's particle i + u * step;
+// bit u of `valid`) with one atomic for all lanes of the same key, if more than
+// kManyApart lanes see their key again 16, 18 or 20 lanes on; returns whether it
+// did, the same in every lane.  The atomics on one word wait for each other, about
+// 1 ns each: 1M random keys of 2 cells 181 us by runs and 24 joined, of 8 cells 125
+// and 22, 4.2M of which half are the same 878 and 196.  Keys that a warp hardly
+// repeats are better left to the runs, as __match_any_sync takes a round per
+// distinct one (4.2M nearly in order 28 and 20 us: 3 such lanes on average; keys of
+// 64 cells too, which the rule leaves at 253 us for 171); and one test for all four
+// keys leaves their atomics together (a test per key: the 4.2M-particle scene's
+// hashes 18 us instead of 12).
+constexpr uint32_t kManyApart = 8;  // of four keys' lanes
+__device__ __forceinline__ bool count_joined(uint4 keys, uint32_t valid, uint32_t i,
+                                             uint32_t step, uint32_t *__restrict__ counts,
+                                             uint32_t *__restrict__ pos) {
+  constexpr unsigned kWarp = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t key[4] = {keys.x, keys.y, keys.z, keys.w};
+  uint32_t apart = 0;  // lanes whose key another lane holds
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    bool again = false;
+#pragma unroll
+    for (const uint32_t o : {16u, 18u, 20u}) {
+      const uint32_t other = __shfl_down_sync(kWarp, key[u], o);  // every lane
+      again |= other == key[u] && lane + o < 32u;
+    }
+    apart += (uint32_t)__popc(__ballot_sync(kWarp, again));
+  }
+  if (apart <= kManyApart) return false;
+  unsigned same[4];
+  uint32_t base[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const bool counts_here = valid >> u & 1u;
+    same[u] = __match_any_sync(kWarp, counts_here ? key[u] : kWarp);
+    base[u] = 0;
+    if (counts_here && lane == (uint32_t)__ffs((int)same[u]) - 1u)
+      base[u] = atomicAdd(&counts[key[u]], (uint32_t)__popc(same[u]));
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const uint32_t first = __shfl_sync(kWarp, base[u], __ffs((int)same[u]) - 1);
+    if (valid >> u & 1u)
+      pos[i + (uint32_t)u * step] = first + (uint32_t)__popc(same[u] & ((1u << lane) - 1u));
+  }
+  return true;
+}
+
 // Counts kKeys keys per lane (whole warp) into counts[] for the counting sort,
 // all their atomics in flight together: one atomic per run of equal keys in
 // neighbouring lanes; pos[i] = the particle's place among the increments of
-// its cell (a group's lanes in order, groups in atomic order).
-// kScattered: keys in any order, so a warp in which some lanes 2, 4, 8 or 16 apart
-// hold the same key joins all equal ones: the atomics on one word wait for each
-// other, about 1 ns each.  1M random keys of 2 cells are counted in 24 us (a run at
-// a time 181), of 8 cells 22 (125), 4.2M of which half are the same 192 (288), 4.2M
-// nearly in order 23 (31; all warps through __match_any_sync, a round per distinct
-// key, 33).  A step's kernels count by runs alone: with so many particles per cell
-// its passes over the pairs take a thousand times as long.
+// its cell (a run's lanes in order, runs in atomic order).
+// kScattered (four keys, equally far apart): keys in any order, so warps of more
+// than kManyRuns runs per key look for lanes to join; the 4.2M-particle scene's
+// hashes have 10 runs.  (A step's kernels count by runs alone: with so many
+// particles per cell its passes over the pairs take a thousand times as long.)
+constexpr uint32_t kManyRuns = 12;  // of a warp's 32 keys
 template <bool kScattered, int kKeys>
 __device__ __forceinline__ void count_cell_keys(const uint32_t (&key)[kKeys],
                                                 const bool (&valid)[kKeys],
                                                 const uint32_t (&i)[kKeys],
                                                 uint32_t *__restrict__ counts,
                                                 uint32_t *__restrict__ pos) {
-  constexpr unsigned kWarp = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31u;
-  unsigned group[kKeys];  // lanes counted by one atomic, the caller among them
-  uint32_t base[kKeys];
+  uint32_t head[kKeys], end[kKeys], base[kKeys], runs = 0;
 #pragma unroll
   for (int u = 0; u < kKeys; ++u) {
-    const uint32_t before = __shfl_up_sync(kWarp, key[u], 1);
-    const bool valid_before = __shfl_up_sync(kWarp, (int)valid[u], 1);
+    const uint32_t before = __shfl_up_sync(0xffffffffu, key[u], 1);
+    const bool valid_before = __shfl_up_sync(0xffffffffu, (int)valid[u], 1);
     const unsigned heads =
-        __ballot_sync(kWarp, lane == 0u || key[u] != before || valid[u] != valid_before);
+        __ballot_sync(0xffffffffu, lane == 0u || key[u] != before || valid[u] != valid_before);
     // the caller's run: from the last head at or below its lane to the next one
-    const unsigned below = kWarp >> (31u - lane);
-    const uint32_t head = 31u - (uint32_t)__clz((int)(heads & below));
+    const unsigned below = 0xffffffffu >> (31u - lane);
+    head[u] = 31u - (uint32_t)__clz((int)(heads & below));
     const unsigned later = heads & ~below;
-    const uint32_t end = later ? (uint32_t)__ffs((int)later) - 1u : 32u;
-    group[u] = kWarp >> (32u - (end - head)) << head;
-    if (kScattered && __popc(heads) > 4) {
-      bool apart = false;  // the caller's key in another run
-#pragma unroll
-      for (uint32_t o = 2; o <= 16; o <<= 1) {
-        const uint32_t other = __shfl_xor_sync(kWarp, key[u], (int)o);  // every lane
-        apart |= other == key[u] && !(group[u] >> (lane ^ o) & 1u);
-      }
-      if (__any_sync(kWarp, apart)) group[u] = __match_any_sync(kWarp, valid[u] ? key[u] : kWarp);
+    end[u] = later ? (uint32_t)__ffs((int)later) - 1u : 32u;
+    runs += (uint32_t)__popc(heads);
+  }
+  if constexpr (kScattered) {
+    static_assert(kKeys == 4, "as count_joined takes them");
+    if (runs > kManyRuns * kKeys) {
+      const uint32_t bits = (valid[0] ? 1u : 0u) | (valid[1] ? 2u : 0u) | (valid[2] ? 4u : 0u) |
+                            (valid[3] ? 8u : 0u);
+      if (count_joined(make_uint4(key[0], key[1], key[2], key[3]), bits, i[0], i[1] - i[0], counts,
+                       pos))
+        return;
     }
-    base[u] = 0;
-    if (valid[u] && lane == (uint32_t)__ffs((int)group[u]) - 1u)
-      base[u] = atomicAdd(&counts[key[u]], (uint32_t)__popc(group[u]));
   }
 #pragma unroll
   for (int u = 0; u < kKeys; ++u) {
-    const uint32_t first = __shfl_sync(kWarp, base[u], __ffs((int)group[u]) - 1);
-    if (valid[u]) pos[i[u]] = first + (uint32_t)__popc(group[u] & ((1u << lane) - 1u));
+    base[u] = 0;
+    if (valid[u] && lane == head[u]) base[u] = atomicAdd(&counts[key[u]], end[u] - head[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < kKeys; ++u) {
+    const uint32_t first = __shfl_sync(0xffffffffu, base[u], (int)head[u]);
+    if (valid[u]) pos[i[u]] = first + (lane - head[u]);
   }
 }
 // Keys a thread takes at a time in the counting, predicting and scattering
