@@ -287,7 +287,7 @@ __device__ __forceinline__ void group_nbr_lambda_of(uint32_t p, const float4 *P,
     LambdaAcc acc{s[0], s[1], s[2], s[3], s[4]};
     if (!grouped) {
       acc = LambdaAcc{c.w_self, 0.f, 0.f, 0.f, 0.f};
-      cnt = scan_members_planes<Mem>(pk, k, key, sc, nc.off, planes, c, [&](uint32_t w, const uint4 &j) {
+      cnt = scan_members_planes<Mem, false>(pk, k, key, sc, nc.off, planes, c, [&](uint32_t w, const uint4 &j) {
         if (4u * w < c.maxn) nbr4[(size_t)w * c.n + k] = j;
         lambda_pair(acc, pk, Mem::ld(&P[j.x]), c);
         lambda_pair(acc, pk, Mem::ld(&P[j.y]), c);
@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
   // group: here from the planes, in the passes as visit_fallback does
   LambdaAcc all{c.w_self, 0.f, 0.f, 0.f, 0.f};
   if (!held)
-    cnt = scan_members_planes<OwnCopy>(pk, k, scene_cell(pk.x, pk.y, pk.z, sc), sc, s_off, planes, c,
+    cnt = scan_members_planes<OwnCopy, false>(pk, k, scene_cell(pk.x, pk.y, pk.z, sc), sc, s_off, planes, c,
                                        [&](uint32_t, const uint4 &j) {
                                          lambda_pair(all, pk, A[j.x], c);
                                          lambda_pair(all, pk, A[j.y], c);

@@ -112,7 +112,7 @@ struct EarlierPhase {
 // candidate and its mask bit took about 11 each.  The builds are bound by L1's
 // data path (79% busy: 128 bytes to the lanes per clock), so the planes' 12
 // bytes per candidate instead of 16 count as much as the instructions.
-// Measured at 1,048,576 particles: fused paper build + lambda 260 -> 201 us,
+// Measured at 1,048,576 particles: fused paper build + lambda 260 -> 196 us,
 // ref-compat build 226 -> 157 us.
 struct Planes {
   const float4 *x, *y, *z;
@@ -177,6 +177,13 @@ __device__ __forceinline__ uint32_t row_mask(const Planes &p, uint32_t c0, uint3
 // per thread measured the same alone, but its carve-out took L1 away from the
 // gather passes of other simulations' streams (three 1,048,576-particle scenes
 // at once: 2.02 ms a frame against 1.54).
+//
+// In crowded scenes the queue has to make room several times.  The lanes of a
+// warp (kWarp) do that together, as soon as one of them has to: each alone in its
+// turn, the rest of the warp waiting, made the fused build of 64,000 particles
+// with 185 members each 320 us instead of 98, and steps of a 262,144-particle
+// REF_COMPAT run with 46 particles in a cell 7.7 ms instead of 3.1.  So every lane
+// takes part in every row and chunk, with empty ones where it has none.
 template <int kCap>
 struct MaskQueue {
   uint2 chunk[kCap];     // (mask, first candidate + 31)
@@ -184,20 +191,31 @@ struct MaskQueue {
   uint32_t members = 0;  // members in them
   uint32_t words = 0;    // list words handed on
 
-  // Adds the members of mask m over the candidates from c0; word(w, slots)
-  // takes word w of the list whenever the queue has to make room.
-  template <typename Word>
-  __device__ __forceinline__ void add(uint32_t m, uint32_t c0, Word &&word) {
-    if (m == 0u) return;
-    if (chunks == (uint32_t)kCap) drain(word);
-    chunk[chunks++] = make_uint2(m, c0 + 31u);
-    members += (uint32_t)__popc(m);
+  // The row of candidates [a, b), in chunks of 32: adds the members that mask(c0)
+  // finds from c0 on; word(w, slots) takes word w of the list whenever the queue
+  // has to make room.  kWarp: all 32 lanes call it alike.
+  template <bool kWarp, typename Mask, typename Word>
+  __device__ __forceinline__ void add_row(uint32_t a, uint32_t b, Mask &&mask, Word &&word) {
+    for (uint32_t c0 = a & ~3u; any<kWarp>(c0 < b); c0 += 32u) {
+      const uint32_t m = c0 < b ? mask(c0) : 0u;
+      if (m != 0u) {
+        chunk[chunks++] = make_uint2(m, c0 + 31u);
+        members += (uint32_t)__popc(m);
+      }
+      if (any<kWarp>(chunks == (uint32_t)kCap)) drain(word);
+    }
   }
+  template <bool kWarp>
+  __device__ __forceinline__ static bool any(bool mine) {
+    return kWarp ? __any_sync(0xffffffffu, mine) : mine;
+  }
+  // Members added so far.
+  __device__ __forceinline__ uint32_t count() const { return 4u * words + members; }
   // Hands on every whole word; at most three members stay.
   template <typename Word>
   __device__ __forceinline__ void drain(Word &&word) {
     uint32_t at = 0;
-    uint2 c = chunk[0];
+    uint2 c = chunks ? chunk[0] : make_uint2(0u, 0u);
     for (; members >= 4u; members -= 4u) {
       uint32_t j[4];
 #pragma unroll

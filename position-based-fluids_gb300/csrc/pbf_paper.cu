@@ -178,13 +178,13 @@ template <int kBlock, bool kMasked>
 __global__ void __launch_bounds__(kBlock)
     k_nbr_build(const float4 *__restrict__ P, Planes planes, NbrCtx nc, PaperConsts c,
                 uint4 *__restrict__ nbr4, uint32_t *__restrict__ nbr_cnt) {
-  const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
-  if (k >= c.n) return;
+  // past the end the last particle once more: the warp stays whole
+  const uint32_t k = min(blockIdx.x * kBlock + threadIdx.x, c.n - 1u);
   const float4 pk = P[k];
   uint32_t cnt = 0;
   const SceneDesc &sc = scene_of(nc.scenes, nc.sid, k);
   if constexpr (kMasked) {
-    cnt = scan_members_planes(
+    cnt = scan_members_planes<EarlierKernel, true>(
         pk, k, nc.skeys[k], sc, nc.off, planes, c,
         [&](uint32_t w, const uint4 &j) {
           if (4u * w < c.maxn) nbr4[(size_t)w * c.n + k] = j;
@@ -215,14 +215,14 @@ __global__ void __launch_bounds__(kBlock)
     k_nbr_lambda(const float4 *__restrict__ P, Planes planes, NbrCtx nc, PaperConsts c,
                  uint4 *__restrict__ nbr4, uint32_t *__restrict__ nbr_cnt,
                  float4 *__restrict__ Q, float *__restrict__ R) {
-  const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
-  if (k >= c.n) return;
+  // past the end the last particle once more: the warp stays whole
+  const uint32_t k = min(blockIdx.x * kBlock + threadIdx.x, c.n - 1u);
   const float4 pk = P[k];
   uint32_t cnt = 0;
   LambdaAcc acc{c.w_self, 0.f, 0.f, 0.f, 0.f};
   const SceneDesc &sc = scene_of(nc.scenes, nc.sid, k);
   if constexpr (kMasked) {
-    cnt = scan_members_planes(
+    cnt = scan_members_planes<EarlierKernel, true>(
         pk, k, nc.skeys[k], sc, nc.off, planes, c,
         [&](uint32_t w, const uint4 &j) {
           if (4u * w < c.maxn) nbr4[(size_t)w * c.n + k] = j;

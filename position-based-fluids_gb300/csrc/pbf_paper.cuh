@@ -272,7 +272,7 @@ __device__ __forceinline__ void scan_members(const float4 &pk, uint32_t key, con
 // zero as well.  The candidate loop is 23 instructions per four candidates
 // (12 of them packed), where one candidate at a time with its member work
 // inside took about 18 each.
-template <typename Mem = EarlierKernel, typename Word>
+template <typename Mem, bool kWarp, typename Word>
 __device__ __forceinline__ uint32_t scan_members_planes(const float4 &pk, uint32_t k, uint32_t key,
                                                         const SceneDesc &s,
                                                         const uint32_t *__restrict__ off,
@@ -289,26 +289,28 @@ __device__ __forceinline__ uint32_t scan_members_planes(const float4 &pk, uint32
   const float2 px = make_float2(-pk.x, -pk.x), py = make_float2(-pk.y, -pk.y),
                pz = make_float2(-pk.z, -pk.z);
   MaskQueue<kMaskQueue> list;
-  uint32_t cnt = 0;
   for (int dz = -1; dz <= 1; ++dz) {
     const int z = cz + dz;
-    if (z < 0 || z >= nz) continue;
     for (int dy = -1; dy <= 1; ++dy) {
       const int y = cy + dy;
-      if (y < 0 || y >= ny) continue;
-      const uint32_t row = s.cell_base + (uint32_t)nx * ((uint32_t)y + (uint32_t)ny * (uint32_t)z);
-      const uint32_t a = Mem::ld(&off[row + x0]);
-      const uint32_t b = Mem::ld(&off[row + x1 + 1]);
-      const bool own = (dz | dy) == 0;
-      for (uint32_t c0 = a & ~3u; c0 < b; c0 += 32u) {
-        const uint32_t m =
-            own ? row_mask<true, Mem>(planes, c0, a, b, px, py, pz, kMinPair2, c.h2)
-                : row_mask<false, Mem>(planes, c0, a, b, px, py, pz, 0.f, c.h2);
-        cnt += (uint32_t)__popc(m);
-        list.add(m, c0, word);
+      uint32_t a = 0, b = 0;  // a row outside the grid holds nothing
+      if (z >= 0 && z < nz && y >= 0 && y < ny) {
+        const uint32_t row =
+            s.cell_base + (uint32_t)nx * ((uint32_t)y + (uint32_t)ny * (uint32_t)z);
+        a = Mem::ld(&off[row + x0]);
+        b = Mem::ld(&off[row + x1 + 1]);
       }
+      const bool own = (dz | dy) == 0;
+      list.template add_row<kWarp>(
+          a, b,
+          [&](uint32_t c0) {
+            return own ? row_mask<true, Mem>(planes, c0, a, b, px, py, pz, kMinPair2, c.h2)
+                       : row_mask<false, Mem>(planes, c0, a, b, px, py, pz, 0.f, c.h2);
+          },
+          word);
     }
   }
+  const uint32_t cnt = list.count();
   list.finish(k, word);
   return cnt;
 }

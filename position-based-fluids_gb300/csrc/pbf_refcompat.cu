@@ -40,8 +40,8 @@ namespace {
 
 constexpr int kThreads = 128;
 
-// Calls row(a, b) for the slot range [a, b) of each row of up to three cells
-// around the current cell of position p, in visiting order.  Cells outside
+// Calls row(a, b) for the slot range [a, b) of each of the nine rows of up to three
+// cells around the current cell of position p, in visiting order.  Cells outside
 // the grid hold nothing (the current cell itself may be outside).
 template <typename Row>
 __device__ __forceinline__ void ref_rows(float4 p, const RefConsts &k,
@@ -52,12 +52,16 @@ __device__ __forceinline__ void ref_rows(float4 p, const RefConsts &k,
   const int c1 = min(max((int)((p.y - k.min[1]) / k.clen[1]), -2), ny + 1);
   const int c2 = min(max((int)((p.z - k.min[2]) / k.clen[2]), -2), nz + 1);
   const int z0 = max(c2 - 1, 0), z1 = min(c2 + 1, nz - 1);
-  if (z0 > z1) return;
-  for (int x = max(c0 - 1, 0); x <= min(c0 + 1, nx - 1); ++x)
-    for (int y = max(c1 - 1, 0); y <= min(c1 + 1, ny - 1); ++y) {
+  for (int q = 0; q < 9; ++q) {
+    const int x = c0 + q / 3 - 1, y = c1 + q % 3 - 1;
+    uint32_t a = 0, b = 0;
+    if (z0 <= z1 && x >= 0 && x < nx && y >= 0 && y < ny) {
       const uint32_t first = (uint32_t)nz * ((uint32_t)y + (uint32_t)ny * (uint32_t)x);
-      row(__ldg(&off[first + z0]), __ldg(&off[first + z1 + 1]));
+      a = __ldg(&off[first + z0]);
+      b = __ldg(&off[first + z1 + 1]);
     }
+    row(a, b);
+  }
 }
 
 __device__ __forceinline__ float wider_h2(const RefConsts &k) {
@@ -72,7 +76,7 @@ __device__ __forceinline__ float wider_h2(const RefConsts &k) {
 // candidates instead of 16, and no lower bound) against an h^2 widened by more
 // than both evaluations can differ, 6 * 2^-24 relative; q itself, which every
 // scan meets, is taken out by its slot.
-template <typename Word>
+template <bool kWarp, typename Word>
 __device__ __forceinline__ uint32_t scan_ref_members(uint32_t q, const float4 &p,
                                                      const RefConsts &k,
                                                      const uint32_t *__restrict__ off,
@@ -81,15 +85,17 @@ __device__ __forceinline__ uint32_t scan_ref_members(uint32_t q, const float4 &p
                pz = make_float2(-p.z, -p.z);
   const float h2 = wider_h2(k);
   MaskQueue<kMaskQueue> list;
-  uint32_t cnt = 0;
   ref_rows(p, k, off, [&](uint32_t a, uint32_t b) {
-    for (uint32_t c0 = a & ~3u; c0 < b; c0 += 32u) {
-      uint32_t m = row_mask<false>(planes, c0, a, b, px, py, pz, 0.0f, h2);
-      if (q - c0 < 32u) m &= ~(0x80000000u >> (q - c0));
-      cnt += (uint32_t)__popc(m);
-      list.add(m, c0, word);
-    }
+    list.template add_row<kWarp>(
+        a, b,
+        [&](uint32_t c0) {
+          uint32_t m = row_mask<false>(planes, c0, a, b, px, py, pz, 0.0f, h2);
+          if (q - c0 < 32u) m &= ~(0x80000000u >> (q - c0));
+          return m;
+        },
+        word);
   });
+  const uint32_t cnt = list.count();
   list.finish(q, word);
   return cnt;
 }
@@ -292,11 +298,11 @@ __global__ void __launch_bounds__(kThreads, 10)
     k_rc_lambda(float4 *__restrict__ PS, Planes planes, float *__restrict__ SS,
                 const uint32_t *__restrict__ off, uint32_t n, RefConsts k, uint32_t maxn,
                 uint4 *__restrict__ nbr4, uint32_t *__restrict__ nbr_cnt) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
+  // past the end the last particle once more: the warp stays whole
+  const uint32_t q = min(blockIdx.x * blockDim.x + threadIdx.x, n - 1u);
   const float4 pi = PS[q];
   RefLambdaSums s;
-  const uint32_t cnt = scan_ref_members(
+  const uint32_t cnt = scan_ref_members<true>(
       q, pi, k, off, planes, [&](uint32_t w, const uint4 &j) {
         if (4u * w < maxn) nbr4[(size_t)w * n + q] = j;
         const float4 d[4] = {PS[j.x], PS[j.y], PS[j.z], PS[j.w]};
@@ -384,8 +390,8 @@ __global__ void __launch_bounds__(kThreads)
     k_rc_xsph(const float4 *__restrict__ PS, Planes planes, const float4 *__restrict__ VS,
               float4 *__restrict__ DV, const uint32_t *__restrict__ input,
               const uint32_t *__restrict__ off, uint32_t n, RefConsts k) {
-  const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
+  // past the end the last particle once more: the warp stays whole
+  const uint32_t q = min(blockIdx.x * blockDim.x + threadIdx.x, n - 1u);
   const float4 pi = PS[q];
   const float4 vi = VS[q];
   float sx = 0.0f, sy = 0.0f, sz = 0.0f;
@@ -397,7 +403,7 @@ __global__ void __launch_bounds__(kThreads)
       sz += t.z;
     }
   };
-  scan_ref_members(q, pi, k, off, planes, [&](uint32_t, const uint4 &j) {
+  scan_ref_members<true>(q, pi, k, off, planes, [&](uint32_t, const uint4 &j) {
     const float4 p[4] = {__ldg(&PS[j.x]), __ldg(&PS[j.y]), __ldg(&PS[j.z]), __ldg(&PS[j.w])};
     const float4 v[4] = {__ldg(&VS[j.x]), __ldg(&VS[j.y]), __ldg(&VS[j.z]), __ldg(&VS[j.w])};
 #pragma unroll
@@ -537,7 +543,7 @@ __global__ void __launch_bounds__(kGroupThreads)
     s.gvy = t[3];
     s.gvz = t[4];
   } else {  // found by one thread
-    cnt = scan_ref_members(q, pi, k, off, planes, [&](uint32_t w, const uint4 &j) {
+    cnt = scan_ref_members<false>(q, pi, k, off, planes, [&](uint32_t w, const uint4 &j) {
       if (4u * w < maxn) nbr4[(size_t)w * n + q] = j;
       const uint32_t slot[4] = {j.x, j.y, j.z, j.w};
       for (int e = 0; e < 4; ++e) s.add(pi, PS[slot[e]], k);
@@ -595,7 +601,7 @@ __global__ void __launch_bounds__(kGroupThreads)
   if (!g.writes) return;
   if (!held) {
     s[0] = s[1] = s[2] = 0.0f;
-    scan_ref_members(q, own.p, k, off, planes, [&](uint32_t, const uint4 &j) {
+    scan_ref_members<false>(q, own.p, k, off, planes, [&](uint32_t, const uint4 &j) {
       const uint32_t slot[4] = {j.x, j.y, j.z, j.w};
       for (int e = 0; e < 4; ++e) {
         RefTerms t;
