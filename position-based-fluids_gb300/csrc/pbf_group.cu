@@ -18,6 +18,8 @@
 // particles (cold caches) the list build with the first lambda takes 8.3 us
 // instead of 18.8, a delta-p pass 4.5 instead of 9.8, lambda 4.2 / 7.7,
 // vorticity 4.4 / 9.7 and XSPH 4.2 / 9.4; an empty kernel takes 2.3.
+#include <type_traits>
+
 #include "pbf_group.cuh"
 #include "pbf_paper.cuh"
 
@@ -400,6 +402,7 @@ struct TinyStep {
   float4 *X, *V, *X2, *V2;
   float *R;
   uint32_t *ID, *skeys, *off, *nbr_cnt, *cnt_max;
+  uint4 *nbr;
   uint32_t ncells, iterations;
 };
 
@@ -575,25 +578,45 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
   const Planes planes = {U, U + words, U + 2u * words};
   uint32_t cnt = group_scan<OwnCopy>(k, pk, scene_cell(pk.x, pk.y, pk.z, sc), sc, s_off, planes,
                                      c.h2, list);
+  if (!g.live) cnt = 0;  // (the list of its last particle is another warp's to write)
   const bool held = cnt != kNotHeld;
-  // a set that the list does not hold is re-derived by every thread of the
-  // group: here from the planes, in the passes as visit_fallback does
+  // a set that the list does not hold is found by every thread of the group alike
+  // and listed in global memory, with the first lambda summed on the way; one that
+  // is too large for that as well is re-derived in each pass, as visit_fallback does
   LambdaAcc all{c.w_self, 0.f, 0.f, 0.f, 0.f};
   if (!held)
-    cnt = scan_members_planes<OwnCopy, false>(pk, k, scene_cell(pk.x, pk.y, pk.z, sc), sc, s_off, planes, c,
-                                       [&](uint32_t, const uint4 &j) {
-                                         lambda_pair(all, pk, A[j.x], c);
-                                         lambda_pair(all, pk, A[j.y], c);
-                                         lambda_pair(all, pk, A[j.z], c);
-                                         lambda_pair(all, pk, A[j.w], c);
-                                       });
+    cnt = scan_members_planes<OwnCopy, false>(
+        pk, k, scene_cell(pk.x, pk.y, pk.z, sc), sc, s_off, planes, c,
+        [&](uint32_t w, const uint4 &j) {
+          if (g.writes && 4u * w < c.maxn) t.nbr[(size_t)w * c.n + k] = j;
+          lambda_pair(all, pk, A[j.x], c);
+          lambda_pair(all, pk, A[j.y], c);
+          lambda_pair(all, pk, A[j.z], c);
+          lambda_pair(all, pk, A[j.w], c);
+        });
   __syncwarp();
   if (g.writes) t.nbr_cnt[k] = cnt;
+  const bool far = !held && cnt <= c.maxn;
   const uint32_t listed = held ? cnt : 0u;
   const auto two = [&](uint32_t, int, uint32_t e) {
     if (e >= (uint32_t)kBuildList) return make_uint2(k, k);
     const ushort2 j = *reinterpret_cast<const ushort2 *>(list + e);
     return make_uint2(j.x, j.y);
+  };
+  // Sums of a pass for the warps with a set that its list does not hold: the far
+  // lists by their groups (apart from the others: one way to read both took 5% of
+  // an ordinary step), the rest by walk(sum).  1,000 particles of some 150 members
+  // 115 us a step; with the sets re-derived in every pass 908.
+  const bool all_held = __all_sync(kAll, held);
+  const auto unheld = [&](const auto &pass, const auto &own, auto &sum, auto &&walk) {
+    std::remove_reference_t<decltype(sum)> f;
+    group_sums(pass, own, k, far ? cnt : 0u, [&](uint32_t, int, uint32_t e) {
+                 return FirstEntries<EarlierPhase>::two(t.nc, k, e);
+               },
+               terms, f);
+    if (held) return;
+    if (!far) walk(f);
+    for (uint32_t i = 0; i < sizeof f / sizeof f[0]; ++i) sum[i] = f[i];
   };
   const uint32_t most = __reduce_max_sync(kAll, cnt);
   cluster_wait();  // every CTA of the cluster runs
@@ -608,16 +631,18 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
       const LambdaPass<OwnCopy> pass{A, c};
       float s[5];
       group_sums(pass, pk, k, listed, two, terms, s);
-      LambdaAcc acc{s[0], s[1], s[2], s[3], s[4]};
-      if (!held) {
-        if (it == 0) {
-          acc = all;
-        } else {
-          acc = LambdaAcc{c.w_self, 0.f, 0.f, 0.f, 0.f};
+      if (!all_held && it > 0)
+        unheld(pass, pk, s, [&](float (&f)[5]) {
+          LambdaAcc acc{c.w_self, 0.f, 0.f, 0.f, 0.f};
           visit_fallback<EarlierPhase>(t.nc, k,
                                        [&](uint32_t j) { lambda_pair(acc, pk, A[j], c); });
-        }
-      }
+          f[0] = acc.rho;
+          f[1] = acc.gx;
+          f[2] = acc.gy;
+          f[3] = acc.gz;
+          f[4] = acc.s;
+        });
+      const LambdaAcc acc = held || it > 0 ? LambdaAcc{s[0], s[1], s[2], s[3], s[4]} : all;
       lambda = acc.lambda(c);
       rho = acc.rho;
       store_copies(B, first, c.n, make_float4(pk.x, pk.y, pk.z, lambda), s_stage[0]);
@@ -639,13 +664,17 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
       const DeltaPass<OwnCopy, kTwelve> pass{B, c};
       float s[3];
       group_sums(pass, qk, k, listed, two, terms, s);
-      DeltaAcc acc{s[0], s[1], s[2]};
-      if (!held) {
-        acc = DeltaAcc{0.f, 0.f, 0.f};
-        visit_fallback<EarlierPhase>(t.nc, k, [&](uint32_t j) {
-          acc.template pair<kTwelve>(qk, B[j], c);
+      if (!all_held)
+        unheld(pass, qk, s, [&](float (&f)[3]) {
+          DeltaAcc acc{0.f, 0.f, 0.f};
+          visit_fallback<EarlierPhase>(t.nc, k, [&](uint32_t j) {
+            acc.template pair<kTwelve>(qk, B[j], c);
+          });
+          f[0] = acc.sx;
+          f[1] = acc.sy;
+          f[2] = acc.sz;
         });
-      }
+      const DeltaAcc acc{s[0], s[1], s[2]};
       const Moved m = delta_moved(acc, x, make_float4(d.x, d.y, d.z, 0.f), sc, c);
       d = m.d;
       pk = make_float4(m.p.x, m.p.y, m.p.z, 0.f);
@@ -664,12 +693,22 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
     const VortPass<OwnCopy> pass{A, U, c};
     float s[9];
     group_sums(pass, own, k, listed, two, terms, s);
+    if (!all_held)
+      unheld(pass, own, s, [&](float (&f)[9]) {
+        VortAcc acc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        visit_fallback<EarlierPhase>(
+            t.nc, k, [&](uint32_t j) { acc.pair(own.p, own.u, PU{A[j], U[j]}, c); });
+        f[0] = acc.wx;
+        f[1] = acc.wy;
+        f[2] = acc.wz;
+        f[3] = acc.sx;
+        f[4] = acc.sy;
+        f[5] = acc.sz;
+        f[6] = acc.xx;
+        f[7] = acc.xy;
+        f[8] = acc.xz;
+      });
     w = VortAcc{s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], s[8]};
-    if (!held) {
-      w = VortAcc{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      visit_fallback<EarlierPhase>(t.nc, k,
-                                   [&](uint32_t j) { w.pair(own.p, own.u, PU{A[j], U[j]}, c); });
-    }
   }
   const float wn = norm3(w.wx, w.wy, w.wz);
   const float4 pw = make_float4(pk.x, pk.y, pk.z, __fmul_rn(wn, own.u.w));
@@ -681,11 +720,15 @@ __global__ void __launch_bounds__(kTinyThreads, 1) k_tiny_step(TinyStep t) {
     const XsphPass<OwnCopy> pass{B, c};
     float s[3];
     group_sums(pass, pw, k, listed, two, terms, s);
+    if (!all_held)
+      unheld(pass, pw, s, [&](float (&f)[3]) {
+        XsphAcc acc{0.f, 0.f, 0.f};
+        visit_fallback<EarlierPhase>(t.nc, k, [&](uint32_t j) { acc.pair(pw, B[j], c); });
+        f[0] = acc.ex;
+        f[1] = acc.ey;
+        f[2] = acc.ez;
+      });
     e = XsphAcc{s[0], s[1], s[2]};
-    if (!held) {
-      e = XsphAcc{0.f, 0.f, 0.f};
-      visit_fallback<EarlierPhase>(t.nc, k, [&](uint32_t j) { e.pair(pw, B[j], c); });
-    }
   }
   if (g.writes)
     xsph_store(k, pw, own.u, make_float4(w.wx, w.wy, w.wz, wn),
@@ -788,6 +831,7 @@ cudaError_t tiny_step(const DeviceState &d, const PaperConsts &c, uint32_t ncell
   t.off = d.offsets;
   t.nbr_cnt = d.nbr_cnt;
   t.cnt_max = d.nbr_max;
+  t.nbr = d.nbr;
   t.ncells = ncells;
   t.iterations = iterations;
   // as many CTAs as the particles need, a power of two of them
