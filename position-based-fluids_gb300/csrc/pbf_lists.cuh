@@ -196,13 +196,15 @@ struct MaskQueue {
   // has to make room.  kWarp: all 32 lanes call it alike.
   template <bool kWarp, typename Mask, typename Word>
   __device__ __forceinline__ void add_row(uint32_t a, uint32_t b, Mask &&mask, Word &&word) {
-    for (uint32_t c0 = a & ~3u; any<kWarp>(c0 < b); c0 += 32u) {
+    for (uint32_t c0 = a & ~3u;; c0 += 32u) {
       const uint32_t m = c0 < b ? mask(c0) : 0u;
       if (m != 0u) {
         chunk[chunks++] = make_uint2(m, c0 + 31u);
         members += (uint32_t)__popc(m);
       }
-      if (any<kWarp>(chunks == (uint32_t)kCap)) drain(word);
+      const bool full = chunks == (uint32_t)kCap;
+      if (!any<kWarp>(full || c0 + 32u < b)) break;  // most rows: one vote
+      if (any<kWarp>(full)) drain(word);
     }
   }
   template <bool kWarp>
