@@ -482,9 +482,10 @@ size_t pbf_op_sort_cells_scratch_bytes(uint32_t n, uint32_t ncells);
  * [0, ncells] (the CSR cell offsets), d_sorted_keys and d_perm the stable
  * order (ties by index: d_perm[q] = index of the q-th key), the same as
  * pbf_op_sort_pairs with values NULL followed by pbf_op_cell_offsets.
- * Keys are counted per cell with warp-aggregated atomics, the counts
- * scanned into the offsets (decoupled look-back), every key scattered to its
- * cell, and each cell put back in index order (by one thread up to 16 keys,
+ * Keys are counted per cell (one atomic for equal keys of neighbouring lanes,
+ * or of a whole warp where it repeats its keys), the counts scanned into the
+ * offsets (decoupled look-back), every key scattered to its cell, and each cell
+ * put back in index order (by one thread up to 16 keys,
  * one warp up to 64, in shared memory up to 8192, through a bitmap of the
  * indices beyond).
  * Outputs must not alias the keys.  No reference counterpart beyond the

@@ -91,7 +91,7 @@ constexpr int kSortThreads = 256;
 constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kMaxSortPasses = 4;
-// Digit widths: 8 bits (one digit per scan thread) or 9 bits (two).
+// Digit widths; a digit pass has a thread per digit of either.
 constexpr uint32_t kMinDigitBits = 8;
 constexpr uint32_t kMaxDigitBits = 9;
 // passes * radix of any plan (four 8-bit passes, two 9-bit ones)
@@ -206,10 +206,15 @@ cudaError_t wait_selftest(uint32_t *scratch, uint32_t spin_limit, uint32_t *err,
 // The step's own order of the particles in a cell is left to the kernel that
 // gathers the state (ordered_slot) for cells of up to kRankCell particles, and
 // for any cell of a scene (a batch: of a capacity) of up to kRankAllParticles,
-// where the launch for the larger cells takes longer than what it does (steps
-// of 32,768 particles 93.5 -> 92.0 us).  The neighbour passes over a crowded
-// cell each test the pairs that ranking it reads, with more work per pair, so
-// the ranks never bound a step.
+// where the launch for the larger cells takes longer than what it does.  Steps
+// with that launch and without: 17,000 particles 84.3 and 82.7 us, 32,768 87.9 and
+// 86.7, 65,536 104.1 and 102.0 (three such scenes at once 57.0 and 54.5), in the
+// reference's equations 186.0 and 184.2, 198.6 and 196.1, 224.4 and 223.1.  The
+// neighbour passes over a crowded cell each test the pairs that ranking it reads,
+// with more work per pair, so the ranks do not bound a crowded step either: all of
+// 65,536 particles in one cell 269.6 and 271.2 ms, at eleven times the rest density
+// 66.2 and 66.3, four times 1.69 and 1.66 (REF_COMPAT 1,759 and 1,761, 140.4 and
+// 139.2, 12.76 and 12.74).
 constexpr uint32_t kRankCell = 64;
 constexpr uint32_t kRankAllParticles = 65536;
 // Layout of the sort's scratch (32-bit words).

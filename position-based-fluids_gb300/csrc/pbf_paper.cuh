@@ -267,11 +267,11 @@ __device__ __forceinline__ void scan_members(const float4 &pk, uint32_t key, con
 
 // The same members in the same order, found as masks: each row is tested up
 // to 32 candidates at a time from the position planes, and the masks' members
-// reach word(w, slots) in whole list words.  Returns the number of members.  Only the row of k's own cell can
-// hold k itself or a coincident particle, so only there r^2 is tested against
-// zero as well.  The candidate loop is 23 instructions per four candidates
-// (12 of them packed), where one candidate at a time with its member work
-// inside took about 18 each.
+// reach word(w, slots) in whole list words.  Returns the number of members.  Only
+// the row of k's own cell can hold k itself or a coincident particle, so only there
+// r^2 is tested against zero as well.  The candidate loop is 23 instructions per
+// four candidates (12 of them packed), where one candidate at a time with its member
+// work inside took about 18 each.  kWarp: all 32 lanes call it (MaskQueue).
 template <typename Mem, bool kWarp, typename Word>
 __device__ __forceinline__ uint32_t scan_members_planes(const float4 &pk, uint32_t k, uint32_t key,
                                                         const SceneDesc &s,

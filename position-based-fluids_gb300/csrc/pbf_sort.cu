@@ -449,17 +449,19 @@ inline uint32_t blocks_for(uint64_t n, uint32_t t) {
 }
 
 // ------------------------------------------------- counting sort by cell --
-// The cell keys of a step sorted in one pass: the predict kernel counts each
-// cell's particles (count_cell_key: warp-aggregated atomics, each particle
-// keeping its place among the increments of its cell), k_count_scan turns
-// the counts into the cell offsets (and zeroes them for the next step),
-// k_count_scatter puts every particle at its cell's offset plus its place,
-// and the cells are then put back in index order -- the order a stable sort
-// gives -- because the places of particles counted by different warps
-// follow the order of their atomics: k_cell_fix sorts cells of up to 16
-// particles in registers and lists the larger ones, k_cell_fix_big sorts
-// those of up to kBigCell in shared memory (one CTA per cell) and larger
-// ones through a per-CTA bitmap of the particle indices.
+// Cell keys sorted in one pass: each cell's particles are counted
+// (count_cell_keys: one atomic per run of a warp's equal keys, each particle keeping
+// its place among the increments of its cell) by the step's predict kernel or, for
+// the operator, by k_count_keys; k_count_scan turns the counts into the cell offsets
+// (and zeroes them for the next sort), and k_count_scatter puts every particle at
+// its cell's offset plus its place.  The places of particles counted by different
+// warps follow the order of their atomics, so the cells are then put back in index
+// order -- the order a stable sort gives.  In a step the gather of the state does
+// that for most cells (ordered_slot) and the scan lists the larger ones for
+// k_cell_fix_big.  The operator runs k_cell_fix over all cells, which sorts those of
+// up to 16 particles in registers (up to kLightCell on sparse grids) and lists the
+// others.  k_cell_fix_big sorts listed cells of up to kBigCell in shared memory (one
+// CTA per cell) and larger ones through a per-CTA bitmap of the particle indices.
 constexpr uint32_t kScanItems = 8;                            // counts per thread and chunk
 constexpr uint32_t kScanChunk = kSortThreads * kScanItems;   // 2048
 constexpr uint32_t kScanChunks = 4;    // chunks per scan tile, where there are many
